@@ -215,23 +215,20 @@ XR_API xr_status xr_rc_set_count_samples(xr_raycaster rc, int32_t enable);
  * sum kernel; identical values, measured 3-4x slower than the gather, never
  * autotuned; block shape and loop are ignored), warps
  * across a 256-thread block (1, 2, 4 or 8; each warp covers 8x4 pixels) and
- * the sample loop: 1 or 2 samples per iteration, or 3 / 4 = 2 / 4 per iteration
- * after each ray is trimmed to its first and last occupied macro cell (sum
- * kernel with empty-space skipping on; otherwise 3 and 4 run as 2), or 5 = 3
- * with the second sample of a pair reusing the first's corners when both lie in
- * one cell (256-bit float32 CELL8 read; elsewhere 5 runs as 3), or 6 = 4 on
- * packed FP32 pairs (float32 256-bit or FP16 / BF16 CELL8 reads; elsewhere 6
- * runs as 4).  layout
+ * the loop number: 1 and 2 sample from the support box on, 3 to 6 after each ray
+ * is trimmed to its first and last occupied macro cell (sum kernel with
+ * empty-space skipping on; otherwise as 2).  layout
  * XR_LAYOUT_AUTO (the default) lets
- * the autotuner time the candidates on the first compute of each shape (volume
+ * the autotuner time the block shapes on the first compute of each shape (volume
  * size, voxel type, detector, projection count) and cache the fastest for the
- * process.  No xReg counterpart (xReg's OpenCL caster has a fixed NDRange). */
+ * process; the cell copy, one load per sample, and loop 4 are always its choice.
+ * A volume that holds an infinity or a value above 2^126 is read in the LINEAR
+ * layout whatever is asked for.  No xReg counterpart (xReg's OpenCL caster has a fixed NDRange). */
 XR_API xr_status xr_rc_set_launch_config(xr_raycaster rc, int32_t layout, int32_t block_warps_x, int32_t unroll);
 /* The configuration the last compute used. */
 XR_API xr_status xr_rc_get_launch_config(xr_raycaster rc, int32_t* layout, int32_t* block_warps_x, int32_t* unroll);
 /* As xr_rc_set_launch_config with the warp shape too: warp_rows 4 = each warp
- * covers 8x4 pixels (what xr_rc_set_launch_config sets), 8 = 4x8.  The
- * autotuner also times 4x8 warps for its fastest layout and loop. */
+ * covers 8x4 pixels (what xr_rc_set_launch_config sets), 8 = 4x8. */
 XR_API xr_status xr_rc_set_launch_config_ex(xr_raycaster rc, int32_t layout, int32_t block_warps_x, int32_t unroll,
                                             int32_t warp_rows);
 XR_API xr_status xr_rc_get_launch_config_ex(xr_raycaster rc, int32_t* layout, int32_t* block_warps_x,

@@ -155,6 +155,7 @@ struct xr_raycaster_s {
     int32_t type = XR_VOXEL_F32;
     float inv_scale = 1.0f;
     int32_t cs[2] = {0, 0};     // CELL8 cell strides (VolView::cs)
+    bool weighted = false;      // VolView::weighted
     bool has_support = false;   // support box of the non-zero voxels (empty-space skipping)
     float sup_lo[3] = {0, 0, 0}, sup_hi[3] = {0, 0, 0};
     DevBuf occ;                 // macro-cell occupancy bitmask
@@ -482,57 +483,57 @@ static xr_status rc_set_volumes_impl(xr_raycaster rc, int32_t n, const xr_volume
     cell_strides(d.n[0], d.n[1], d.n[2], v->cs);
     const size_t esz = vt == XR_VOXEL_F32 ? 4 : 2;
     XR_CUDA_TRY(v->voxels.reserve((size_t)nv * esz));
+    DevBuf tmp;
+    const float* src = voxels[i];
     if (vt == XR_VOXEL_F32) {
       XR_CUDA_TRY(cudaMemcpyAsync(v->voxels.p, voxels[i], (size_t)nv * 4,
                                   on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
+      src = v->voxels.as<float>();
+    } else if (!on_device) {
+      XR_CUDA_TRY(tmp.reserve((size_t)nv * 4));
+      XR_CUDA_TRY(cudaMemcpyAsync(tmp.p, voxels[i], (size_t)nv * 4, cudaMemcpyHostToDevice, s));
+      src = tmp.as<float>();
+    }
+    // largest magnitude (NaN left out)
+    XR_CUDA_TRY(cudaMemsetAsync(rc->d_counters.as<char>() + 16, 0, 4, s));
+    max_abs_kernel<<<1024, 256, 0, s>>>(src, nv, reinterpret_cast<unsigned int*>(rc->d_counters.as<char>() + 16));
+    XR_CUDA_TRY(cudaGetLastError());
+    unsigned int bits = 0;
+    XR_CUDA_TRY(cudaMemcpyAsync(&bits, rc->d_counters.as<char>() + 16, 4, cudaMemcpyDeviceToHost, s));
+    XR_CUDA_TRY(cudaStreamSynchronize(s));
+    float mx;
+    std::memcpy(&mx, &bits, 4);
+    float sc = scale > 0.0f ? scale : 1.0f;
+    if (vt == XR_VOXEL_F32) {
+      sc = 1.0f;
       v->inv_scale = 1.0f;
-      if (rc->build_cells) {
-        XR_CUDA_TRY(v->cells.reserve(cell_layout_bytes(d.n[0], d.n[1], d.n[2], vt)));
-        XR_CUDA_TRY(launch_build_cells(v->voxels.as<float>(), (int)d.n[0], (int)d.n[1], (int)d.n[2], vt, 1.0f,
-                                       v->cells.p, s));
-      }
-      xr_status st = vol_support(rc, *v, v->voxels.as<float>(), s);
-      if (st != XR_OK) return st;
+    } else if (vt == XR_VOXEL_F16) {
+      // The half2 blend multiplies stored values by x weights scaled by 2^15
+      // (so that fractions down to 2^-24 stay normal halves) and the y blend
+      // by 2^15 more; stored values below 1 keep the blend below 2^15.  So
+      // FP16 always stores the maximum in [0.5, 1) (a given scale is not used).
+      XR_CHECK_ARG(std::isfinite(mx), "set_volumes: non-finite voxel");
+      // the scale (at most 2^90) and its inverse times 2^-30 stay normal floats
+      XR_CHECK_ARG(mx == 0.0f || mx >= 0x1p-90f, "set_volumes: FP16 volume maximum below 2^-90");
+      sc = mx > 0.0f ? (float)std::ldexp(1.0, (int)std::floor(std::log2(1.0 / (double)mx))) : 1.0f;
+      v->inv_scale = (float)(1.0 / ((double)sc * 32768.0 * 32768.0));
     } else {
-      DevBuf tmp;
-      const float* src = voxels[i];
-      if (!on_device) {
-        XR_CUDA_TRY(tmp.reserve((size_t)nv * 4));
-        XR_CUDA_TRY(cudaMemcpyAsync(tmp.p, voxels[i], (size_t)nv * 4, cudaMemcpyHostToDevice, s));
-        src = tmp.as<float>();
-      }
-      float sc = scale > 0.0f ? scale : 1.0f;
-      if (vt == XR_VOXEL_F16) {
-        // The half2 blend multiplies stored values by x weights scaled by 2^15
-        // (so that fractions down to 2^-24 stay normal halves) and the y blend
-        // by 2^15 more; stored values below 1 keep the blend below 2^15.  So
-        // FP16 always stores the maximum in [0.5, 1) (a given scale is not used).
-        XR_CUDA_TRY(cudaMemsetAsync(rc->d_counters.as<char>() + 16, 0, 4, s));
-        max_abs_kernel<<<1024, 256, 0, s>>>(src, nv, reinterpret_cast<unsigned int*>(rc->d_counters.as<char>() + 16));
-        XR_CUDA_TRY(cudaGetLastError());
-        unsigned int bits = 0;
-        XR_CUDA_TRY(cudaMemcpyAsync(&bits, rc->d_counters.as<char>() + 16, 4, cudaMemcpyDeviceToHost, s));
-        XR_CUDA_TRY(cudaStreamSynchronize(s));
-        float mx;
-        std::memcpy(&mx, &bits, 4);
-        XR_CHECK_ARG(std::isfinite(mx), "set_volumes: non-finite voxel");
-        // the scale (at most 2^90) and its inverse times 2^-30 stay normal floats
-        XR_CHECK_ARG(mx == 0.0f || mx >= 0x1p-90f, "set_volumes: FP16 volume maximum below 2^-90");
-        sc = mx > 0.0f ? (float)std::ldexp(1.0, (int)std::floor(std::log2(1.0 / (double)mx))) : 1.0f;
-        v->inv_scale = (float)(1.0 / ((double)sc * 32768.0 * 32768.0));
-      } else {
-        v->inv_scale = 1.0f / sc;
-      }
+      v->inv_scale = 1.0f / sc;
+    }
+    // Differences of corners must be finite for the blends of float32 and BF16
+    // volumes; a volume where they might not be is read as it lies (VolView::weighted).
+    v->weighted = vt != XR_VOXEL_F16 && !(mx * sc <= 0x1p126f);
+    if (vt != XR_VOXEL_F32) {
       convert_voxels_kernel<<<2048, 256, 0, s>>>(src, nv, sc, vt, v->voxels.p);
       XR_CUDA_TRY(cudaGetLastError());
-      if (rc->build_cells) {
-        XR_CUDA_TRY(v->cells.reserve(cell_layout_bytes(d.n[0], d.n[1], d.n[2], vt)));
-        XR_CUDA_TRY(launch_build_cells(src, (int)d.n[0], (int)d.n[1], (int)d.n[2], vt, sc, v->cells.p, s));
-      }
-      xr_status st = vol_support(rc, *v, src, s);
-      if (st != XR_OK) return st;
-      XR_CUDA_TRY(cudaStreamSynchronize(s));  // tmp is released at scope exit
     }
+    if (rc->build_cells && !v->weighted) {
+      XR_CUDA_TRY(v->cells.reserve(cell_layout_bytes(d.n[0], d.n[1], d.n[2], vt)));
+      XR_CUDA_TRY(launch_build_cells(src, (int)d.n[0], (int)d.n[1], (int)d.n[2], vt, sc, v->cells.p, s));
+    }
+    xr_status st = vol_support(rc, *v, src, s);
+    if (st != XR_OK) return st;
+    XR_CUDA_TRY(cudaStreamSynchronize(s));  // tmp is released at scope exit
     vols.push_back(std::move(v));
   }
   XR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -873,7 +874,7 @@ struct TuneKeyHash {
   }
 };
 struct TuneCfg {
-  int32_t layout, bw, unroll, tall;
+  int32_t bw, tall;
   float ms;
 };
 std::mutex g_tune_mu;
@@ -925,39 +926,48 @@ static bool rc_config_cached(xr_raycaster rc, const xr_raycaster_s::Vol& vol, co
   return g_tune.find(tune_key(rc, vol, p)) != g_tune.end();
 }
 
-// Picks the launch configuration for p (layout, block_warps_x, unroll, warp shape).
-static xr_status rc_choose_config(xr_raycaster rc, const xr_raycaster_s::Vol& vol, DrrParams& p, cudaStream_t s) {
-  const bool has_cells = vol.cells.p != nullptr;
+// Layout the kernels read a volume's voxels fastest in: the cell copy with one
+// load per sample (256 bits of float32, 128 of FP16 / BF16), else the voxels.
+static int32_t best_layout(const xr_raycaster_s::Vol& vol) {
+  if (vol.cells.p == nullptr) return XR_LAYOUT_LINEAR;
+  return vol.type == XR_VOXEL_F32 ? 2 : XR_LAYOUT_CELL8;
+}
+
+// Picks the launch configuration for p (layout, block_warps_x, warp shape) and
+// the loop number that xr_rc_get_launch_config reports: 1 and 2 run without the
+// macro-cell trim, 3 and above with it.
+static xr_status rc_choose_config(xr_raycaster rc, const xr_raycaster_s::Vol& vol, DrrParams& p, cudaStream_t s,
+                                  int32_t* loop) {
   if (rc->cfg_layout != XR_LAYOUT_AUTO) {
+    const bool has_cells = vol.cells.p != nullptr || vol.weighted;
     if (rc->cfg_layout != XR_LAYOUT_LINEAR && !has_cells)
       return fail(XR_ERR_INVALID_ARG, "compute: CELL8 layout requested but the volume has no cell copy");
     if (rc->cfg_layout == 2 && vol.type != XR_VOXEL_F32)
       return fail(XR_ERR_INVALID_ARG, "compute: the 256-bit CELL8 read needs a float32 volume");
     if (rc->cfg_layout == 3 && (vol.type != XR_VOXEL_F32 || p.kernel_id != XR_LINE_INT_SUM))
       return fail(XR_ERR_INVALID_ARG, "compute: the brick-staged layout needs a float32 volume and the sum kernel");
-    p.vol.layout = rc->cfg_layout;
+    p.vol.layout = vol.weighted ? XR_LAYOUT_LINEAR : rc->cfg_layout;  // only LINEAR has the weighted blend
     p.block_warps_x = rc->cfg_bw;
-    p.unroll = rc->cfg_unroll;
     p.warp_tall = rc->cfg_warp_rows == 8 ? 1 : 0;
+    *loop = rc->cfg_unroll;
+    if (rc->cfg_unroll <= 2) p.vol.occ = nullptr;
     return XR_OK;
   }
+  *loop = 4;
+  p.vol.layout = best_layout(vol);
   const TuneKey key = tune_key(rc, vol, p);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
-      p.vol.layout = it->second.layout;
       p.block_warps_x = it->second.bw;
-      p.unroll = it->second.unroll;
       p.warp_tall = it->second.tall;
       return XR_OK;
     }
   }
-  // default when tuning is not possible right now
-  p.vol.layout = has_cells ? XR_LAYOUT_CELL8 : XR_LAYOUT_LINEAR;
-  p.block_warps_x = 2;
-  p.unroll = 1;
-  p.warp_tall = 0;
+  // default when tuning is not possible right now: the shape it mostly chooses
+  p.block_warps_x = 1;
+  p.warp_tall = 1;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   XR_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
   // Tuning re-runs the kernel; it needs a stream that is not being captured and an
@@ -965,55 +975,25 @@ static xr_status rc_choose_config(xr_raycaster rc, const xr_raycaster_s::Vol& vo
   if (cap != cudaStreamCaptureStatusNone || p.store != XR_PROJ_STORE_REPLACE || p.bg_projs) return XR_OK;
   DrrParams t = p;
   t.sample_counter = nullptr;
-  TuneCfg best{p.vol.layout, p.block_warps_x, p.unroll, 0, 1e30f};
-  // layout 2 = CELL8 read with one 256-bit load per sample (float32 only)
-  const int32_t layouts[3] = {XR_LAYOUT_LINEAR, XR_LAYOUT_CELL8, 2};
+  TuneCfg best{p.block_warps_x, p.warp_tall, 1e30f};
+  // Block shapes: 1, 2 or 4 warps across, of 8x4 or 4x8 pixels.  (Layout and
+  // loop are not tuned: the cell copy with the trimmed four-sample loop was the
+  // fastest of all, for each voxel type, on every shape measured.)
   const int32_t bws[3] = {1, 2, 4};
-  // loops 3 and 4 = 2 and 4 samples per iteration after the macro-cell trim (sum
-  // kernel); 5 = loop 3 whose pairs share one load when both samples fall in one
-  // cell (256-bit float32 CELL8 read), 6 = loop 4 on packed FP32 pairs (256-bit
-  // float32 or 128-bit half CELL8 reads)
-  const int32_t unrolls[6] = {1, 2, 3, 4, 5, 6};
-  for (int32_t lay : layouts) {
-    if (lay != XR_LAYOUT_LINEAR && !has_cells) continue;
-    if (lay == 2 && vol.type != XR_VOXEL_F32) continue;
-    for (int32_t bw : bws)
-      for (int32_t un : unrolls) {
-        if (un >= 3 && !(p.vol.occ && p.kernel_id == XR_LINE_INT_SUM)) continue;
-        if (un == 5 && lay != 2) continue;
-        if (un == 6 && !(lay == 2 || (lay == XR_LAYOUT_CELL8 && vol.type != XR_VOXEL_F32))) continue;
-        t.vol.layout = lay;
-        t.block_warps_x = bw;
-        t.unroll = un;
-        t.warp_tall = 0;
-        float ms = 0.0f;
-        xr_status st = time_config(t, s, &ms);
-        if (st != XR_OK) return st;
-        if (ms < best.ms) best = TuneCfg{lay, bw, un, 0, ms};
-      }
-  }
-  // 4x8-pixel warps for the fastest layout and loop (rays of a warp span more
-  // detector rows, which changes how their cells share L1 lines)
-  {
-    const TuneCfg wide = best;
+  for (int32_t tall : {1, 0})
     for (int32_t bw : bws) {
-      t.vol.layout = wide.layout;
       t.block_warps_x = bw;
-      t.unroll = wide.unroll;
-      t.warp_tall = 1;
+      t.warp_tall = tall;
       float ms = 0.0f;
       xr_status st = time_config(t, s, &ms);
       if (st != XR_OK) return st;
-      if (ms < best.ms) best = TuneCfg{wide.layout, bw, wide.unroll, 1, ms};
+      if (ms < best.ms) best = TuneCfg{bw, tall, ms};
     }
-  }
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune[key] = best;
   }
-  p.vol.layout = best.layout;
   p.block_warps_x = best.bw;
-  p.unroll = best.unroll;
   p.warp_tall = best.tall;
   return XR_OK;
 }
@@ -1073,6 +1053,8 @@ static xr_status rc_prepare(xr_raycaster rc, int32_t vol_idx, cudaStream_t s, Dr
   p.vol.inv_scale = vol.inv_scale;
   p.vol.cs[0] = vol.cs[0];
   p.vol.cs[1] = vol.cs[1];
+  cell_floor_constants(vol.desc.n[0], vol.desc.n[1], vol.desc.n[2], vol.type, p.vol.kfl, &p.vol.cell_bytes);
+  p.vol.weighted = vol.weighted ? 1 : 0;
   p.vol.has_support = (rc->skip_empty && vol.has_support) ? 1 : 0;
   p.vol.occ = rc->skip_empty ? vol.occ.as<uint32_t>() : nullptr;
   p.vol.nmx = vol.nmx;
@@ -1124,11 +1106,12 @@ static xr_status rc_enqueue_compute(xr_raycaster rc, int32_t vol_idx) {
   xr_status st = rc_prepare(rc, vol_idx, s, p);
   if (st != XR_OK) return st;
   const auto& vol = *rc->vols[(size_t)vol_idx];
-  st = rc_choose_config(rc, vol, p, s);
+  int32_t loop = 0;
+  st = rc_choose_config(rc, vol, p, s, &loop);
   if (st != XR_OK) return st;
   rc->last_layout = p.vol.layout;
   rc->last_bw = p.block_warps_x;
-  rc->last_unroll = p.unroll;
+  rc->last_unroll = loop;
   rc->last_warp_rows = p.warp_tall ? 8 : 4;
   XR_CUDA_TRY(launch_drr(p, s));
   if (rc->ext_host)
@@ -2159,26 +2142,17 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
     if ((st = rc_prepare(rc, obj->vol_idx, s, J.d.p, false)) != XR_OK) return st;
     XR_CHECK_ARG(J.d.p.kernel_id == XR_LINE_INT_SUM, "evaluation: the fused step uses the line-integral sum kernel");
     const auto& vol = *rc->vols[(size_t)obj->vol_idx];
-    // the ray caster's autotuned layout and block shape; the fused kernel runs
-    // the four-sample loop (packed pairs where the tuner chose them); without
-    // the macro-cell trim, or with a configuration fixed by the caller that the
-    // fused kernel lacks, float32 volumes read their cell copy with one 256-bit
-    // load and half volumes with one 128-bit load
+    // each job in its ray caster's autotuned block shape
     DrrParams& P = J.d.p;
-    const bool cells = vol.cells.p != nullptr;
-    const int32_t wide = cells ? (vol.type == XR_VOXEL_F32 ? 2 : XR_LAYOUT_CELL8) : XR_LAYOUT_LINEAR;
-    // each job in its autotuned block shape and sample loop: the DRR job
-    // kernel runs loop 3 (for the tuner's 1 to 3), 4 (4, 5) or the packed 6,
-    // the fused kernel loop 4 or 6
     if (!rc_config_cached(rc, vol, P)) {  // the tuner times real launches: this caster's geometry first
       XR_CUDA_TRY(launch_proj_geom(vol.desc, rc->d_cams.as<xr_camera_desc>(), rc->d_xforms.as<double>(),
                                    rc->d_cam_idx.as<int32_t>(), rc->num_projs, rc->pose_count,
                                    rc->d_geo.as<ProjGeom>(), s));
       ++tuning_launches;
     }
-    if ((st = rc_choose_config(rc, vol, P, s)) != XR_OK) return st;
-    P.unroll = (P.unroll == 6 && cells) ? 6 : (!fused && P.unroll <= 3 ? 3 : 4);
-    P.vol.layout = wide;
+    int32_t loop = 0;
+    if ((st = rc_choose_config(rc, vol, P, s, &loop)) != XR_OK) return st;
+    P.vol.layout = best_layout(vol);
     const int wc = P.warp_tall ? 4 : 8, tw = wc * P.block_warps_x, th = (8 / P.block_warps_x) * (32 / wc);
     J.d.tiles_x = (int32_t)((P.cols + tw - 1) / tw);
     J.d.tiles_y = (int32_t)((P.rows + th - 1) / th);
@@ -2191,7 +2165,7 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
     }
     rc->last_layout = P.vol.layout;
     rc->last_bw = P.block_warps_x;
-    rc->last_unroll = P.unroll;
+    rc->last_unroll = loop;
     rc->last_warp_rows = P.warp_tall ? 8 : 4;
     GeomJob G{};
     G.p2i = phys_to_idx_xform(vol.desc);
@@ -2325,7 +2299,7 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
     if (fused)
       XR_CUDA_TRY(launch_eval_fused(reinterpret_cast<const FusedJob*>(d + off_f) + ranges[gi].first,
                                     (int)(ranges[gi].second - ranges[gi].first), group_items[gi],
-                                    f0.d.p.vol.voxel_type, f0.d.p.vol.layout, f0.d.p.unroll,
+                                    f0.d.p.vol.voxel_type, f0.d.p.vol.layout,
                                     fw.d_counter.as<unsigned long long>(), &blocks, s));
     else {
       XR_CUDA_TRY(launch_drr_jobs(reinterpret_cast<const MultiJobDrr*>(d + off_m) + ranges[gi].first,

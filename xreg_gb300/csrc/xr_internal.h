@@ -28,8 +28,18 @@ struct VolView {
   int32_t voxel_type;
   int32_t layout;      // XR_LAYOUT_LINEAR / XR_LAYOUT_CELL8
   float inv_scale;     // multiplies the ray sum (1 for F32)
-  // CELL8 cell order, z fastest: cell (ix, iy, iz) is number ix cs[0] + iy cs[1] + iz
+  // CELL8 cell order, z fastest: cell (ix, iy, iz), -1 <= i < n, is number
+  // (ix + 1) cs[0] + (iy + 1) cs[1] + iz + 1
   int32_t cs[2];
+  // Round-down floor constants of the axes, 2^23 + m (cell_floor_constants);
+  // zeros: none, every ray takes the clamped sampler.  cell_bytes 1: they give a
+  // cell's byte offset (copies below 4 GB), 0: its number.
+  float kfl[3];
+  int32_t cell_bytes;
+  // 1: the voxels hold infinities or values above 2^126, so the trilinear takes
+  // the weighted form on the LINEAR layout (differences of corners would not be
+  // finite); such a volume has no cells.
+  int32_t weighted;
   // Support box: every sample whose continuous index lies outside
   // (sup_lo, sup_hi) on some axis interpolates only zero voxels.  has_support 0
   // disables sample skipping; an all-zero volume has an empty box (lo > hi).
@@ -62,7 +72,6 @@ struct DrrParams {
   int32_t store;          // XR_PROJ_STORE_REPLACE / ACCUM
   int32_t block_warps_x;  // warps across a block (1, 2, 4, 8)
   int32_t warp_tall;      // 0: each warp covers 8x4 pixels (cols x rows); 1: 4x8
-  int32_t unroll;         // sample loop 1..5 (xr_rc_set_launch_config)
 };
 
 // ---- launchers (xr_geom.cu) ----
@@ -94,8 +103,7 @@ struct MultiJobDrr {
   }
 };
 // One launch whose grid covers the (tile, projection) items of jobs sharing a
-// voxel type and layout (no work counter: one block per item); each job runs
-// its own sample loop, p.unroll 3, 4 or 6 (6 with the cell layouts only).
+// voxel type and layout (no work counter: one block per item).
 // grouped: every job's pose_group is 4 (otherwise every job's is 0).
 cudaError_t launch_drr_jobs(const MultiJobDrr* d_jobs, int njobs, long long total_items, int32_t voxel_type,
                             int32_t layout, bool grouped, cudaStream_t s);
@@ -112,6 +120,8 @@ cudaError_t launch_build_cells(const float* vox_f32, int nx, int ny, int nz, int
                                void* out, cudaStream_t s);
 // The x and y cell strides of that order (VolView::cs).
 void cell_strides(int64_t nx, int64_t ny, int64_t nz, int32_t cs[2]);
+// VolView::kfl and cell_bytes of a volume; zeros in kfl where there are none.
+void cell_floor_constants(int64_t nx, int64_t ny, int64_t nz, int32_t voxel_type, float kfl[3], int32_t* bytes);
 
 // ---- launchers (xr_metrics.cu) ----
 struct FixedNCC {           // per direction (one for NCC, x and y for grad-NCC)
@@ -155,8 +165,7 @@ struct FusedJob {
 };
 // One persistent launch over the jobs of one (voxel type, layout) group.
 cudaError_t launch_eval_fused(const FusedJob* d_jobs, int njobs, long long total_items, int32_t voxel_type,
-                              int32_t layout, int32_t unroll, unsigned long long* d_counter, int* blocks_out,
-                              cudaStream_t s);
+                              int32_t layout, unsigned long long* d_counter, int* blocks_out, cudaStream_t s);
 // Grad-NCC (5x5 smoothing) of every image of the jobs with `metric` set, their
 // DRRs already written: one launch over all their 32x64 tiles (the split
 // path's tile code), each image's FP64 combine by the block that completes its
