@@ -43,6 +43,10 @@ struct DevBuf {
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { release(); }
+  void swap(DevBuf& o) {
+    std::swap(p, o.p);
+    std::swap(bytes, o.bytes);
+  }
   void release() {
     if (p) cudaFree(p);
     p = nullptr;
@@ -73,24 +77,6 @@ struct DeviceGuard {
   }
   ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
 };
-
-__global__ void convert_voxels_kernel(const float* __restrict__ in, int64_t n, float scale, int vt, void* out) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float v = in[i] * scale;
-    if (vt == XR_VOXEL_F16) static_cast<__half*>(out)[i] = __float2half_rn(v);
-    else static_cast<__nv_bfloat16*>(out)[i] = __float2bfloat16_rn(v);
-  }
-}
-
-__global__ void max_abs_kernel(const float* __restrict__ in, int64_t n, unsigned int* out) {
-  unsigned int m = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float a = fabsf(in[i]);
-    if (a == a) m = max(m, __float_as_uint(a));
-  }
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
 
 __global__ void cam_idx_distribute_kernel(int32_t* out, int64_t n, int64_t per_cam) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -436,30 +422,15 @@ extern "C" XR_API xr_status xr_rc_synchronize(xr_raycaster rc) {
 // continuous index coordinates every sample outside (min - 1 - m, max + 1 + m)
 // on some axis interpolates only zero voxels.  The margin m = 0.5 voxel covers
 // the drift of positions advanced by repeated float addition.
-static xr_status vol_support(xr_raycaster rc, xr_raycaster_s::Vol& v, const float* vox_f32, cudaStream_t s) {
-  int* d_box = reinterpret_cast<int*>(rc->d_counters.as<char>() + 32);
-  XR_CUDA_TRY(launch_support_box(vox_f32, (int)v.desc.n[0], (int)v.desc.n[1], (int)v.desc.n[2], d_box, s));
-  int box[6];
-  XR_CUDA_TRY(cudaMemcpyAsync(box, d_box, sizeof(box), cudaMemcpyDeviceToHost, s));
-  XR_CUDA_TRY(cudaStreamSynchronize(s));
-  v.nmx = (int32_t)(((v.desc.n[0] - 1) + (1 << kMacroShift) - 1) >> kMacroShift);
-  v.nmy = (int32_t)(((v.desc.n[1] - 1) + (1 << kMacroShift) - 1) >> kMacroShift);
-  v.nmz = (int32_t)(((v.desc.n[2] - 1) + (1 << kMacroShift) - 1) >> kMacroShift);
-  const size_t words = ((size_t)v.nmx * v.nmy * v.nmz + 31) / 32;
-  XR_CUDA_TRY(v.occ.reserve(words * 4));
-  XR_CUDA_TRY(launch_build_occupancy(vox_f32, (int)v.desc.n[0], (int)v.desc.n[1], (int)v.desc.n[2],
-                                     v.occ.as<uint32_t>(), v.nmx, v.nmy, v.nmz, s));
+static void vol_support(xr_raycaster_s::Vol& v, const VolStats& st) {
   v.has_support = true;
-  if (box[3] < box[0]) {  // no non-zero voxel
-    for (int k = 0; k < 3; ++k) { v.sup_lo[k] = 1.0f; v.sup_hi[k] = 0.0f; }
-  } else {
-    for (int k = 0; k < 3; ++k) {
-      v.sup_lo[k] = (float)box[k] - 1.5f;
-      v.sup_hi[k] = (float)box[3 + k] + 1.5f;
-    }
+  for (int k = 0; k < 3; ++k) {
+    v.sup_lo[k] = st.hi[0] == 0 ? 1.0f : (float)(0x7fffffff - (int)st.lo[k]) - 1.5f;  // no non-zero voxel: lo > hi
+    v.sup_hi[k] = st.hi[0] == 0 ? 0.0f : (float)((int)st.hi[k] - 1) + 1.5f;
   }
-  return XR_OK;
 }
+
+static int32_t macro_cells(int64_t n) { return (int32_t)(((n - 1) + (1 << kMacroShift) - 1) >> kMacroShift); }
 
 static xr_status rc_set_volumes_impl(xr_raycaster rc, int32_t n, const xr_volume_desc* descs,
                                      const float* const* voxels, int32_t vt, float scale, bool on_device) {
@@ -477,32 +448,32 @@ static xr_status rc_set_volumes_impl(xr_raycaster rc, int32_t n, const xr_volume
     XR_CHECK_ARG(d.spacing[0] > 0 && d.spacing[1] > 0 && d.spacing[2] > 0, "set_volumes: spacing must be > 0");
     XR_CHECK_ARG(finite_all(d.spacing, 3) && finite_all(d.origin, 3) && finite_all(d.direction, 9),
                  "set_volumes: non-finite geometry");
+    const int nx = (int)d.n[0], ny = (int)d.n[1], nz = (int)d.n[2];
     auto v = std::make_unique<xr_raycaster_s::Vol>();
     v->desc = d;
     v->type = vt;
+    v->nmx = macro_cells(d.n[0]);
+    v->nmy = macro_cells(d.n[1]);
+    v->nmz = macro_cells(d.n[2]);
     cell_strides(d.n[0], d.n[1], d.n[2], v->cs);
-    const size_t esz = vt == XR_VOXEL_F32 ? 4 : 2;
-    XR_CUDA_TRY(v->voxels.reserve((size_t)nv * esz));
+    const size_t vox_bytes = (size_t)nv * (vt == XR_VOXEL_F32 ? 4 : 2);
+    XR_CUDA_TRY(v->occ.reserve(((size_t)v->nmx * v->nmy * v->nmz + 31) / 32 * 4));
+    // float32 voxels on the device: the caller's, the volume's own copy, or a staging copy
     DevBuf tmp;
     const float* src = voxels[i];
-    if (vt == XR_VOXEL_F32) {
-      XR_CUDA_TRY(cudaMemcpyAsync(v->voxels.p, voxels[i], (size_t)nv * 4,
-                                  on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
-      src = v->voxels.as<float>();
-    } else if (!on_device) {
-      XR_CUDA_TRY(tmp.reserve((size_t)nv * 4));
-      XR_CUDA_TRY(cudaMemcpyAsync(tmp.p, voxels[i], (size_t)nv * 4, cudaMemcpyHostToDevice, s));
-      src = tmp.as<float>();
+    if (!on_device) {
+      DevBuf& to = vt == XR_VOXEL_F32 ? v->voxels : tmp;
+      XR_CUDA_TRY(to.reserve((size_t)nv * 4));
+      XR_CUDA_TRY(cudaMemcpyAsync(to.p, voxels[i], (size_t)nv * 4, cudaMemcpyHostToDevice, s));
+      src = to.as<float>();
     }
-    // largest magnitude (NaN left out)
-    XR_CUDA_TRY(cudaMemsetAsync(rc->d_counters.as<char>() + 16, 0, 4, s));
-    max_abs_kernel<<<1024, 256, 0, s>>>(src, nv, reinterpret_cast<unsigned int*>(rc->d_counters.as<char>() + 16));
-    XR_CUDA_TRY(cudaGetLastError());
-    unsigned int bits = 0;
-    XR_CUDA_TRY(cudaMemcpyAsync(&bits, rc->d_counters.as<char>() + 16, 4, cudaMemcpyDeviceToHost, s));
+    VolStats* d_stats = reinterpret_cast<VolStats*>(rc->d_counters.as<char>() + 16);
+    VolStats st;
+    XR_CUDA_TRY(launch_volume_stats(src, nx, ny, nz, v->occ.as<uint32_t>(), v->nmx, v->nmy, v->nmz, d_stats, s));
+    XR_CUDA_TRY(cudaMemcpyAsync(&st, d_stats, sizeof(st), cudaMemcpyDeviceToHost, s));
     XR_CUDA_TRY(cudaStreamSynchronize(s));
     float mx;
-    std::memcpy(&mx, &bits, 4);
+    std::memcpy(&mx, &st.max_bits, 4);
     float sc = scale > 0.0f ? scale : 1.0f;
     if (vt == XR_VOXEL_F32) {
       sc = 1.0f;
@@ -523,17 +494,45 @@ static xr_status rc_set_volumes_impl(xr_raycaster rc, int32_t n, const xr_volume
     // Differences of corners must be finite for the blends of float32 and BF16
     // volumes; a volume where they might not be is read as it lies (VolView::weighted).
     v->weighted = vt != XR_VOXEL_F16 && !(mx * sc <= 0x1p126f);
-    if (vt != XR_VOXEL_F32) {
-      convert_voxels_kernel<<<2048, 256, 0, s>>>(src, nv, sc, vt, v->voxels.p);
-      XR_CUDA_TRY(cudaGetLastError());
+    vol_support(*v, st);
+    const bool cells = rc->build_cells && !v->weighted;
+    const size_t cell_bytes = cells ? cell_layout_bytes(d.n[0], d.n[1], d.n[2], vt) : 0;
+    // One volume in place of one of the same or a larger size: its buffers are
+    // written over (allocating and freeing them took 1.4 ms of the 5.1 ms of
+    // setting a 512 x 512 x 300 FP16 volume).  Nothing can be refused from here on.
+    // Other streams may still read the old volume: freeing it would have waited
+    // for the device, and so does this.
+    if (n == 1 && rc->vols.size() == 1) {
+      xr_raycaster_s::Vol& old = *rc->vols[0];
+      const bool vox_fit = v->voxels.p || (old.voxels.p && old.voxels.bytes >= vox_bytes);
+      const bool cells_fit = !cells || (old.cells.p && old.cells.bytes >= cell_bytes);
+      // not when src lies in the buffers that would be written over, nor when the
+      // old ones are much larger
+      const char* q = reinterpret_cast<const char*>(src);
+      auto holds = [&](const DevBuf& b) { return b.p && q < static_cast<char*>(b.p) + b.bytes && q + nv * 4 > static_cast<char*>(b.p); };
+      if (vox_fit && cells_fit && !holds(old.voxels) && !holds(old.cells) &&
+          old.voxels.bytes + old.cells.bytes <= 2 * (vox_bytes + cell_bytes) + (size_t(1) << 20)) {
+        XR_CUDA_TRY(cudaDeviceSynchronize());
+        if (!v->voxels.p) v->voxels.swap(old.voxels);
+        if (cells) v->cells.swap(old.cells);
+        rc->vols.clear();  // the old volume is gone, also if a CUDA call below fails
+        rc->generation++;
+      }
     }
-    if (rc->build_cells && !v->weighted) {
-      XR_CUDA_TRY(v->cells.reserve(cell_layout_bytes(d.n[0], d.n[1], d.n[2], vt)));
-      XR_CUDA_TRY(launch_build_cells(src, (int)d.n[0], (int)d.n[1], (int)d.n[2], vt, sc, v->cells.p, s));
+    void* own_vox = nullptr;  // where the voxels still have to be written
+    if (!v->voxels.p || vt != XR_VOXEL_F32 || on_device) {
+      XR_CUDA_TRY(v->voxels.reserve(vox_bytes));
+      own_vox = v->voxels.p;
     }
-    xr_status st = vol_support(rc, *v, src, s);
-    if (st != XR_OK) return st;
-    XR_CUDA_TRY(cudaStreamSynchronize(s));  // tmp is released at scope exit
+    if (cells) {
+      XR_CUDA_TRY(v->cells.reserve(cell_bytes));
+      XR_CUDA_TRY(launch_build_cells(src, nx, ny, nz, vt, sc, v->cells.p, own_vox, s));
+    } else if (own_vox && vt == XR_VOXEL_F32) {
+      XR_CUDA_TRY(cudaMemcpyAsync(own_vox, src, vox_bytes, cudaMemcpyDeviceToDevice, s));
+    } else if (own_vox) {
+      XR_CUDA_TRY(launch_convert_voxels(src, nv, vt, sc, own_vox, s));
+    }
+    if (tmp.p) XR_CUDA_TRY(cudaStreamSynchronize(s));  // tmp is released at scope exit
     vols.push_back(std::move(v));
   }
   XR_CUDA_TRY(cudaStreamSynchronize(s));

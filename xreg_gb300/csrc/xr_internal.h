@@ -107,21 +107,34 @@ struct MultiJobDrr {
 // grouped: every job's pose_group is 4 (otherwise every job's is 0).
 cudaError_t launch_drr_jobs(const MultiJobDrr* d_jobs, int njobs, long long total_items, int32_t voxel_type,
                             int32_t layout, bool grouped, cudaStream_t s);
-// Macro-cell occupancy bitmask of a volume (see VolView::occ); d_occ holds
-// ceil(nmx * nmy * nmz / 32) words and is cleared here.
-cudaError_t launch_build_occupancy(const float* vox_f32, int nx, int ny, int nz, uint32_t* d_occ, int nmx, int nmy,
-                                   int nmz, cudaStream_t s);
-// Index bounds of the non-zero voxels into d_box[6] (min xyz, max xyz; max < min if none).
-cudaError_t launch_support_box(const float* vox_f32, int nx, int ny, int nz, int* d_box, cudaStream_t s);
-// Bytes of the CELL8 copy of a volume, and the kernel that builds it from
-// float32 voxels (cells numbered z fastest, then x, then y: VolView::cs).
+// Bytes of the CELL8 copy of a volume (cells numbered z fastest, then x, then y: VolView::cs).
 size_t cell_layout_bytes(int64_t nx, int64_t ny, int64_t nz, int32_t voxel_type);
-cudaError_t launch_build_cells(const float* vox_f32, int nx, int ny, int nz, int32_t voxel_type, float scale,
-                               void* out, cudaStream_t s);
 // The x and y cell strides of that order (VolView::cs).
 void cell_strides(int64_t nx, int64_t ny, int64_t nz, int32_t cs[2]);
 // VolView::kfl and cell_bytes of a volume; zeros in kfl where there are none.
 void cell_floor_constants(int64_t nx, int64_t ny, int64_t nz, int32_t voxel_type, float kfl[3], int32_t* bytes);
+
+// ---- launchers (xr_volume.cu) ----
+// HUToLinAtt of n values.
+cudaError_t launch_hu_to_mu(const float* hu, int64_t n, float* mu, cudaStream_t s);
+// Statistics of a volume's float32 voxels: the bits of the largest magnitude (NaN
+// left out) and the index bounds of the non-zero voxels, lo as 2^31 - 1 - min and
+// hi as max + 1 (0: none).
+struct VolStats {
+  unsigned int max_bits;
+  unsigned int lo[3], hi[3];
+};
+// Clears and fills the statistics and the macro-cell occupancy bitmask (see
+// VolView::occ; d_occ holds ceil(nmx * nmy * nmz / 32) words).
+cudaError_t launch_volume_stats(const float* vox_f32, int nx, int ny, int nz, uint32_t* d_occ, int nmx, int nmy, int nmz,
+                                VolStats* d_stats, cudaStream_t s);
+// The CELL8 copy from float32 voxels, scaled by `scale` for the 16-bit types, and,
+// unless out_vox is nullptr, the voxels in the volume's own type.
+cudaError_t launch_build_cells(const float* vox_f32, int nx, int ny, int nz, int32_t voxel_type, float scale,
+                               void* out, void* out_vox, cudaStream_t s);
+// The voxels in a 16-bit type alone.
+cudaError_t launch_convert_voxels(const float* vox_f32, int64_t n, int32_t voxel_type, float scale, void* out,
+                                  cudaStream_t s);
 
 // ---- launchers (xr_metrics.cu) ----
 struct FixedNCC {           // per direction (one for NCC, x and y for grad-NCC)

@@ -1,8 +1,6 @@
 // xr_preproc.cu -- data preparation either side of the hot path, on the device:
 //
-// * HU -> linear attenuation (HUToLinAttFilter::GenerateData,
-//   lib/image/xregHUToLinAtt.cpp:45-69): mu = max(hu * (mu_w - mu_a) 1e-3 + mu_w - mu_lower, 0)
-//   in double, stored as float; mu_w = 0.02683, mu_a = 0.02485e-4 /mm, hu_lower = -1000.
+// * HU -> linear attenuation (the kernel is in xr_volume.cu).
 // * Fixed-image downsampling for a coarser registration level (DownsampleProjData
 //   -> DownsampleImage, lib/image/xregProjData.cpp:40-53,
 //   lib/itk/xregITKResampleUtils.h:51-131,183-187): for factor < 1, a discrete
@@ -37,16 +35,6 @@
 
 namespace xr {
 namespace {
-
-__global__ void hu_to_mu_kernel(const float* __restrict__ hu, int64_t n, float* __restrict__ mu) {
-  const double mu_w = 0.02683 * 1.0, mu_a = 0.02485 * 0.0001, hu_lower = -1000.0;
-  const double hu_scale = (mu_w - mu_a) * 1.0e-3;
-  const double mu_lower = (hu_lower * hu_scale) + mu_w;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = ((double)hu[i] * hu_scale) + mu_w - mu_lower;
-    mu[i] = (float)(v > 0.0 ? v : 0.0);
-  }
-}
 
 constexpr int kMaxTaps = 32;
 
@@ -218,9 +206,7 @@ using namespace xr;
 extern "C" XR_API xr_status xr_hu_to_lin_att(const float* d_hu, int64_t n, float* d_mu, void* stream) {
   if (!d_hu || !d_mu || n < 0) return fail(XR_ERR_INVALID_ARG, "xr_hu_to_lin_att: bad argument");
   if (n == 0) return XR_OK;
-  hu_to_mu_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 8192), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      d_hu, n, d_mu);
-  XR_CUDA_TRY(cudaGetLastError());
+  XR_CUDA_TRY(launch_hu_to_mu(d_hu, n, d_mu, static_cast<cudaStream_t>(stream)));
   return XR_OK;
 }
 

@@ -1317,45 +1317,6 @@ cudaError_t launch_kernel_id(const DrrParams& p, cudaStream_t s) {
                                         : launch_layout<VT, XR_LINE_INT_SUM>(p, s);
 }
 
-// One thread per cell (x fastest, so the voxel reads coalesce): gathers the 8
-// corners from the float32 voxels (indices clamped to the volume) and stores
-// them as cell number (ix + 1) csx + (iy + 1) csy + iz + 1 (z fastest).
-template <int VT>
-__global__ void build_cells_kernel(const float* __restrict__ vox, int nx, int ny, int nz, float scale, int32_t csx,
-                                   int32_t csy, void* out) {
-  const int64_t ncx = nx + 1, ncy = ny + 1, ncz = nz + 1;
-  const int64_t ncell = ncx * ncy * ncz;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ncell; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t ix = t % ncx, iy = (t / ncx) % ncy, iz = t / (ncx * ncy);  // index + 1
-    const int64_t c = ix * csx + iy * csy + iz;
-    const int64_t x0 = ix > 0 ? ix - 1 : 0, y0 = iy > 0 ? iy - 1 : 0, z0 = iz > 0 ? iz - 1 : 0;
-    const int64_t b = (z0 * ny + y0) * nx + x0;
-    const int64_t sx = min(ix, (int64_t)nx - 1) - x0, sy = (min(iy, (int64_t)ny - 1) - y0) * nx,
-                  sz = (min(iz, (int64_t)nz - 1) - z0) * nx * ny;
-    // z-pairs: v000 v001 v100 v101 v010 v011 v110 v111 (vxyz)
-    const float v[8] = {vox[b], vox[b + sz], vox[b + sx], vox[b + sz + sx],
-                        vox[b + sy], vox[b + sz + sy], vox[b + sy + sx], vox[b + sz + sy + sx]};
-    if (VT == XR_VOXEL_F32) {
-      float4* o = static_cast<float4*>(out) + 2 * c;
-      o[0] = make_float4(v[0], v[1], __fsub_rn(v[2], v[0]), __fsub_rn(v[3], v[1]));
-      o[1] = make_float4(v[4], v[5], __fsub_rn(v[6], v[4]), __fsub_rn(v[7], v[5]));
-    } else {
-      uint4 q;
-      unsigned int* w = &q.x;
-      for (int k = 0; k < 4; ++k) {
-        if (VT == XR_VOXEL_F16) {
-          __half2 h = __floats2half2_rn(v[2 * k] * scale, v[2 * k + 1] * scale);
-          w[k] = *reinterpret_cast<unsigned int*>(&h);
-        } else {
-          __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * k] * scale, v[2 * k + 1] * scale);
-          w[k] = *reinterpret_cast<unsigned int*>(&h);
-        }
-      }
-      static_cast<uint4*>(out)[c] = q;
-    }
-  }
-}
-
 }  // namespace
 
 cudaError_t launch_brick(const DrrParams& p, cudaStream_t s) {
@@ -1391,75 +1352,6 @@ cudaError_t launch_drr(const DrrParams& p, cudaStream_t s) {
     case XR_VOXEL_BF16: return launch_kernel_id<XR_VOXEL_BF16>(p, s);
     default: return cudaErrorInvalidValue;
   }
-}
-
-// Marks macro cell m occupied when any trilinear cell in it has a non-zero
-// corner: voxel (x, y, z) is a corner of cells x-1..x, y-1..y, z-1..z.
-// Dilated macro-cell occupancy: bit m is set when some trilinear cell with base
-// index in [8m - 1, 8m + 8] on every axis has a non-zero corner, i.e. some
-// non-zero voxel lies in [8m - 1, 8m + 9].
-__global__ void occupancy_kernel(const float* __restrict__ vox, int nx, int ny, int nz, uint32_t* occ, int nmx,
-                                 int nmy, int nmz) {
-  const int64_t n = (int64_t)nx * ny * nz;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    if (vox[i] == 0.0f) continue;
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((int64_t)nx * ny));
-    const int x0 = max(x - 2, 0) >> kMacroShift, x1 = min((x + 1) >> kMacroShift, nmx - 1);
-    const int y0 = max(y - 2, 0) >> kMacroShift, y1 = min((y + 1) >> kMacroShift, nmy - 1);
-    const int z0 = max(z - 2, 0) >> kMacroShift, z1 = min((z + 1) >> kMacroShift, nmz - 1);
-    for (int mz = z0; mz <= z1; ++mz)
-      for (int my = y0; my <= y1; ++my)
-        for (int mx = x0; mx <= x1; ++mx) {
-          const int m = (mz * nmy + my) * nmx + mx;
-          const uint32_t bit = 1u << (m & 31);
-          if (!(occ[m >> 5] & bit)) atomicOr(&occ[m >> 5], bit);
-        }
-  }
-}
-
-__global__ void support_init_kernel(int* box) {
-  if (threadIdx.x < 3) box[threadIdx.x] = 0x7fffffff;
-  else if (threadIdx.x < 6) box[threadIdx.x] = -1;
-}
-
-// Index bounds of the non-zero voxels: box = (min x, min y, min z, max x, max y, max z).
-__global__ void support_box_kernel(const float* __restrict__ vox, int nx, int ny, int nz, int* box) {
-  int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, mx[3] = {-1, -1, -1};
-  const int64_t n = (int64_t)nx * ny * nz;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    if (vox[i] != 0.0f) {
-      const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((int64_t)nx * ny));
-      mn[0] = min(mn[0], x); mn[1] = min(mn[1], y); mn[2] = min(mn[2], z);
-      mx[0] = max(mx[0], x); mx[1] = max(mx[1], y); mx[2] = max(mx[2], z);
-    }
-  }
-  for (int k = 0; k < 3; ++k) {
-    for (int o = 16; o > 0; o >>= 1) {
-      mn[k] = min(mn[k], __shfl_down_sync(0xffffffffu, mn[k], o));
-      mx[k] = max(mx[k], __shfl_down_sync(0xffffffffu, mx[k], o));
-    }
-  }
-  if ((threadIdx.x & 31) == 0) {
-    for (int k = 0; k < 3; ++k) {
-      atomicMin(&box[k], mn[k]);
-      atomicMax(&box[3 + k], mx[k]);
-    }
-  }
-}
-
-cudaError_t launch_build_occupancy(const float* vox_f32, int nx, int ny, int nz, uint32_t* d_occ, int nmx, int nmy,
-                                   int nmz, cudaStream_t s) {
-  const size_t words = ((size_t)nmx * nmy * nmz + 31) / 32;
-  cudaError_t e = cudaMemsetAsync(d_occ, 0, words * sizeof(uint32_t), s);
-  if (e != cudaSuccess) return e;
-  occupancy_kernel<<<2048, 256, 0, s>>>(vox_f32, nx, ny, nz, d_occ, nmx, nmy, nmz);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_support_box(const float* vox_f32, int nx, int ny, int nz, int* d_box, cudaStream_t s) {
-  support_init_kernel<<<1, 32, 0, s>>>(d_box);
-  support_box_kernel<<<2048, 256, 0, s>>>(vox_f32, nx, ny, nz, d_box);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_eval_fused(const FusedJob* d_jobs, int njobs, long long total, int32_t voxel_type, int32_t layout,
@@ -1502,25 +1394,6 @@ size_t cell_layout_bytes(int64_t nx, int64_t ny, int64_t nz, int32_t voxel_type)
   cell_strides(nx, ny, nz, cs);
   const size_t ncell = (size_t)cs[1] * (size_t)(ny + 1);
   return ncell * (voxel_type == XR_VOXEL_F32 ? 32 : 16);
-}
-
-cudaError_t launch_build_cells(const float* vox_f32, int nx, int ny, int nz, int32_t voxel_type, float scale,
-                               void* out, cudaStream_t s) {
-  int32_t cs[2];
-  cell_strides(nx, ny, nz, cs);
-  switch (voxel_type) {
-    case XR_VOXEL_F32:
-      build_cells_kernel<XR_VOXEL_F32><<<2048, 256, 0, s>>>(vox_f32, nx, ny, nz, 1.0f, cs[0], cs[1], out);
-      break;
-    case XR_VOXEL_F16:
-      build_cells_kernel<XR_VOXEL_F16><<<2048, 256, 0, s>>>(vox_f32, nx, ny, nz, scale, cs[0], cs[1], out);
-      break;
-    case XR_VOXEL_BF16:
-      build_cells_kernel<XR_VOXEL_BF16><<<2048, 256, 0, s>>>(vox_f32, nx, ny, nz, scale, cs[0], cs[1], out);
-      break;
-    default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
 }
 
 // Strides of 2 modulo 8.  The L1 serves a cell load in passes of 4 lanes
