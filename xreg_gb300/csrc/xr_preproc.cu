@@ -28,6 +28,13 @@
 // taken out from the centre until its two-sided sum reaches 1 - max_error and
 // normalised to sum 1 — the construction ITK's GaussianOperator follows.  Here
 // I_k is summed from its power series in double.
+//
+// The smoothing and the spline run in float-float (about 48 bits) instead of
+// double: this GPU issues one double instruction per 64 cycles and scheduler, and
+// its results are rounded to float.  Values that float-float cannot carry
+// (infinities, NaN, magnitudes near the end of float's range) take the double
+// operations.
+#include "xr_gradtile.cuh"
 #include "xr_internal.h"
 
 #include <cmath>
@@ -37,13 +44,103 @@ namespace xr {
 namespace {
 
 constexpr int kMaxTaps = 32;
+using gt::FF;
 
 struct GaussKernel {
   int radius;
   double c[kMaxTaps + 1];
+  float hi[kMaxTaps + 1], lo[kMaxTaps + 1];  // c = hi + lo
 };
 
-// Separable pass along x (dir 0) or y (dir 1), edges replicated.
+__device__ __forceinline__ FF two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  return FF{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ FF renorm(float hi, float lo) {
+  const float s = __fadd_rn(hi, lo);
+  return FF{s, __fsub_rn(lo, __fsub_rn(s, hi))};
+}
+__device__ __forceinline__ FF ff_mul(FF a, FF b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  return renorm(p, __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.hi, b.hi, -p))));
+}
+__device__ __forceinline__ FF ff_sum(FF a, FF b) {
+  const FF s = two_sum(a.hi, b.hi);
+  return renorm(s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)));
+}
+__device__ __forceinline__ FF ff_of(double v) {
+  const float hi = (float)v;
+  return FF{hi, (float)(v - (double)hi)};
+}
+__device__ __forceinline__ FF ff_of(float v) { return FF{v, 0.0f}; }
+__device__ __forceinline__ FF ff_of(float2 v) { return FF{v.x, v.y}; }
+__device__ __forceinline__ double value(float v) { return (double)v; }
+__device__ __forceinline__ double value(float2 v) { return (double)v.x + (isfinite(v.x) ? (double)v.y : 0.0); }
+constexpr float kHuge = 1.0e37f;  // magnitudes above it are left to double
+
+// One pixel of the separable pass along x (dir 0) or y (dir 1), edges replicated,
+// in double.
+template <typename TIn>
+__device__ __noinline__ double gauss_at_double(const TIn* __restrict__ in, int rows, int cols, int r, int c, int dir,
+                                               const GaussKernel& k) {
+  double s = __dmul_rn(k.c[0], value(in[(int64_t)r * cols + c]));
+  for (int t = 1; t <= k.radius; ++t) {
+    const int64_t a = dir == 0 ? (int64_t)r * cols + max(c - t, 0) : (int64_t)max(r - t, 0) * cols + c;
+    const int64_t b = dir == 0 ? (int64_t)r * cols + min(c + t, cols - 1) : (int64_t)min(r + t, rows - 1) * cols + c;
+    s = __dadd_rn(s, __dmul_rn(k.c[t], __dadd_rn(value(in[a]), value(in[b]))));
+  }
+  return s;
+}
+
+// The same in float-float: c_t (a + b) with the sum and the product exact to about
+// 2^-47; a result that is not finite or not below kHuge is taken in double.
+template <typename TIn, int DIR>
+__device__ __forceinline__ FF gauss_at(const TIn* __restrict__ in, int rows, int cols, int r, int c,
+                                       const GaussKernel& k) {
+  const FF m = ff_of(in[(int64_t)r * cols + c]);
+  FF acc = ff_mul(m, FF{k.hi[0], k.lo[0]});
+#pragma unroll 4
+  for (int t = 1; t <= k.radius; ++t) {
+    const int64_t ia = DIR == 0 ? (int64_t)r * cols + max(c - t, 0) : (int64_t)max(r - t, 0) * cols + c;
+    const int64_t ib = DIR == 0 ? (int64_t)r * cols + min(c + t, cols - 1) : (int64_t)min(r + t, rows - 1) * cols + c;
+    const FF a = ff_of(in[ia]), b = ff_of(in[ib]);
+    const FF s = two_sum(a.hi, b.hi);
+    const float e = __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo));
+    const float p = __fmul_rn(s.hi, k.hi[t]);
+    const float pe = __fmaf_rn(e, k.hi[t], __fmaf_rn(s.hi, k.lo[t], __fmaf_rn(s.hi, k.hi[t], -p)));
+    const FF q = two_sum(acc.hi, p);
+    acc = FF{q.hi, __fadd_rn(acc.lo, __fadd_rn(q.lo, pe))};
+  }
+  acc = renorm(acc.hi, acc.lo);
+  if (fabsf(acc.hi) < kHuge && acc.lo == acc.lo) return acc;
+  return ff_of(gauss_at_double(in, rows, cols, r, c, DIR, k));
+}
+
+// Separable pass along x: float in, float-float out.
+__global__ void gauss_x_kernel(const float* __restrict__ in, int rows, int cols, const GaussKernel k,
+                               float2* __restrict__ out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+    const FF v = gauss_at<float, 0>(in, rows, cols, r, c, k);
+    out[(int64_t)r * cols + c] = make_float2(v.hi, isfinite(v.hi) ? v.lo : 0.0f);
+  }
+}
+
+// Pass along y, rounded to the float image type; *beyond is set when a value is not
+// finite or not below kHuge.
+__global__ void gauss_y_kernel(const float2* __restrict__ in, int rows, int cols, const GaussKernel k,
+                               float* __restrict__ out, int* __restrict__ beyond) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+    const float v = gauss_at<float2, 1>(in, rows, cols, r, c, k).hi;
+    out[(int64_t)r * cols + c] = v;
+    if (!(fabsf(v) < kHuge)) *beyond = 1;
+  }
+}
+
+// The passes in double, for images that spline_kernel does not take.
 template <typename TIn>
 __global__ void gauss_pass_kernel(const TIn* __restrict__ in, int rows, int cols, int dir, GaussKernel k,
                                   double* __restrict__ out) {
@@ -78,14 +175,10 @@ __global__ void widen_kernel(const float* __restrict__ in, int64_t n, double* __
     out[i] = (double)in[i];
 }
 
-// Cubic B-spline prefilter of `count` lines of `len` samples in place: line l
-// starts at c + l * line_stride, samples `stride` apart.  One thread per line.
+// Cubic B-spline prefilter of a line of `len` samples, `stride` apart, in place.
 // z = the pole, gain = (1 - z)(1 - 1/z), horizon = terms of the causal start.
-__global__ void bspline_prefilter_kernel(double* __restrict__ c, int count, int len, int64_t line_stride,
-                                         int64_t stride, double z, double gain, int horizon) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= count || len < 2) return;
-  double* v = c + (int64_t)l * line_stride;
+__device__ void bspline_prefilter_line(double* __restrict__ v, int len, int64_t stride, double z, double gain,
+                                       int horizon) {
   for (int n = 0; n < len; ++n) v[n * stride] = __dmul_rn(v[n * stride], gain);
   // causal initialisation (mirror boundaries)
   {
@@ -119,6 +212,13 @@ __global__ void bspline_prefilter_kernel(double* __restrict__ c, int count, int 
   for (int n = len - 2; n >= 0; --n) v[n * stride] = __dmul_rn(z, __dsub_rn(v[(n + 1) * stride], v[n * stride]));
 }
 
+// `count` lines, line l at c + l * line_stride; one thread per line.
+__global__ void bspline_prefilter_kernel(double* __restrict__ c, int count, int len, int64_t line_stride,
+                                         int64_t stride, double z, double gain, int horizon) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l < count && len >= 2) bspline_prefilter_line(c + (int64_t)l * line_stride, len, stride, z, gain, horizon);
+}
+
 __device__ __forceinline__ int mirror_index(int k, int n) {
   if (n == 1) return 0;
   if (k < 0) k = -k;
@@ -134,11 +234,12 @@ __device__ __forceinline__ void cubic_weights(double x, int i1, double w[4]) {
   w[1] = __dsub_rn(__dsub_rn(__dsub_rn(1.0, w[0]), w[2]), w[3]);
 }
 
-// Output pixel (r, c) = cubic B-spline of the coefficients at (c / factor, r / factor).
-__global__ void bspline_resample_kernel(const double* __restrict__ coef, int rows, int cols, double factor,
-                                        int orows, int ocols, float* __restrict__ out) {
+// Output pixels i0, i0 + step, ...: pixel (r, c) = cubic B-spline of the coefficients
+// at (c / factor, r / factor).
+__device__ void bspline_resample(const double* __restrict__ coef, int rows, int cols, double factor, int orows,
+                                 int ocols, int64_t i0, int64_t step, float* __restrict__ out) {
   const int64_t n = (int64_t)orows * ocols;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = i0; i < n; i += step) {
     const int r = (int)(i / ocols), c = (int)(i - (int64_t)r * ocols);
     const double x = __ddiv_rn((double)c, factor), y = __ddiv_rn((double)r, factor);
     if (!(x >= -0.5 && x < cols - 0.5 && y >= -0.5 && y < rows - 0.5)) { out[i] = 0.0f; continue; }
@@ -159,6 +260,157 @@ __global__ void bspline_resample_kernel(const double* __restrict__ coef, int row
       for (int a = 0; a < 4; ++a)
         acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(wx[a], wy[b]), coef[(int64_t)iy[b] * cols + ix[a]]));
     out[i] = (float)acc;
+  }
+}
+
+__global__ void bspline_resample_kernel(const double* __restrict__ coef, int rows, int cols, double factor,
+                                        int orows, int ocols, float* __restrict__ out) {
+  bspline_resample(coef, rows, cols, factor, orows, ocols, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                   (int64_t)gridDim.x * blockDim.x, out);
+}
+
+// The whole spline in double by one block, for an image with values that
+// float-float does not carry (*beyond); otherwise it returns at once.
+__global__ void __launch_bounds__(1024) spline_double_kernel(const float* __restrict__ img, int rows, int cols,
+                                                             double factor, int orows, int ocols, double z,
+                                                             double gain, int horizon, const int* __restrict__ beyond,
+                                                             double* __restrict__ coef, float* __restrict__ out) {
+  if (!*beyond) return;
+  for (int64_t i = threadIdx.x; i < (int64_t)rows * cols; i += blockDim.x) coef[i] = (double)img[i];
+  __syncthreads();
+  for (int r = threadIdx.x; r < rows; r += blockDim.x)
+    bspline_prefilter_line(coef + (int64_t)r * cols, cols, 1, z, gain, horizon);
+  __syncthreads();
+  for (int c = threadIdx.x; c < cols; c += blockDim.x) bspline_prefilter_line(coef + c, rows, cols, z, gain, horizon);
+  __syncthreads();
+  bspline_resample(coef, rows, cols, factor, orows, ocols, threadIdx.x, blockDim.x, out);
+}
+
+// The spline along one axis, prefilter and interpolation together, in float-float:
+// `lines` lines of `len` contiguous samples in, out[j][line] (transposed, so that
+// the same kernel takes the other axis next) = the spline at j / factor.
+// The recursions decay by |z| = 0.27 a sample, so a line is cut into chunks that
+// start kWarm samples early from zero (0.27^28 = 1e-16): a warp takes 32 lines by
+// one chunk, its samples and coefficients in shared memory (33-word pitch: lanes
+// along samples or along lines meet no bank conflicts).  One thread per line in
+// double took 864 us along the rows of a 1436 x 1436 image and 1406 along its
+// columns, one chain of dependent double operations each; the two passes of this
+// kernel take 27 and 15 (quarter-size output).
+constexpr int kChunk = 64, kWarm = 28;
+constexpr int kSpan = kChunk + 3 + 2 * kWarm;  // coefficients -1 .. kChunk + 1 and both warm-ups
+constexpr int kOuts = kChunk + 8;              // candidate outputs of a chunk (factor < 1), with room for rounding
+
+template <typename TIn, typename TOut>
+__global__ void __launch_bounds__(32) spline_kernel(const TIn* __restrict__ in, int lines, int len, double factor,
+                                                    int outs, double z_d, double gain_d, int horizon,
+                                                    const int* __restrict__ beyond, TOut* __restrict__ out) {
+  __shared__ float hi[kSpan][33], lo[kSpan][33];
+  __shared__ FF w[kOuts][4];
+  __shared__ int first[kOuts];  // index of an output's second coefficient, -1: outside the image
+  if (*beyond) return;
+  const int lane = threadIdx.x, l0 = blockIdx.y * 32;
+  const int start = blockIdx.x * kChunk;  // this chunk's outputs have floor(position) in [start, start + kChunk)
+  const int k0 = max(start - 1 - kWarm, 0), k1 = min(start + kChunk + 2 + kWarm, len);
+  for (int k = k0 + lane; k < k1; k += 32) {
+#pragma unroll
+    for (int r = 0; r < 32; r += 16) {  // 16 loads in flight
+      TIn v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = in[(int64_t)min(l0 + r + i, lines - 1) * len + k];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const FF f = ff_of(v[i]);
+        hi[k - k0][r + i] = f.hi;
+        lo[k - k0][r + i] = f.lo;
+      }
+    }
+  }
+  // outputs of this chunk and their weights, one output per lane at a time
+  const bool tail = start + kChunk >= len;  // positions past the last sample belong to the last chunk
+  const int jb = max((int)((float)start * (float)factor) - 2, 0);
+  const int je = tail ? outs : min(outs, (int)((float)(start + kChunk) * (float)factor) + 3);
+  int j0 = outs, j1 = 0;
+  for (int j = jb + lane; j < je; j += 32) {
+    const double x = __ddiv_rn((double)j, factor);
+    const int x1 = (int)floorf((float)x);
+    if (x1 < start || (x1 >= start + kChunk && !tail)) continue;
+    j0 = min(j0, j);
+    j1 = max(j1, j + 1);
+    double wd[4];
+    cubic_weights(x, x1, wd);
+    for (int a = 0; a < 4; ++a) w[j - jb][a] = ff_of(wd[a]);
+    first[j - jb] = x < len - 0.5 ? x1 : -1;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    j0 = min(j0, __shfl_xor_sync(0xffffffffu, j0, o));
+    j1 = max(j1, __shfl_xor_sync(0xffffffffu, j1, o));
+  }
+  __syncwarp();
+  // causal, then anti-causal recursion of this lane's line
+  const FF z = ff_of(z_d), gain = ff_of(gain_d);
+  const int n = k1 - k0;
+  FF c{0.0f, 0.0f};
+  int k = 0;
+  if (k0 == 0) {  // the line's own start (mirror boundary), summed to the horizon
+    FF zn = z;
+    c = ff_mul(FF{hi[0][lane], lo[0][lane]}, gain);
+    for (int i = 1; i < horizon; ++i) {
+      c = ff_sum(c, ff_mul(zn, ff_mul(FF{hi[i][lane], lo[i][lane]}, gain)));
+      zn = ff_mul(zn, z);
+    }
+    hi[0][lane] = c.hi;
+    lo[0][lane] = c.lo;
+    k = 1;
+  }
+  // c = gain s[k] + z c: hi + lo without renormalising (lo stays below an ulp or
+  // two of hi, the recursion contracts), so that a step's dependent chain is one
+  // product and one sum; the next sample is read before this one is stored
+  FF v = ff_mul(FF{hi[k][lane], lo[k][lane]}, gain);
+  for (; k < n; ++k) {
+    const FF nx{hi[min(k + 1, n - 1)][lane], lo[min(k + 1, n - 1)][lane]};
+    const float q = __fmul_rn(z.hi, c.hi);
+    const float qe = __fmaf_rn(z.hi, c.lo, __fmaf_rn(z.lo, c.hi, __fmaf_rn(z.hi, c.hi, -q)));
+    c = two_sum(v.hi, q);
+    c.lo = __fadd_rn(c.lo, __fadd_rn(qe, v.lo));
+    hi[k][lane] = c.hi;
+    lo[k][lane] = c.lo;
+    v = ff_mul(nx, gain);
+  }
+  k = n - 1;
+  if (k1 == len) {  // the line's own end
+    const FF b{hi[n - 2][lane], lo[n - 2][lane]};
+    c = ff_mul(ff_of(__ddiv_rn(z_d, __dsub_rn(__dmul_rn(z_d, z_d), 1.0))), ff_sum(ff_mul(z, b), c));
+    hi[k][lane] = c.hi;
+    lo[k][lane] = c.lo;
+    --k;
+  } else {
+    c = FF{0.0f, 0.0f};
+  }
+  const int kl = max(start - 2, 0) - k0;  // a mirrored index reaches start - 2
+  v = FF{hi[k][lane], lo[k][lane]};
+  for (; k >= kl; --k) {  // c = z (c - c+[k])
+    const FF nx{hi[max(k - 1, 0)][lane], lo[max(k - 1, 0)][lane]};
+    FF d = two_sum(c.hi, -v.hi);
+    d.lo = __fadd_rn(d.lo, __fsub_rn(c.lo, v.lo));
+    c.hi = __fmul_rn(z.hi, d.hi);
+    c.lo = __fmaf_rn(z.hi, d.lo, __fmaf_rn(z.lo, d.hi, __fmaf_rn(z.hi, d.hi, -c.hi)));
+    hi[k][lane] = c.hi;
+    lo[k][lane] = c.lo;
+    v = nx;
+  }
+  if (l0 + lane >= lines) return;
+  for (int j = j0; j < j1; ++j) {
+    v = FF{0.0f, 0.0f};
+    const int x1 = first[j - jb];
+    if (x1 >= 0) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const int i = mirror_index(x1 - 1 + a, len) - k0;
+        v = ff_sum(v, ff_mul(w[j - jb][a], FF{hi[i][lane], lo[i][lane]}));
+      }
+    }
+    if constexpr (sizeof(TOut) == sizeof(float2)) out[(int64_t)j * lines + l0 + lane] = make_float2(v.hi, v.lo);
+    else out[(int64_t)j * lines + l0 + lane] = v.hi;
   }
 }
 
@@ -220,18 +472,36 @@ extern "C" XR_API xr_status xr_downsample_image_size(int64_t rows, int64_t cols,
   return XR_OK;
 }
 
+static GaussKernel gauss_kernel(double variance) {
+  GaussKernel k{};
+  k.radius = discrete_gaussian_taps(variance, 0.01, 32, k.c);
+  for (int t = 0; t <= k.radius; ++t) {
+    k.hi[t] = (float)k.c[t];
+    k.lo[t] = (float)(k.c[t] - (double)k.hi[t]);
+  }
+  return k;
+}
+
+static dim3 image_grid(int64_t rows, int64_t cols) {
+  return dim3((unsigned)((cols + 127) / 128), (unsigned)std::min<int64_t>(rows, 65535));
+}
+
 static unsigned grid_for(int64_t n) { return (unsigned)std::min<int64_t>((n + 255) / 256, 8192); }
+
+struct Spline {
+  double z = std::sqrt(3.0) - 2.0;
+  double gain = (1.0 - z) * (1.0 - 1.0 / z);
+  int horizon = (int)std::ceil(std::log(1.0e-10) / std::log(std::fabs(z)));
+};
 
 // Cubic B-spline coefficients of a rows x cols double image in place: along x
 // (one thread per row), then along y (one thread per column).
 static cudaError_t bspline_coefficients(double* c, int64_t rows, int64_t cols, cudaStream_t s) {
-  const double z = std::sqrt(3.0) - 2.0;
-  const double gain = (1.0 - z) * (1.0 - 1.0 / z);
-  const int horizon = (int)std::ceil(std::log(1.0e-10) / std::log(std::fabs(z)));
-  bspline_prefilter_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, s>>>(c, (int)rows, (int)cols, cols, 1, z, gain,
-                                                                          horizon);
-  bspline_prefilter_kernel<<<(unsigned)((cols + 127) / 128), 128, 0, s>>>(c, (int)cols, (int)rows, 1, cols, z, gain,
-                                                                          horizon);
+  const Spline p;
+  bspline_prefilter_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, s>>>(c, (int)rows, (int)cols, cols, 1, p.z, p.gain,
+                                                                          p.horizon);
+  bspline_prefilter_kernel<<<(unsigned)((cols + 127) / 128), 128, 0, s>>>(c, (int)cols, (int)rows, 1, cols, p.z, p.gain,
+                                                                          p.horizon);
   return cudaGetLastError();
 }
 
@@ -246,10 +516,34 @@ extern "C" XR_API xr_status xr_downsample_image(const float* d_src, int64_t rows
   const int64_t n = rows * cols;
   double* a = d_scratch;
   double* b = d_scratch + n;
+  const double sigma = 0.5 / factor;
+  // Chunked float-float passes where a line has a chunk's samples and the output is
+  // smaller on both axes (their buffers share the scratch: smoothed floats, then a
+  // flag, in the second half; the row pass's output over the first).  Otherwise,
+  // small or hardly reduced images, the double kernels.
+  if (factor < 1.0 && rows >= kChunk && cols >= kChunk && orows < rows && ocols < cols) {
+    const GaussKernel k = gauss_kernel(sigma * sigma);
+    const Spline p;
+    float2* x_out = reinterpret_cast<float2*>(a);  // smoothed along x, then the spline along x [ocols][rows]
+    float* smooth = reinterpret_cast<float*>(b);
+    int* beyond = reinterpret_cast<int*>(smooth + n);
+    XR_CUDA_TRY(cudaMemsetAsync(beyond, 0, sizeof(int), s));
+    gauss_x_kernel<<<image_grid(rows, cols), 128, 0, s>>>(d_src, (int)rows, (int)cols, k, x_out);
+    gauss_y_kernel<<<image_grid(rows, cols), 128, 0, s>>>(x_out, (int)rows, (int)cols, k, smooth, beyond);
+    auto grid = [](int64_t len, int64_t lines) {
+      return dim3((unsigned)((len + kChunk - 1) / kChunk), (unsigned)((lines + 31) / 32));
+    };
+    spline_kernel<float, float2><<<grid(cols, rows), 32, 0, s>>>(smooth, (int)rows, (int)cols, factor, (int)ocols, p.z,
+                                                                 p.gain, p.horizon, beyond, x_out);
+    spline_kernel<float2, float><<<grid(rows, ocols), 32, 0, s>>>(x_out, (int)ocols, (int)rows, factor, (int)orows, p.z,
+                                                                  p.gain, p.horizon, beyond, d_dst);
+    spline_double_kernel<<<1, 1024, 0, s>>>(smooth, (int)rows, (int)cols, factor, (int)orows, (int)ocols, p.z, p.gain,
+                                            p.horizon, beyond, a, d_dst);
+    XR_CUDA_TRY(cudaGetLastError());
+    return XR_OK;
+  }
   if (factor < 1.0) {
-    GaussKernel k{};
-    const double sigma = 0.5 / factor;
-    k.radius = discrete_gaussian_taps(sigma * sigma, 0.01, 32, k.c);
+    const GaussKernel k = gauss_kernel(sigma * sigma);
     gauss_pass_kernel<float><<<grid_for(n), 256, 0, s>>>(d_src, (int)rows, (int)cols, 0, k, a);
     gauss_pass_kernel<double><<<grid_for(n), 256, 0, s>>>(a, (int)rows, (int)cols, 1, k, b);
     round_to_float_kernel<<<grid_for(n), 256, 0, s>>>(b, n);
@@ -292,34 +586,27 @@ namespace {
 
 __global__ void crop_kernel(const float* __restrict__ in, int cols, int width, int orows, int ocols,
                             float* __restrict__ out) {
-  const int64_t n = (int64_t)orows * ocols;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(i / ocols), c = (int)(i - (int64_t)r * ocols);
-    out[i] = in[(int64_t)(r + width) * cols + (c + width)];
-  }
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ocols) return;
+  for (int r = blockIdx.y; r < orows; r += gridDim.y)
+    out[(int64_t)r * ocols + c] = in[(int64_t)(r + width) * cols + (c + width)];
 }
 
-constexpr int kRedBlocks = 512;
+constexpr int kRedBlocks = 1024;  // partials of the statistics (the scratch holds as many)
 constexpr float kLogEps = 1.0e-6f;
 
 // Second Gaussian pass (along y) rounded to float, reduced to its maximum, and
 // the smallest source value above 1e-6; per-block partials.
-__global__ void log_remap_stats_kernel(const double* __restrict__ a, const float* __restrict__ src, int rows,
-                                       int cols, GaussKernel k, float* __restrict__ part_max,
+__global__ void log_remap_stats_kernel(const float2* __restrict__ a, const float* __restrict__ src, int rows,
+                                       int cols, const GaussKernel k, float* __restrict__ part_max,
                                        float* __restrict__ part_min) {
-  const int64_t n = (int64_t)rows * cols;
   float mx = -INFINITY, mn = INFINITY;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(i / cols), c = (int)(i - (int64_t)r * cols);
-    double s = __dmul_rn(k.c[0], a[i]);
-    for (int t = 1; t <= k.radius; ++t) {
-      const int lo = max(r - t, 0), hi = min(r + t, rows - 1);
-      s = __dadd_rn(s, __dmul_rn(k.c[t], __dadd_rn(a[(int64_t)lo * cols + c], a[(int64_t)hi * cols + c])));
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += gridDim.x * blockDim.x)
+    for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+      mx = fmaxf(mx, gauss_at<float2, 1>(a, rows, cols, r, c, k).hi);
+      const float x = src[(int64_t)r * cols + c];
+      if (x > kLogEps) mn = fminf(mn, x);
     }
-    mx = fmaxf(mx, (float)s);
-    const float x = src[i];
-    if (x > kLogEps) mn = fminf(mn, x);
-  }
   __shared__ float smx[32], smn[32];
   for (int o = 16; o > 0; o >>= 1) {
     mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, o));
@@ -330,17 +617,21 @@ __global__ void log_remap_stats_kernel(const double* __restrict__ a, const float
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int j = 1; j < (int)(blockDim.x >> 5); ++j) { mx = fmaxf(mx, smx[j]); mn = fminf(mn, smn[j]); }
-    part_max[blockIdx.x] = mx;
-    part_min[blockIdx.x] = mn;
+    part_max[blockIdx.y * gridDim.x + blockIdx.x] = mx;
+    part_min[blockIdx.y * gridDim.x + blockIdx.x] = mn;
   }
 }
 
 // scal[0] = I0, scal[1] = -log(min_pos / I0) (min_pos 0 when no value exceeds 1e-6).
 __global__ void log_remap_finalize_kernel(const float* __restrict__ part_max, const float* __restrict__ part_min,
                                           int nblk, int use_max, float i0, float* __restrict__ scal) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   float mx = -INFINITY, mn = INFINITY;
-  for (int j = 0; j < nblk; ++j) { mx = fmaxf(mx, part_max[j]); mn = fminf(mn, part_min[j]); }
+  for (int j = threadIdx.x; j < nblk; j += 32) { mx = fmaxf(mx, part_max[j]); mn = fminf(mn, part_min[j]); }
+  for (int o = 16; o > 0; o >>= 1) {
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+  }
+  if (threadIdx.x != 0) return;
   const float I0 = use_max ? mx : i0;
   const float min_pos = (mn == INFINITY) ? 0.0f : mn;
   scal[0] = I0;
@@ -365,7 +656,7 @@ extern "C" XR_API xr_status xr_crop_image_boundary(const float* d_src, int64_t r
   if (width < 0 || rows - 2 * width < 1 || cols - 2 * width < 1 || rows > (1 << 30) || cols > (1 << 30))
     return fail(XR_ERR_INVALID_ARG, "xr_crop_image_boundary: the crop leaves no pixels");
   const int64_t orows = rows - 2 * width, ocols = cols - 2 * width;
-  crop_kernel<<<grid_for(orows * ocols), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  crop_kernel<<<image_grid(orows, ocols), 128, 0, static_cast<cudaStream_t>(stream)>>>(
       d_src, (int)cols, (int)width, (int)orows, (int)ocols, d_dst);
   XR_CUDA_TRY(cudaGetLastError());
   return XR_OK;
@@ -379,15 +670,16 @@ extern "C" XR_API xr_status xr_log_remap(const float* d_src, int64_t rows, int64
   if (!use_max_as_i0 && !(i0 > 0.0f)) return fail(XR_ERR_INVALID_ARG, "xr_log_remap: I0 must be positive");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int64_t n = rows * cols;
-  double* a = d_scratch;
+  float2* a = reinterpret_cast<float2*>(d_scratch);
   float* part_max = reinterpret_cast<float*>(d_scratch + n);
   float* part_min = part_max + kRedBlocks;
   float* scal = part_min + kRedBlocks;
-  GaussKernel k{};
-  k.radius = discrete_gaussian_taps(2.0, 0.01, 32, k.c);
-  gauss_pass_kernel<float><<<grid_for(n), 256, 0, s>>>(d_src, (int)rows, (int)cols, 0, k, a);
-  const int nblk = (int)std::min<int64_t>((n + 255) / 256, kRedBlocks);
-  log_remap_stats_kernel<<<nblk, 256, 0, s>>>(a, d_src, (int)rows, (int)cols, k, part_max, part_min);
+  const GaussKernel k = gauss_kernel(2.0);
+  gauss_x_kernel<<<image_grid(rows, cols), 128, 0, s>>>(d_src, (int)rows, (int)cols, k, a);
+  const unsigned bx = (unsigned)std::min<int64_t>((cols + 255) / 256, 64);
+  const dim3 grid(bx, (unsigned)std::min<int64_t>(rows, kRedBlocks / bx));
+  const int nblk = (int)(grid.x * grid.y);
+  log_remap_stats_kernel<<<grid, 256, 0, s>>>(a, d_src, (int)rows, (int)cols, k, part_max, part_min);
   log_remap_finalize_kernel<<<1, 32, 0, s>>>(part_max, part_min, nblk, use_max_as_i0, i0, scal);
   log_remap_kernel<<<grid_for(n), 256, 0, s>>>(d_src, n, scal, d_dst);
   XR_CUDA_TRY(cudaGetLastError());
