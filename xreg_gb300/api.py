@@ -739,33 +739,46 @@ def downsample_image(img: np.ndarray, factor: float, device: int = -1) -> np.nda
     return dst.cpu().numpy()
 
 
-def crop_image_boundary(img: np.ndarray, width: int, device: int = -1) -> np.ndarray:
-    """CropImage2DBoundary on the GPU (xr_crop_image_boundary)."""
+def _to_device(img: np.ndarray, device: int):
     import torch
     dev = torch.device("cuda", device if device >= 0 else torch.cuda.current_device())
-    src = torch.from_numpy(np.ascontiguousarray(img, dtype=np.float32)).to(dev)
+    return torch.from_numpy(np.ascontiguousarray(img, dtype=np.float32)).to(dev)
+
+
+def _to_host(t) -> np.ndarray:
+    return t.cpu().numpy()
+
+
+def _crop_tensor(src, width: int):
+    """xr_crop_image_boundary of a device image on the current stream."""
+    import torch
     rows, cols = src.shape
-    dst = torch.empty((max(rows - 2 * width, 0), max(cols - 2 * width, 0)), dtype=torch.float32, device=dev)
-    s = torch.cuda.current_stream(dev)
+    dst = torch.empty((max(rows - 2 * width, 0), max(cols - 2 * width, 0)), dtype=torch.float32, device=src.device)
     call("xr_crop_image_boundary", C.c_void_p(src.data_ptr()), rows, cols, int(width), C.c_void_p(dst.data_ptr()),
-         C.c_void_p(s.cuda_stream))
-    s.synchronize()
-    return dst.cpu().numpy()
+         C.c_void_p(torch.cuda.current_stream(src.device).cuda_stream))
+    return dst
+
+
+def _log_remap_tensor(src, use_max_as_i0: bool, i0: float):
+    """xr_log_remap of a device image on the current stream."""
+    import torch
+    rows, cols = src.shape
+    scratch = torch.empty(rows * cols + 1025, dtype=torch.float64, device=src.device)
+    dst = torch.empty_like(src)
+    call("xr_log_remap", C.c_void_p(src.data_ptr()), rows, cols, int(bool(use_max_as_i0)), float(i0),
+         C.c_void_p(scratch.data_ptr()), C.c_void_p(dst.data_ptr()),
+         C.c_void_p(torch.cuda.current_stream(src.device).cuda_stream))
+    return dst
+
+
+def crop_image_boundary(img: np.ndarray, width: int, device: int = -1) -> np.ndarray:
+    """CropImage2DBoundary on the GPU (xr_crop_image_boundary)."""
+    return _to_host(_crop_tensor(_to_device(img, device), width))
 
 
 def log_remap(img: np.ndarray, use_max_as_i0: bool = True, i0: float = 1.0, device: int = -1) -> np.ndarray:
     """ImageIntensLogTransFilter as ProjPreProc runs it, on the GPU (xr_log_remap)."""
-    import torch
-    dev = torch.device("cuda", device if device >= 0 else torch.cuda.current_device())
-    src = torch.from_numpy(np.ascontiguousarray(img, dtype=np.float32)).to(dev)
-    rows, cols = src.shape
-    scratch = torch.empty(rows * cols + 1025, dtype=torch.float64, device=dev)
-    dst = torch.empty_like(src)
-    s = torch.cuda.current_stream(dev)
-    call("xr_log_remap", C.c_void_p(src.data_ptr()), rows, cols, int(bool(use_max_as_i0)), float(i0),
-         C.c_void_p(scratch.data_ptr()), C.c_void_p(dst.data_ptr()), C.c_void_p(s.cuda_stream))
-    s.synchronize()
-    return dst.cpu().numpy()
+    return _to_host(_log_remap_tensor(_to_device(img, device), use_max_as_i0, i0))
 
 
 def proj_preproc(img: np.ndarray, cam: CameraModel, crop_width: int = 50, no_log_remap: bool = False,
@@ -773,14 +786,16 @@ def proj_preproc(img: np.ndarray, cam: CameraModel, crop_width: int = 50, no_log
     """ProjPreProc::operator() (xregProjPreProc.cpp:31-139) for one projection with
     its defaults (crop 50 pixels from every side, then the log remap with I0 from
     the smoothed maximum; metal auto-masking is not part of it here).  Returns
-    (image, camera)."""
-    out, c = np.ascontiguousarray(img, dtype=np.float32), cam
+    (image, camera).  The image goes to the device and back once."""
+    c = cam.crop_boundary(crop_width) if crop_width > 0 else cam
+    if crop_width <= 0 and no_log_remap:
+        return np.ascontiguousarray(img, dtype=np.float32), c
+    out = _to_device(img, device)
     if crop_width > 0:
-        c = cam.crop_boundary(crop_width)
-        out = crop_image_boundary(out, crop_width, device)
+        out = _crop_tensor(out, crop_width)
     if not no_log_remap:
-        out = log_remap(out, True, 1.0, device)
-    return out, c
+        out = _log_remap_tensor(out, True, 1.0)
+    return _to_host(out), c
 
 
 # ------------------------------------------------------------ poses on disk
