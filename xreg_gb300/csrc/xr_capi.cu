@@ -2152,7 +2152,10 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
     int32_t loop = 0;
     if ((st = rc_choose_config(rc, vol, P, s, &loop)) != XR_OK) return st;
     P.vol.layout = best_layout(vol);
-    const int wc = P.warp_tall ? 4 : 8, tw = wc * P.block_warps_x, th = (8 / P.block_warps_x) * (32 / wc);
+    rc->last_bw = P.block_warps_x;
+    const int warps = fused ? 8 : kDrrWarps;
+    P.block_warps_x = std::min(P.block_warps_x, warps);
+    const int wc = P.warp_tall ? 4 : 8, tw = wc * P.block_warps_x, th = (warps / P.block_warps_x) * (32 / wc);
     J.d.tiles_x = (int32_t)((P.cols + tw - 1) / tw);
     J.d.tiles_y = (int32_t)((P.rows + th - 1) / th);
     J.d.pose_group = 0;
@@ -2163,7 +2166,6 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
       J.d.tiles_y = (int32_t)((P.rows + 7) / 8);
     }
     rc->last_layout = P.vol.layout;
-    rc->last_bw = P.block_warps_x;
     rc->last_unroll = loop;
     rc->last_warp_rows = P.warp_tall ? 8 : 4;
     GeomJob G{};

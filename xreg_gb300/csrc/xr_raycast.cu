@@ -96,6 +96,11 @@ constexpr int kThreads = 256;
 // Resident blocks per SM the DRR kernels are compiled for: 48 registers, which
 // hold four cells in flight per thread; measured faster than 40 or 64.
 constexpr int kMinBlocksPerSM = 5;
+// Warps per block of drr_kernel and drr_jobs_kernel.  Rays differ in length, and a
+// block keeps its place until its longest is done: 4 warps measured 1.5 to 4 %
+// faster than 8 (population 4867 -> 4785 us, FP16 coarse 2837 -> 2718, BF16 1570 ->
+// 1521), 2 or 1 mixed (4749 / 2728 / 1545, 5178 / 2710 / 1497).
+constexpr int kWarps = kDrrWarps;
 // CELL8 data read with one 256-bit load per sample (float32 volumes only).
 constexpr int kLayoutCell8Wide = 2;
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return max(min(v, hi), lo); }
@@ -694,10 +699,10 @@ __device__ __forceinline__ void lane_pixel(int lane, int wl, int& col, int& row)
 }
 
 template <int VT, int KERNEL, int LAYOUT>
-__global__ void __launch_bounds__(kThreads, kMinBlocksPerSM)
+__global__ void __launch_bounds__(32 * kWarps, kMinBlocksPerSM * 8 / kWarps)
 drr_kernel(const DrrParams p, const int64_t proj_base) {
   // Each warp covers an 8 x 4 (or, tall, 4 x 8) patch of pixels so its 32 rays
-  // stay close inside the volume; a block is bw x (8 / bw) warps.  The
+  // stay close inside the volume; a block is bw x (kWarps / bw) warps.  The
   // projection is the fastest grid index: blocks resident at the same time trace
   // the same detector tile for many nearby poses, whose footprints overlap in L2.
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -707,7 +712,7 @@ drr_kernel(const DrrParams p, const int64_t proj_base) {
   int lc, lr;
   lane_pixel(lane, wl, lc, lr);
   const int col = blockIdx.y * (wc * bw) + (warp % bw) * wc + lc;
-  const int row = blockIdx.z * ((8 / bw) * wr) + (warp / bw) * wr + lr;
+  const int row = blockIdx.z * ((kWarps / bw) * wr) + (warp / bw) * wr + lr;
   const int64_t proj = proj_base + blockIdx.x;
   unsigned long long ns = 0;
   unsigned int nl = 0;
@@ -1119,8 +1124,9 @@ eval_fused_kernel(const FusedJob* __restrict__ jobs, int njobs, long long total,
 // 3.4% faster than 48 on an uneven set of 8 jobs.
 // GROUPED: every job's items are pose groups (MultiJobDrr::pose_group); a
 // separate instantiation, so the per-projection kernels keep their registers.
+constexpr int jobs_threads(bool grouped) { return grouped ? kThreads : 32 * kWarps; }
 template <int VT, int LAYOUT, bool GROUPED>
-__global__ void __launch_bounds__(kThreads, kMinBlocksPerSM - 1)
+__global__ void __launch_bounds__(jobs_threads(GROUPED), (kMinBlocksPerSM - 1) * kThreads / jobs_threads(GROUPED))
 drr_jobs_kernel(const MultiJobDrr* __restrict__ jobs, int njobs, long long item0) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long item = item0 + blockIdx.x;
@@ -1203,7 +1209,7 @@ drr_jobs_kernel(const MultiJobDrr* __restrict__ jobs, int njobs, long long item0
     int lc, lr;
     lane_pixel(lane, wl, lc, lr);
     col = tx * (wc * bw) + (warp % bw) * wc + lc;
-    row = ty * ((8 / bw) * wr) + (warp / bw) * wr + lr;
+    row = ty * ((kWarps / bw) * wr) + (warp / bw) * wr + lr;
   }
   if (col >= J.p.cols || row >= J.p.rows) return;
   unsigned int nl;
@@ -1258,7 +1264,7 @@ cudaError_t launch_jobs_g(const MultiJobDrr* d_jobs, int njobs, long long total,
   const long long max_x = 0x7fffffff;
   for (long long base = 0; base < total; base += max_x) {
     const long long n = (total - base) < max_x ? (total - base) : max_x;
-    drr_jobs_kernel<VT, LAYOUT, GROUPED><<<(unsigned)n, kThreads, 0, s>>>(d_jobs, njobs, base);
+    drr_jobs_kernel<VT, LAYOUT, GROUPED><<<(unsigned)n, jobs_threads(GROUPED), 0, s>>>(d_jobs, njobs, base);
   }
   return cudaGetLastError();
 }
@@ -1283,12 +1289,12 @@ cudaError_t launch_t(const DrrParams& p, cudaStream_t s) {
   }
   const int bw = p.block_warps_x;
   const int wc = p.warp_tall ? 4 : 8;
-  const int tx = wc * bw, ty = (8 / bw) * (32 / wc);
+  const int tx = wc * bw, ty = (kWarps / bw) * (32 / wc);
   const int64_t max_x = 0x7fffffff;
   for (int64_t base = 0; base < p.num_projs; base += max_x) {
     const int64_t n = (p.num_projs - base) < max_x ? (p.num_projs - base) : max_x;
     const dim3 grid((unsigned)n, (p.cols + tx - 1) / tx, (p.rows + ty - 1) / ty);
-    drr_kernel<VT, KERNEL, LAYOUT><<<grid, kThreads, 0, s>>>(p, base);
+    drr_kernel<VT, KERNEL, LAYOUT><<<grid, 32 * kWarps, 0, s>>>(p, base);
   }
   return cudaGetLastError();
 }
@@ -1330,10 +1336,12 @@ cudaError_t launch_brick(const DrrParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_drr(const DrrParams& p, cudaStream_t s) {
+cudaError_t launch_drr(const DrrParams& params, cudaStream_t s) {
+  DrrParams p = params;
+  p.block_warps_x = std::min(p.block_warps_x, kWarps);
   if (p.num_projs <= 0) return cudaSuccess;
   if (p.vol.layout == kLayoutBrick) return launch_brick(p, s);
-  if (!(p.block_warps_x == 1 || p.block_warps_x == 2 || p.block_warps_x == 4 || p.block_warps_x == 8))
+  if (!(p.block_warps_x == 1 || p.block_warps_x == 2 || p.block_warps_x == 4))
     return cudaErrorInvalidValue;
   if (p.warp_tall != 0 && p.warp_tall != 1) return cudaErrorInvalidValue;
   if (p.vol.layout != XR_LAYOUT_LINEAR && !p.vol.cells) return cudaErrorInvalidValue;
