@@ -76,3 +76,33 @@ def test_values_without_finite_differences(xr, oracle, value, vt):
     np.testing.assert_array_equal(np.isfinite(imgs[0]), ok)
     rel, zero = drr_rel_err(np.where(ok, imgs[0], 0.0), np.where(ok, ref, 0.0))
     assert zero == 0.0 and rel <= TOL[vt], rel
+
+
+# launches on either side of the rule for the deep march (at most about 155,000
+# rays): ray counts that are not multiples of a batch, and one pose of the larger
+# launch alone
+@pytest.mark.parametrize("vt", [0, 1, 2])
+@pytest.mark.parametrize("kernel", [0, 1])
+def test_small_launches_equal_large_ones(xr, vt, kernel):
+    vol = synth.phantom_volume((48, 44, 40), (2.0, 2.0, 2.0), 5)
+    cam = small_camera((130, 141), 2.0)
+    poses = synth.sample_poses(vol, synth.gt_pose(vol), 12, 20.0, 10.0, seed=4)
+    rc = xr.RayCasterLineIntCUDA()
+    rc.set_volume(vol, vt)
+    rc.set_camera_model(cam)
+    rc.set_ray_step_size(0.3)
+    rc.set_kernel_id(kernel)
+    rc.set_num_projs(len(poses))
+    rc.allocate_resources()
+    rc.distribute_xforms_among_cam_models(poses)  # 219,960 rays
+    rc.compute()
+    many = rc.projs()
+    rc.set_launch_config(0, 1, 4, 8)
+    rc.compute()
+    np.testing.assert_array_equal(rc.projs(), many)
+    rc.set_launch_config(-1)
+    for n in (1, 8):
+        rc.set_num_projs(n)
+        rc.distribute_xforms_among_cam_models(poses[3:3 + n])
+        rc.compute()
+        np.testing.assert_array_equal(rc.projs(), many[3:3 + n])

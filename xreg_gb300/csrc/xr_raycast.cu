@@ -101,6 +101,7 @@ constexpr int kMinBlocksPerSM = 5;
 // faster than 8 (population 4867 -> 4785 us, FP16 coarse 2837 -> 2718, BF16 1570 ->
 // 1521), 2 or 1 mixed (4749 / 2728 / 1545, 5178 / 2710 / 1497).
 constexpr int kWarps = kDrrWarps;
+constexpr int kDeepBlocksPerSM = 4;  // of the deep march (launch_t): 128 registers
 // CELL8 data read with one 256-bit load per sample (float32 volumes only).
 constexpr int kLayoutCell8Wide = 2;
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return max(min(v, hi), lo); }
@@ -467,7 +468,7 @@ struct CellWalk<XR_VOXEL_BF16, BYTES> {
 // scalar batches of four 5144 / 2873 / 1726, packed batches - / 3025 / 1690,
 // packed reload 7029 / 3464 / 1613 (the reload form spills at float32's and
 // FP16's register need), scalar reload of three 5317 / - / -.
-template <int VT, int KERNEL, int LAYOUT, bool BYTES>
+template <int VT, int KERNEL, int LAYOUT, bool BYTES, bool DEEP>
 __device__ __forceinline__ float march_cells(const VolView& vol, float px, float py, float pz, float sx, float sy,
                                              float sz, unsigned int n, float sum) {
   using Cell = CellData<VT, LAYOUT>;
@@ -475,6 +476,28 @@ __device__ __forceinline__ float march_cells(const VolView& vol, float px, float
   using Frac = typename Walk::Frac;
   const void* data = vol.cells;
   Walk walk(vol, px, py, pz, sx, sy, sz);
+  if constexpr (DEEP) {  // batches of eight, the last one masked
+    constexpr unsigned int kDeep = 8;
+    unsigned int c = 0;
+    while (n > 0) {
+      const unsigned int m = min(n, kDeep);
+      Frac f[kDeep];
+      Cell q[kDeep];
+#pragma unroll
+      for (unsigned int k = 0; k < kDeep; ++k) {
+        const unsigned int ck = walk.next(f[k]);
+        c = k < m ? ck : c;  // past the last sample: the last cell again
+        q[k].template load<BYTES>(data, c);
+      }
+#pragma unroll
+      for (unsigned int k = 0; k < kDeep; ++k) {
+        const float v = fold<KERNEL>(sum, q[k].value(f[k]));
+        sum = k < m ? v : sum;
+      }
+      n -= m;
+    }
+    return sum;
+  }
   if constexpr (VT == XR_VOXEL_BF16) {
     if (n >= 4) {
       Frac f[4];
@@ -536,7 +559,7 @@ __device__ __forceinline__ float march_samples(const VolView& vol, const void* d
 // (the caller checks that the pixel exists).  Returns the number of samples of
 // the reference step rule; *loaded receives how many of them were loaded (the
 // others were proven zero and skipped).
-template <int VT, int KERNEL, int LAYOUT>
+template <int VT, int KERNEL, int LAYOUT, bool DEEP = false>
 __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, const int64_t proj, const int row,
                                                           const int col, unsigned int* loaded) {
   float sum = (KERNEL == XR_LINE_INT_MAX) ? -FLT_MAX : 0.0f;
@@ -667,8 +690,9 @@ __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, co
           if constexpr (LAYOUT == XR_LAYOUT_LINEAR)
             sum = march_samples<VT, KERNEL, LAYOUT, true>(p.vol, data, px, py, pz, sx, sy, sz, n, sum);
           else
-            sum = p.vol.cell_bytes ? march_cells<VT, KERNEL, LAYOUT, true>(p.vol, px, py, pz, sx, sy, sz, n, sum)
-                                   : march_cells<VT, KERNEL, LAYOUT, false>(p.vol, px, py, pz, sx, sy, sz, n, sum);
+            sum = p.vol.cell_bytes
+                      ? march_cells<VT, KERNEL, LAYOUT, true, DEEP>(p.vol, px, py, pz, sx, sy, sz, n, sum)
+                      : march_cells<VT, KERNEL, LAYOUT, false, DEEP>(p.vol, px, py, pz, sx, sy, sz, n, sum);
         } else {
           sum = march_samples<VT, KERNEL, LAYOUT, false>(p.vol, data, px, py, pz, sx, sy, sz, n, sum);
         }
@@ -698,8 +722,8 @@ __device__ __forceinline__ void lane_pixel(int lane, int wl, int& col, int& row)
   row = ((lane >> 1) & 1) + ((lane >> (wl + 1)) << 1);
 }
 
-template <int VT, int KERNEL, int LAYOUT>
-__global__ void __launch_bounds__(32 * kWarps, kMinBlocksPerSM * 8 / kWarps)
+template <int VT, int KERNEL, int LAYOUT, bool DEEP>
+__global__ void __launch_bounds__(32 * kWarps, DEEP ? kDeepBlocksPerSM : kMinBlocksPerSM * 8 / kWarps)
 drr_kernel(const DrrParams p, const int64_t proj_base) {
   // Each warp covers an 8 x 4 (or, tall, 4 x 8) patch of pixels so its 32 rays
   // stay close inside the volume; a block is bw x (kWarps / bw) warps.  The
@@ -716,7 +740,7 @@ drr_kernel(const DrrParams p, const int64_t proj_base) {
   const int64_t proj = proj_base + blockIdx.x;
   unsigned long long ns = 0;
   unsigned int nl = 0;
-  if (col < p.cols && row < p.rows) ns = trace_pixel<VT, KERNEL, LAYOUT>(p, proj, row, col, &nl);
+  if (col < p.cols && row < p.rows) ns = trace_pixel<VT, KERNEL, LAYOUT, DEEP>(p, proj, row, col, &nl);
   if (p.sample_counter) {
     unsigned long long nlw = nl;
     for (int o = 16; o > 0; o >>= 1) {
@@ -1275,15 +1299,15 @@ cudaError_t launch_jobs_t(const MultiJobDrr* d_jobs, int njobs, long long total,
                  : launch_jobs_g<VT, LAYOUT, false>(d_jobs, njobs, total, s);
 }
 
-template <int VT, int KERNEL, int LAYOUT>
-cudaError_t launch_t(const DrrParams& p, cudaStream_t s) {
+template <int VT, int KERNEL, int LAYOUT, bool DEEP>
+cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
   // The kernel uses no shared memory: ask for the largest L1 (the gathers hit
   // it), once per device (a preference; setting it twice is harmless).
   static std::atomic<bool> carveout_set[kMaxDevices];
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
       !carveout_set[dev].load(std::memory_order_relaxed)) {
-    cudaFuncSetAttribute(drr_kernel<VT, KERNEL, LAYOUT>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(drr_kernel<VT, KERNEL, LAYOUT, DEEP>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxL1);
     carveout_set[dev].store(true, std::memory_order_relaxed);
   }
@@ -1294,9 +1318,33 @@ cudaError_t launch_t(const DrrParams& p, cudaStream_t s) {
   for (int64_t base = 0; base < p.num_projs; base += max_x) {
     const int64_t n = (p.num_projs - base) < max_x ? (p.num_projs - base) : max_x;
     const dim3 grid((unsigned)n, (p.cols + tx - 1) / tx, (p.rows + ty - 1) / ty);
-    drr_kernel<VT, KERNEL, LAYOUT><<<grid, 32 * kWarps, 0, s>>>(p, base);
+    drr_kernel<VT, KERNEL, LAYOUT, DEEP><<<grid, 32 * kWarps, 0, s>>>(p, base);
   }
   return cudaGetLastError();
+}
+
+// A launch of few rays is bound by the latency of a ray's loads one after another
+// (a quarter of the warps the SMs hold, data that no earlier pose brought into L2),
+// so it takes eight cells in flight per thread at 128 registers where a large one
+// takes four at 48.  Up to twice the rays that are resident at 128 registers;
+// measured, four against eight, in us with the geometry launch: 256^3 float32, one
+// pose of 256^2 116 / 64, 330^2 114 / 87, 384^2 113 / 94; 320 x 320 x 256 FP16,
+// three views of 192^2 127 / 98; BF16, two views of 240^2 84 / 83, of 300 x 260
+// (156,000 rays) 97 / 98; FP16, two views of 384^2 (294,912 rays) 148 / 150.
+template <int VT, int KERNEL, int LAYOUT>
+cudaError_t launch_t(const DrrParams& p, cudaStream_t s) {
+  if constexpr (LAYOUT != XR_LAYOUT_LINEAR) {
+    static std::atomic<int> cached[kMaxDevices];  // SMs per device; zero = not known yet
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+      sms = cached[dev].load(std::memory_order_relaxed);
+      if (!sms && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+        cached[dev].store(sms, std::memory_order_relaxed);
+    }
+    if (p.num_projs * p.rows * p.cols <= 2 * (int64_t)sms * kDeepBlocksPerSM * 32 * kWarps)
+      return launch_depth<VT, KERNEL, LAYOUT, true>(p, s);
+  }
+  return launch_depth<VT, KERNEL, LAYOUT, false>(p, s);
 }
 
 template <int VT, int KERNEL>
