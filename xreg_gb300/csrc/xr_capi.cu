@@ -2190,8 +2190,8 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
     const int rows = (int)rc->rows(), cols = (int)rc->cols();
     J.nviews = nv;
     J.pop = pop;
-    J.mt_x = (cols + 31) / 32;
-    J.mt_y = (rows + 63) / 64;
+    J.mt_x = (cols + kMetricTileCols - 1) / kMetricTileCols;
+    J.mt_y = (rows + kMetricTileRows - 1) / kMetricTileRows;
     J.out = obj->d_sims.as<float>();
     J.metric = obj_metric_fusable(obj) ? 1 : 0;
     for (int32_t v = 0; v < nv; ++v) {

@@ -1,7 +1,7 @@
 // xr_gradtile.cuh -- device code shared by the split grad-NCC metric kernels
 // (xr_metrics.cu) and the fused evaluation kernel (xr_raycast.cu): compensated
-// reductions, the moments of one 32 x 64-pixel tile of a moving image's
-// gradients, and the per-image FP64 combine.  Both paths run exactly this code
+// reductions, the moments of one tile of a moving image's gradients, and the
+// per-image FP64 combine.  Both paths run exactly this code
 // on the same tiles, so their similarity values are identical bit for bit.
 //
 // Gradients (xregImgSimMetric2DGradImgCPU.cpp:48-65,86-101): OpenCV's sigma-0
@@ -15,10 +15,16 @@
 namespace xr {
 namespace gt {
 
-constexpr int kThreads = 256;                     // block size of every tile kernel
-constexpr int kGW = 32;                           // tile columns = threads across
-constexpr int kGR = 8;                            // rows per thread
-constexpr int kGH = kGR * (kThreads / kGW);       // tile rows (64)
+constexpr int kThreads = 256;                     // block size of the NCC and patch kernels
+// A tile is 2 x 2 strips, one per warp: a strip is kStripRows rows of the columns
+// whose blur and Sobel stencils a warp's 32 columns hold.
+constexpr int kStripRows = 32;
+constexpr int kGH = 2 * kStripRows;               // tile rows
+template <int KR>
+constexpr int kTileCols = 2 * (32 - 2 * (KR + 1));
+constexpr int kGW = kTileCols<2>;                 // tile columns of the 5x5 blur (52)
+static_assert(kGH == kMetricTileRows && kGW == kMetricTileCols, "the host's tile counts");
+constexpr int kTileThreads = 128;                 // the four warps
 constexpr int kFinalizeThreads = 128;             // threads of the per-image combine
 
 __device__ __forceinline__ int reflect101(int i, int n) {
@@ -118,194 +124,156 @@ __device__ __forceinline__ double ncc_sim_from_moments(double sm, double smm, do
   return (1.0 - ncc) * 0.5;
 }
 
-// Shared memory of one tile: the horizontally blurred rows, blurred in place
-// down the columns (the vertical pass reads every input before it writes).
-template <int KR>
-struct GradTileSmem {
-  static constexpr int H = KR + 1;                // halo: blur radius + Sobel
-  static constexpr int WI = kGW + 2 * H, HI = kGH + 2 * H;
-  static constexpr int WB = kGW + 2, HB = kGH + 2;
-  float hb[HI][WB + 1];
-  FF red[6 * (kThreads / 32)];
-};
-
-// The tile's six moments from every thread's partial sums: plain float within
-// a warp (256 pixels), float-float across the warps (red: [6][8]); v valid in
-// thread 0.
-__device__ __forceinline__ void tile_moments_reduce(const float (&m)[6], FF* red, double (&v)[6]) {
-  constexpr int kWarps = kThreads / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    float w = m[k];
-    for (int o = 16; o > 0; o >>= 1) w = __fadd_rn(w, __shfl_down_sync(0xffffffffu, w, o));
-    if (lane == 0) red[k * kWarps + warp] = FF{w, 0.0f};
-  }
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      FF w = (lane < kWarps) ? red[k * kWarps + lane] : FF{0.0f, 0.0f};
-      for (int o = 16; o > 0; o >>= 1) w = ff_add(w, ff_shfl_down(w, o));
-      v[k] = (double)w.hi + (double)w.lo;
-    }
-  }
-  __syncthreads();  // red (and the tile's shared memory) is reused by the caller's next tile
-}
-
-// Image pixel (row, col) of a tile's input; CG reads through L2 only (pixels
-// written earlier in the same kernel by other blocks).
+// A pixel of a tile's input; CG reads through L2 only (pixels written earlier in
+// the same kernel by other blocks).
 template <bool CG>
-__device__ __forceinline__ float tile_px(const float* __restrict__ src, int cols, int gr, int gc) {
-  const float* p = src + (int64_t)gr * cols + gc;
+__device__ __forceinline__ float tile_px(const float* __restrict__ p) {
   return CG ? __ldcg(p) : __ldg(p);
 }
 
-// Moments of the moving gradients over the 32 x 64-pixel tile at (y0, x0),
-// 256 threads: each thread owns one column and eight consecutive rows, so the
-// Sobel stencil slides down the column; sums are plain float per thread (8
-// terms) and per warp (256 pixels), float-float across the warps.  v (valid in
-// thread 0): S_gx, S_gx^2, S_gx fx, S_gy, S_gy^2, S_gy fy.
+// Moments of the moving gradients over the kGH x kTileCols<KR> tile at (y0, x0), by
+// the block's first four warps (all of its threads call it): each lane owns a
+// column and goes down its strip's rows; the horizontal neighbours come by
+// shuffles, the vertical ones stay in registers, so a pixel is read once from
+// global memory and nothing goes through shared memory.  Sums are plain float over
+// 8 rows of a column, float-float over the column, the lanes and the warps.  The
+// value of moment k (S_gx, S_gx^2, S_gx fx, S_gy, S_gy^2, S_gy fy) is returned in
+// thread k < 6.  red: [6][4].
+// Bound by instruction issue: about 50 per pixel and lane, of which 26 of 32 lanes
+// and 32 of 38 rows count.  100 images of 384^2 with their combines: 61 us, 150 with
+// the tile's rows blurred in shared memory (5 loads and an index division per
+// blurred value); one image 16 us.
 template <int KR, bool CG>
-__device__ void grad_tile_moments(const float* __restrict__ src, int rows, int cols, int y0, int x0,
-                                  const float* __restrict__ fhx, const float* __restrict__ fhy,
-                                  const uint8_t* __restrict__ mask, GradTileSmem<KR>& sm, double (&v)[6]) {
-  using S = GradTileSmem<KR>;
-  constexpr int H = S::H, HI = S::HI, WB = S::WB, HB = S::HB;
-  const int tx = threadIdx.x % kGW, ty = threadIdx.x / kGW;
-  // Rows / cols past the last tile pixel only feed pixels that are skipped;
-  // clamping before the reflection keeps every read inside the image.
-  const bool interior = y0 >= H && x0 >= H && y0 + kGH + H <= rows && x0 + kGW + H <= cols;
-  auto in = [&](int r, int c) -> float {
-    int gr = y0 - H + r, gc = x0 - H + c;
-    if (!interior) {
-      gr = reflect101(min(gr, rows - 1 + H), rows);
-      gc = reflect101(min(gc, cols - 1 + H), cols);
-    }
-    return tile_px<CG>(src, cols, gr, gc);
-  };
-  if constexpr (KR == 0) {
-    for (int i = threadIdx.x; i < HB * WB; i += kThreads) {
-      const int r = i / WB, c = i - r * WB;
-      sm.hb[r][c] = in(r, c);
-    }
-  } else {
-    // horizontal pass over all input rows, blurred columns [x0-1, x0+kGW+1)
-    for (int i = threadIdx.x; i < HI * WB; i += kThreads) {
-      const int r = i / WB, c = i - r * WB;
-      sm.hb[r][c] = (KR == 2) ? blur5(in(r, c), in(r, c + 1), in(r, c + 2), in(r, c + 3), in(r, c + 4))
-                              : blur3(in(r, c), in(r, c + 1), in(r, c + 2));
-    }
-    __syncthreads();
-    // vertical pass in place: WB columns x 4 chunks of rows, every output of a
-    // chunk computed before the barrier, written after it
-    constexpr int kChunks = 4, kCh = (HB + kChunks - 1) / kChunks;
-    const int c = threadIdx.x % WB, j = threadIdx.x / WB;
-    float o[kCh];
-    if (j < kChunks) {
+__device__ double grad_tile_moments(const float* __restrict__ src, int rows, int cols, int y0, int x0,
+                                    const float* __restrict__ fhx, const float* __restrict__ fhy,
+                                    const uint8_t* __restrict__ mask, FF* red) {
+  constexpr int H = KR + 1, kWin = 2 * KR + 1, kGroup = 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < 4) {
+    const int xs = x0 + (warp & 1) * (32 - 2 * H), ys = y0 + (warp >> 1) * kStripRows;  // the strip's first pixel
+    const int x = xs - H + lane;
+    // Rows / cols past the image's last pixel plus the halo only feed pixels that are
+    // skipped; clamping before the reflection keeps every read inside the image.
+    const float* pc = src + reflect101(min(x, cols - 1 + H), cols);
+    const int xf = min(max(x, 0), cols - 1);  // lanes without a pixel of their own read some fixed value
+    const bool owner = lane >= H && lane < 32 - H && x < cols;
+    float hb[kWin];           // horizontally blurred rows
+    float bl[3], lf[3], rt[3];  // blurred rows and their left and right neighbours
+    FF acc[6];
 #pragma unroll
-      for (int k = 0; k < kCh; ++k) {
-        const int r = j * kCh + k;
-        if (r < HB)
-          o[k] = (KR == 2) ? blur5(sm.hb[r][c], sm.hb[r + 1][c], sm.hb[r + 2][c], sm.hb[r + 3][c], sm.hb[r + 4][c])
-                           : blur3(sm.hb[r][c], sm.hb[r + 1][c], sm.hb[r + 2][c]);
+    for (int q = 0; q < 6; ++q) acc[q] = FF{0.0f, 0.0f};
+    auto row_of = [&](int r) -> const float* {  // input row r of the strip, from its first halo row
+      const int y = min(ys - H + r, rows - 1 + H);
+      return pc + (int64_t)reflect101(y, rows) * cols;
+    };
+    // takes one input row: the newest blurred row follows (garbage until the window is full)
+    auto push = [&](float p) {
+      float h = p;
+      if constexpr (KR == 2)
+        h = blur5(__shfl_up_sync(0xffffffffu, p, 2), __shfl_up_sync(0xffffffffu, p, 1), p,
+                  __shfl_down_sync(0xffffffffu, p, 1), __shfl_down_sync(0xffffffffu, p, 2));
+      else if constexpr (KR == 1)
+        h = blur3(__shfl_up_sync(0xffffffffu, p, 1), p, __shfl_down_sync(0xffffffffu, p, 1));
+#pragma unroll
+      for (int i = 0; i + 1 < kWin; ++i) hb[i] = hb[i + 1];
+      hb[kWin - 1] = h;
+      bl[0] = bl[1]; bl[1] = bl[2];
+      lf[0] = lf[1]; lf[1] = lf[2];
+      rt[0] = rt[1]; rt[1] = rt[2];
+      if constexpr (KR == 2) bl[2] = blur5(hb[0], hb[1], hb[2], hb[3], hb[4]);
+      else if constexpr (KR == 1) bl[2] = blur3(hb[0], hb[1], hb[2]);
+      else bl[2] = hb[0];
+      lf[2] = __shfl_up_sync(0xffffffffu, bl[2], 1);
+      rt[2] = __shfl_down_sync(0xffffffffu, bl[2], 1);
+    };
+#pragma unroll
+    for (int i = 0; i < kWin; ++i) hb[i] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) bl[i] = lf[i] = rt[i] = 0.0f;
+    {
+      float p[2 * H];
+#pragma unroll
+      for (int i = 0; i < 2 * H; ++i) p[i] = tile_px<CG>(row_of(i));
+#pragma unroll
+      for (int i = 0; i < 2 * H; ++i) push(p[i]);
+    }
+#pragma unroll 1
+    for (int g = 0; g < kStripRows && ys + g < rows; g += kGroup) {
+      float p[kGroup], fx[kGroup], fy[kGroup], m[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      const int64_t first = (int64_t)(ys + g) * cols + xf;
+      auto sums = [&](int i) {
+        float gx, gy;
+        sobel3(lf[0], bl[0], rt[0], lf[1], rt[1], lf[2], bl[2], rt[2], gx, gy);
+        moments_add(m, gx, gy, fx[i], fy[i]);
+      };
+      if (!mask && ys + g + H >= 0 && ys + g + kGroup + H <= rows) {  // no row to reflect, none to skip
+        const float* q = pc + (int64_t)(ys + g + H) * cols;
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          p[i] = tile_px<CG>(q + (int64_t)i * cols);
+          fx[i] = __ldg(fhx + first + (int64_t)i * cols);
+          fy[i] = __ldg(fhy + first + (int64_t)i * cols);
+        }
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          push(p[i]);
+          sums(i);
+        }
+      } else {
+        bool use[kGroup];
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) p[i] = tile_px<CG>(row_of(2 * H + g + i));
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          const int64_t pix = first + (int64_t)i * cols;
+          use[i] = owner && ys + g + i < rows && (!mask || mask[pix]);
+          fx[i] = use[i] ? __ldg(fhx + pix) : 0.0f;
+          fy[i] = use[i] ? __ldg(fhy + pix) : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          push(p[i]);
+          if (use[i]) sums(i);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const float t = __fadd_rn(acc[q].hi, m[q]), d = __fsub_rn(t, acc[q].hi);
+        acc[q].lo = __fadd_rn(acc[q].lo, __fadd_rn(__fsub_rn(acc[q].hi, __fsub_rn(t, d)), __fsub_rn(m[q], d)));
+        acc[q].hi = t;
       }
     }
-    __syncthreads();
-    if (j < kChunks) {
 #pragma unroll
-      for (int k = 0; k < kCh; ++k) {
-        const int r = j * kCh + k;
-        if (r < HB) sm.hb[r][c] = o[k];
-      }
+    for (int q = 0; q < 6; ++q) {
+      acc[q].hi = owner ? acc[q].hi : 0.0f;
+      acc[q].lo = owner ? acc[q].lo : 0.0f;
+    }
+    // over the lanes: the halves of the warp take three moments each, then 16 lanes each
+    const bool upper = lane >= 16;
+    FF v[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const FF mine = upper ? acc[q + 3] : acc[q], theirs = upper ? acc[q] : acc[q + 3];
+      const FF got{__shfl_xor_sync(0xffffffffu, theirs.hi, 16), __shfl_xor_sync(0xffffffffu, theirs.lo, 16)};
+      v[q] = ff_add(mine, got);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) v[q] = ff_add(v[q], ff_shfl_down(v[q], o));
+      if ((lane & 15) == 0) red[(q + (upper ? 3 : 0)) * 4 + warp] = v[q];
     }
   }
   __syncthreads();
-  const auto& bl = sm.hb;  // blurred region [HB][WB]
-  float m[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  const int gxc = x0 + tx;
-  if (gxc < cols) {
-    const int rb = ty * kGR;  // first output row (tile-local); blurred rows rb .. rb + kGR + 1
-    float a0 = bl[rb][tx], b0 = bl[rb][tx + 1], c0 = bl[rb][tx + 2];
-    float a1 = bl[rb + 1][tx], b1 = bl[rb + 1][tx + 1], c1 = bl[rb + 1][tx + 2];
+  double out = 0.0;
+  if (threadIdx.x < 6) {
+    FF t = red[threadIdx.x * 4];
 #pragma unroll
-    for (int k = 0; k < kGR; ++k) {
-      const float a2 = bl[rb + k + 2][tx], b2 = bl[rb + k + 2][tx + 1], c2 = bl[rb + k + 2][tx + 2];
-      const int gyr = y0 + rb + k;
-      if (gyr < rows) {
-        const int64_t pix = (int64_t)gyr * cols + gxc;
-        if (!mask || mask[pix]) {
-          float gx, gy;
-          sobel3(a0, b0, c0, a1, c1, a2, b2, c2, gx, gy);
-          moments_add(m, gx, gy, fhx[pix], fhy[pix]);
-        }
-      }
-      a0 = a1; b0 = b1; c0 = c1;
-      a1 = a2; b1 = b2; c1 = c2;
-    }
+    for (int w = 1; w < 4; ++w) t = ff_add(t, red[threadIdx.x * 4 + w]);
+    out = (double)t.hi + (double)t.lo;
   }
-  tile_moments_reduce(m, sm.red, v);
-}
-
-// The same moments with the 5x5 blur (KR = 2) computed in registers, without
-// the tile's shared-memory rows: each thread streams down its rows (plus the
-// halo), keeping the last five horizontally blurred rows and the last three
-// blurred rows of the three columns its Sobel stencil reads; reads go through
-// L2 only.  Every value comes from the same operations as in
-// grad_tile_moments, so the moments are identical bit for bit; red: [6][8].
-__device__ inline void grad_tile_moments_regs5(const float* __restrict__ src, int rows, int cols, int y0, int x0,
-                                               const float* __restrict__ fhx, const float* __restrict__ fhy,
-                                               const uint8_t* __restrict__ mask, FF* red, double (&v)[6]) {
-  constexpr int H = 3;
-  const int tx = threadIdx.x % kGW, ty = threadIdx.x / kGW;
-  const bool interior = y0 >= H && x0 >= H && y0 + kGH + H <= rows && x0 + kGW + H <= cols;
-  auto in = [&](int r, int c) -> float {  // tile input coordinates, as grad_tile_moments
-    int gr = y0 - H + r, gc = x0 - H + c;
-    if (!interior) {
-      gr = reflect101(min(gr, rows - 1 + H), rows);
-      gc = reflect101(min(gc, cols - 1 + H), cols);
-    }
-    return __ldcg(src + (int64_t)gr * cols + gc);
-  };
-  float m[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  const int gxc = x0 + tx;
-  if (gxc < cols) {
-    const int rb = ty * kGR;
-    // horizontally blurred rows r-4 .. r and blurred rows q-2 .. q of columns
-    // tx .. tx + 2 (zero until filled: the first iterations shift them in)
-    float h[5][3] = {}, b[3][3] = {};
-#pragma unroll 1
-    for (int r = 0; r < kGR + 6; ++r) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) h[i][j] = h[i + 1][j];
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-        h[4][j] = blur5(in(rb + r, tx + j), in(rb + r, tx + j + 1), in(rb + r, tx + j + 2), in(rb + r, tx + j + 3),
-                        in(rb + r, tx + j + 4));
-      if (r >= 4) {  // blurred row rb + r - 4
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          b[0][j] = b[1][j];
-          b[1][j] = b[2][j];
-          b[2][j] = blur5(h[0][j], h[1][j], h[2][j], h[3][j], h[4][j]);
-        }
-        if (r >= 6) {  // output row rb + r - 6 from blurred rows r - 6 .. r - 4
-          const int gyr = y0 + rb + r - 6;
-          if (gyr < rows) {
-            const int64_t pix = (int64_t)gyr * cols + gxc;
-            if (!mask || mask[pix]) {
-              float gx, gy;
-              sobel3(b[0][0], b[0][1], b[0][2], b[1][0], b[1][2], b[2][0], b[2][1], b[2][2], gx, gy);
-              moments_add(m, gx, gy, fhx[pix], fhy[pix]);
-            }
-          }
-        }
-      }
-    }
-  }
-  tile_moments_reduce(m, red, v);
+  __syncthreads();  // red is reused by the caller's next tile
+  return out;
 }
 
 // Per-image combine: the tile partials (nblk x 6 doubles, read through L2 when

@@ -159,12 +159,13 @@ struct FusedView {
 };
 // A job of a fused evaluation launch: its DRR work items (16x16-pixel tiles,
 // projection fastest), and when `metric` is 1 the grad-NCC of every image
-// computed tile by tile as soon as the DRR pixels a 32x64 metric tile reads are
+// computed tile by tile as soon as the DRR pixels a 64x52-pixel metric tile reads are
 // written, then each image's value, then each pose's mean over views.
 // Counters live in `cnt` (zero between launches; the block that completes a
 // counter resets it): [nviews * pop * mt] DRR tiles done per metric tile, then
 // [nviews * pop] metric tiles done per image, then [pop] views done per pose.
 constexpr int kMaxFusedViews = 16;
+constexpr int kMetricTileRows = 64, kMetricTileCols = 52;  // gt::kGH, gt::kGW
 struct FusedJob {
   MultiJobDrr d;
   int32_t metric;         // 1: grad-NCC fused behind the DRR; 0: DRR only
@@ -182,7 +183,7 @@ struct FusedJob {
 cudaError_t launch_eval_fused(const FusedJob* d_jobs, int njobs, long long total_items, int32_t voxel_type,
                               int32_t layout, unsigned long long* d_counter, int* blocks_out, cudaStream_t s);
 // Grad-NCC (5x5 smoothing) of every image of the jobs with `metric` set, their
-// DRRs already written: one launch over all their 32x64 tiles (the split
+// DRRs already written: one launch over all their tiles (the split
 // path's tile code), each image's FP64 combine by the block that completes its
 // tiles, each pose's mean over views by the block that completes its views,
 // and (jobs with `cma`) the CMA-ES update by the block that completes the

@@ -236,28 +236,24 @@ __global__ void __launch_bounds__(kThreads) grad_images_kernel(const float* __re
   }
 }
 
-// Moments of the moving gradients, one 32 x 64-pixel tile per block
-// (gt::grad_tile_moments, shared with the fused evaluation kernel).
+// Moments of the moving gradients, one tile per block (gt::grad_tile_moments,
+// shared with the fused evaluation kernel).
 using gt::kGH;
 using gt::kGW;
 
 template <int KR>
-__global__ void __launch_bounds__(kThreads) grad_moments_kernel(const float* __restrict__ imgs, int rows, int cols,
-                                                                const float* __restrict__ fhx,
-                                                                const float* __restrict__ fhy,
-                                                                const uint8_t* __restrict__ mask,
-                                                                double* __restrict__ partials) {
-  __shared__ gt::GradTileSmem<KR> sm;
-  const int tiles_x = (cols + kGW - 1) / kGW;
-  const int y0 = (blockIdx.x / tiles_x) * kGH, x0 = (blockIdx.x % tiles_x) * kGW;
+__global__ void __launch_bounds__(gt::kTileThreads, 5) grad_moments_kernel(const float* __restrict__ imgs, int rows,
+                                                                        int cols, const float* __restrict__ fhx,
+                                                                        const float* __restrict__ fhy,
+                                                                        const uint8_t* __restrict__ mask,
+                                                                        double* __restrict__ partials) {
+  __shared__ FF red[6 * 4];
+  const int tiles_x = (cols + gt::kTileCols<KR> - 1) / gt::kTileCols<KR>;
+  const int y0 = (blockIdx.x / tiles_x) * kGH, x0 = (blockIdx.x % tiles_x) * gt::kTileCols<KR>;
   const int64_t img = blockIdx.y;
-  double v[6];
-  gt::grad_tile_moments<KR, false>(imgs + img * (int64_t)rows * cols, rows, cols, y0, x0, fhx, fhy, mask, sm, v);
-  if (threadIdx.x == 0) {
-    double* o = partials + (img * gridDim.x + blockIdx.x) * 6;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) o[k] = v[k];
-  }
+  const double v = gt::grad_tile_moments<KR, false>(imgs + img * (int64_t)rows * cols, rows, cols, y0, x0, fhx, fhy, mask,
+                                                    red);
+  if (threadIdx.x < 6) partials[(img * gridDim.x + blockIdx.x) * 6 + threadIdx.x] = v;
 }
 
 // One block of 128 threads per image: the tile partials combined in double
@@ -271,7 +267,7 @@ __global__ void grad_finalize_kernel(const double* __restrict__ partials, int nb
 }
 
 // Batched grad-NCC over many jobs' images (launch_grad_multi): one block per
-// 32x64 tile, grid-stride; the counters of FusedJob::cnt (images, then poses)
+// tile, grid-stride; the counters of FusedJob::cnt (images, then poses)
 // chain the per-image combine and the mean over views behind the tiles.
 // A device CMA-ES job's update from its lambda values (the float means over
 // views, widened to double as the host step does) by a whole block: the stages
@@ -379,9 +375,9 @@ __device__ __noinline__ void grad_multi_finish(const FusedJob& J, const FusedVie
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 6) grad_multi_kernel(const FusedJob* __restrict__ jobs, int njobs,
-                                                                 long long total) {
-  __shared__ gt::GradTileSmem<2> sm;
+__global__ void __launch_bounds__(gt::kTileThreads, 5) grad_multi_kernel(const FusedJob* __restrict__ jobs, int njobs,
+                                                                      long long total) {
+  __shared__ FF red[6 * 4];
   __shared__ double dred[6 * (gt::kFinalizeThreads / 32)];
   __shared__ int s_last, s_job_done;
   for (long long t = blockIdx.x; t < total; t += gridDim.x) {
@@ -394,14 +390,14 @@ __global__ void __launch_bounds__(kThreads, 6) grad_multi_kernel(const FusedJob*
     const int M = (int)(local - img * mt);
     const int64_t nimg = (int64_t)J.nviews * J.pop, v = img / J.pop, k = img - v * J.pop;
     const FusedView& V = J.views[v];
-    double vals[6];
-    gt::grad_tile_moments<2, false>(J.d.p.out + img * (int64_t)rows * cols, rows, cols, (M / J.mt_x) * kGH,
-                                    (M % J.mt_x) * kGW, V.fhx, V.fhy, V.mask, sm, vals);
-    if (threadIdx.x == 0) {
-      double* o = V.partials + (k * mt + M) * 6;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) o[q] = vals[q];
+    const double val = gt::grad_tile_moments<2, false>(J.d.p.out + img * (int64_t)rows * cols, rows, cols,
+                                                       (M / J.mt_x) * kGH, (M % J.mt_x) * kGW, V.fhx, V.fhy, V.mask, red);
+    if (threadIdx.x < 6) {
+      V.partials[(k * mt + M) * 6 + threadIdx.x] = val;
       __threadfence();
+      __syncwarp(0x3f);
+    }
+    if (threadIdx.x == 0) {
       unsigned int* ci = J.cnt + nimg * mt + img;
       s_last = atomicAdd(ci, 1u) + 1u == (unsigned int)mt;
       if (s_last) *ci = 0u;
@@ -927,15 +923,22 @@ cudaError_t launch_grad_images(const float* img, int rows, int cols, int64_t nim
 cudaError_t launch_grad_moments(const float* mov, int rows, int cols, int64_t nimgs, int smooth_ksize,
                                 const float* fhat_x, const float* fhat_y, const uint8_t* mask, double* partials,
                                 cudaStream_t s, int* nblk_out) {
-  const int tiles = ((rows + kGH - 1) / kGH) * ((cols + kGW - 1) / kGW);
+  int tw = 0;
+  switch (smooth_ksize) {
+    case 0: tw = gt::kTileCols<0>; break;
+    case 3: tw = gt::kTileCols<1>; break;
+    case 5: tw = gt::kTileCols<2>; break;
+    default: return cudaErrorInvalidValue;
+  }
+  const int tiles = ((rows + kGH - 1) / kGH) * ((cols + tw - 1) / tw);
   if (nblk_out) *nblk_out = tiles;
   if (nimgs <= 0 || !partials) return cudaSuccess;
   const dim3 grid(tiles, (unsigned)nimgs);
+  constexpr int nt = gt::kTileThreads;
   switch (smooth_ksize) {
-    case 0: grad_moments_kernel<0><<<grid, kThreads, 0, s>>>(mov, rows, cols, fhat_x, fhat_y, mask, partials); break;
-    case 3: grad_moments_kernel<1><<<grid, kThreads, 0, s>>>(mov, rows, cols, fhat_x, fhat_y, mask, partials); break;
-    case 5: grad_moments_kernel<2><<<grid, kThreads, 0, s>>>(mov, rows, cols, fhat_x, fhat_y, mask, partials); break;
-    default: return cudaErrorInvalidValue;
+    case 0: grad_moments_kernel<0><<<grid, nt, 0, s>>>(mov, rows, cols, fhat_x, fhat_y, mask, partials); break;
+    case 3: grad_moments_kernel<1><<<grid, nt, 0, s>>>(mov, rows, cols, fhat_x, fhat_y, mask, partials); break;
+    default: grad_moments_kernel<2><<<grid, nt, 0, s>>>(mov, rows, cols, fhat_x, fhat_y, mask, partials); break;
   }
   return cudaGetLastError();
 }
@@ -945,10 +948,11 @@ cudaError_t launch_grad_multi(const FusedJob* d_jobs, int njobs, long long total
   int dev = 0, sms = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grad_multi_kernel, kThreads, 0);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grad_multi_kernel, gt::kTileThreads, 0);
   if (e != cudaSuccess) return e;
   const long long cap = (long long)sms * (per_sm > 0 ? per_sm : 1);
-  grad_multi_kernel<<<(unsigned)(total < cap ? total : cap), kThreads, 0, s>>>(d_jobs, njobs, total);
+  grad_multi_kernel<<<(unsigned)(total < cap ? total : cap), gt::kTileThreads, 0, s>>>(d_jobs, njobs, total);
   return cudaGetLastError();
 }
 

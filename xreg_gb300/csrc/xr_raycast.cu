@@ -999,7 +999,7 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
 // next (job, tile, projection) item from a global counter; projections are
 // the fastest index within a job), with each job's grad-NCC (5x5 smoothing) computed inside the same launch.
 // No block ever waits for another.  After a block writes a 16x16 DRR tile it
-// counts the tile towards every 32x64 metric tile whose input (the tile with
+// counts the tile towards every 64x52 metric tile whose input (the tile with
 // its 3-pixel blur + Sobel halo, clipped to the image) the tile overlaps; the
 // block whose count completes a metric tile computes that tile's moments at
 // once, reading the DRR pixels back through L2 (gt::grad_tile_moments, the
@@ -1047,15 +1047,16 @@ __device__ __noinline__ bool fused_metric_tile(const FusedJob& J, int64_t proj, 
   const int64_t nimg = (int64_t)J.nviews * J.pop;
   const int64_t v = proj / J.pop, k = proj - v * J.pop;
   const FusedView& V = J.views[v];
-  double vals[6];
-  gt::grad_tile_moments_regs5(P.out + proj * (int64_t)rows * cols, rows, cols, (M / J.mt_x) * gt::kGH,
-                              (M % J.mt_x) * gt::kGW, V.fhx, V.fhy, V.mask, red, vals);
+  const double val = gt::grad_tile_moments<2, true>(P.out + proj * (int64_t)rows * cols, rows, cols,
+                                                    (M / J.mt_x) * gt::kGH, (M % J.mt_x) * gt::kGW, V.fhx, V.fhy, V.mask,
+                                                    red);
   bool last = false;
-  if (threadIdx.x == 0) {
-    double* o = V.partials + (k * mt + M) * 6;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) o[q] = vals[q];
+  if (threadIdx.x < 6) {
+    V.partials[(k * mt + M) * 6 + threadIdx.x] = val;
     __threadfence();
+    __syncwarp(0x3f);
+  }
+  if (threadIdx.x == 0) {
     unsigned int* ci = J.cnt + nimg * mt + proj;
     last = atomicAdd(ci, 1u) + 1u == (unsigned int)mt;
     if (last) *ci = 0u;
@@ -1091,7 +1092,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocksPerSM)
 eval_fused_kernel(const FusedJob* __restrict__ jobs, int njobs, long long total, unsigned long long* counter) {
   // under 1 KB of shared memory: the SM's unified L1 stays with the DRR gathers
   __shared__ long long s_item;
-  __shared__ gt::FF s_red[6 * (kThreads / 32)];
+  __shared__ gt::FF s_red[6 * 4];
   __shared__ double s_dred[6 * (gt::kFinalizeThreads / 32)];
   __shared__ int s_claim[16];
   __shared__ int s_nclaim, s_last;
