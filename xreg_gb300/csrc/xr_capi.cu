@@ -2093,7 +2093,10 @@ static xr_status metric_job(xr_objective obj, int64_t pop, FusedJob& J, std::vec
     m->rc_id = rc->id;
     m->proj_offset = (int64_t)v * pop;
     if (J.metric) {
-      XR_CHECK_ARG(m->nblk == J.mt_x * J.mt_y && m->capacity >= pop, "evaluation: metric buffers do not fit");
+      XR_CHECK_ARG(m->nblk == J.mt_x * J.mt_y, "evaluation: metric buffers do not fit");
+      // a metric allocated again for fewer images than this population
+      XR_CUDA_TRY(m->d_partials.reserve((size_t)pop * m->nblk * 6 * 8));
+      XR_CUDA_TRY(m->d_sims.reserve((size_t)pop * 4));
       FusedView V{};
       V.fhx = m->fx.fhat;
       V.fhy = m->fy.fhat;
@@ -2267,6 +2270,8 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
     gj.push_back(G);
     // the metric behind the DRR
     J.metric = obj_metric_fusable(obj) ? 1 : 0;
+    for (xr_simmetric m : obj->metrics)
+      XR_CHECK_ARG(!J.metric || m->capacity >= pop, "evaluation: metric buffers do not fit");
     if ((st = metric_job(obj, pop, J, fv[(size_t)i], s)) != XR_OK) return st;
     if (dopt) {
       J.report = d_report + i;
