@@ -473,18 +473,17 @@ __global__ void patch_fixed_stats_kernel(const float* __restrict__ img, int cols
   }
 }
 
-// Shared-memory layout for one tile of kPC x (kPC rb) patch centres (columns x
-// rows; dynamic): rb = patches scored per thread, stacked in a column.
+// Shared-memory layout of patch_ncc_kernel for one tile of kPC x kPC patch centres.
 struct PatchLayout {
   int Wr, Wc;    // patch-window region (moving gradient / fixed tiles)
   int WIr, WIc;  // staged input
   int WBr, WBc;  // blurred
   size_t fbytes;  // float part
   size_t bytes;   // plus the Wr x Wc mask tile
-  __host__ __device__ static PatchLayout make(int radius, int stride, int grad, int kr, int rb) {
+  __host__ __device__ static PatchLayout make(int radius, int stride, int grad, int kr) {
     PatchLayout L;
     L.Wc = (kPC - 1) * stride + 2 * radius + 1;
-    L.Wr = (kPC * rb - 1) * stride + 2 * radius + 1;
+    L.Wr = L.Wc;
     L.WBc = grad ? L.Wc + 2 : L.Wc;
     L.WBr = grad ? L.Wr + 2 : L.Wr;
     L.WIc = grad ? L.WBc + 2 * kr : L.Wc;
@@ -540,82 +539,20 @@ __device__ __forceinline__ float patch_var(const float* __restrict__ m, int P, i
   return sd * sd;
 }
 
-// RB vertically adjacent unmasked patches of one thread (tile-local rows
-// lr RB .. lr RB + RB - 1, column c0): each moving / fixed value is read once
-// from shared memory for every patch whose window holds it.  Per patch the
-// operations and their order are those of patch_score without a mask (sum in
-// row-major order, mean, then variance and covariance in row-major order), so
-// each score has the same bits.  DC / SC > 0: the patch edge and stride known
-// at compile time (xReg's default 11 x 11, stride 1): each row's columns unroll
-// (no loop control or address arithmetic per element).
-template <int RB, int DC, int SC>
-__device__ __forceinline__ void patch_scores_rows(const float* __restrict__ m, const float* __restrict__ f, int Wc,
-                                                  int rbase, int c0, int d_rt, int stride_rt,
-                                                  const float (&fmean)[RB], const float (&fscale)[RB],
-                                                  float (&score)[RB]) {
-  const int d = DC > 0 ? DC : d_rt;
-  const int stride = SC > 0 ? SC : stride_rt;
-  const int span = (RB - 1) * stride + d;
-  constexpr int kUnroll = DC > 0 ? DC : 1;  // the columns of a patch row (the rows stay a loop: registers)
-  float acc[RB], v[RB], cov[RB];
-#pragma unroll
-  for (int j = 0; j < RB; ++j) { acc[j] = 0.0f; v[j] = 0.0f; cov[j] = 0.0f; }
-#pragma unroll 1
-  for (int rr = 0; rr < span; ++rr) {
-    bool in[RB];
-#pragma unroll
-    for (int j = 0; j < RB; ++j) in[j] = rr >= j * stride && rr < j * stride + d;
-    const float* row = m + (rbase + rr) * Wc + c0;
-#pragma unroll kUnroll
-    for (int c = 0; c < d; ++c) {
-      const float x = row[c];
-#pragma unroll
-      for (int j = 0; j < RB; ++j)
-        if (in[j]) acc[j] += x;
-    }
-  }
-  const float n = (float)(d * d);
-  float mu[RB];
-#pragma unroll
-  for (int j = 0; j < RB; ++j) mu[j] = d * d > 1 ? acc[j] / n : acc[j];
-#pragma unroll 1
-  for (int rr = 0; rr < span; ++rr) {
-    bool in[RB];
-#pragma unroll
-    for (int j = 0; j < RB; ++j) in[j] = rr >= j * stride && rr < j * stride + d;
-    const int o = (rbase + rr) * Wc + c0;
-#pragma unroll kUnroll
-    for (int c = 0; c < d; ++c) {
-      const float x = m[o + c], fx = f[o + c];
-#pragma unroll
-      for (int j = 0; j < RB; ++j)
-        if (in[j]) {
-          const float dm = x - mu[j];
-          v[j] = fmaf(dm, dm, v[j]);
-          cov[j] = fmaf(dm, fx - fmean[j], cov[j]);
-        }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < RB; ++j) {
-    float sd = d * d > 1 ? sqrtf(v[j] / (n - 1.0f)) : 0.0f;
-    sd = fmaxf(sd, 1.0e-6f);
-    score[j] = 1.0f - (cov[j] / sd) * fscale[j];
-  }
-}
-
 // PASS 0: per image and direction, the sum over used patches with an unmasked
 // centre of count x moving-patch variance (the normaliser of variance weights).
 // PASS 1: per image and direction, the sum over used patches of
 // count x weight x score (weight 1 when not weighting in the combine).
-template <int GRAD, int KR, int PASS, int RB, int DC = 0, int SC = 0>
+// The general kernel, one patch per thread: moving-variance weights, masked
+// statistics, and tiles too large for patch_rows_kernel.
+template <int GRAD, int KR, int PASS>
 __global__ void __launch_bounds__(kThreads) patch_ncc_kernel(const float* __restrict__ imgs, int rows, int cols,
                                                              int radius, int stride, int ncr, int ncc,
                                                              PatchFixed px, PatchFixed py, PatchRun run,
                                                              double* __restrict__ partials) {
   extern __shared__ float sm[];
   __shared__ FF red[2 * 32];
-  const PatchLayout L = PatchLayout::make(radius, stride, GRAD, KR, RB);
+  const PatchLayout L = PatchLayout::make(radius, stride, GRAD, KR);
   const int Wr = L.Wr, Wc = L.Wc, WIr = L.WIr, WIc = L.WIc, WBr = L.WBr, WBc = L.WBc;
   const int WW = Wr * Wc;
   float* s_in = sm;                              // WIr x WIc
@@ -629,7 +566,7 @@ __global__ void __launch_bounds__(kThreads) patch_ncc_kernel(const float* __rest
 
   const int tiles_x = (ncc + kPC - 1) / kPC;
   const int tpr = blockIdx.x / tiles_x, tpc = blockIdx.x - tpr * tiles_x;
-  const int pr0 = tpr * kPC * RB, pc0 = tpc * kPC;
+  const int pr0 = tpr * kPC, pc0 = tpc * kPC;
   const int y0 = pr0 * stride, x0 = pc0 * stride;  // top-left pixel of the window region
   const int64_t npix = (int64_t)rows * cols;
   const int64_t img = blockIdx.y;
@@ -694,50 +631,7 @@ __global__ void __launch_bounds__(kThreads) patch_ncc_kernel(const float* __rest
   const int pc = pc0 + lc;
   const int d = 2 * radius + 1;
   const int c0 = lc * stride;
-  if (RB > 1) {
-    // several unmasked patches per thread, no moving-variance weights (the
-    // host picks this form only then); PASS 1 only
-    if (PASS == 1 && pc < ncc) {
-      int64_t pidx[RB];
-      int cnt[RB];
-      bool any = false;
-#pragma unroll
-      for (int j = 0; j < RB; ++j) {
-        const int pr = pr0 + lr * RB + j;
-        pidx[j] = (int64_t)pr * ncc + pc;
-        cnt[j] = pr < ncr ? (run.cnt ? run.cnt[pidx[j]] : 1) : 0;
-        any = any || cnt[j] > 0;
-      }
-      if (any) {
-        const int rbase = lr * RB * stride;
-        float kept[RB];  // per-patch score as xReg keeps it (0.5 (s_x + s_y) for GRAD)
-#pragma unroll
-        for (int j = 0; j < RB; ++j) kept[j] = 0.0f;
-        for (int k = 0; k < (GRAD ? 2 : 1); ++k) {
-          const PatchFixed& P = k == 0 ? px : py;
-          float fm[RB], fs[RB], sc[RB], w[RB];
-#pragma unroll
-          for (int j = 0; j < RB; ++j) {
-            fm[j] = cnt[j] > 0 ? P.mean[pidx[j]] : 0.0f;
-            fs[j] = cnt[j] > 0 ? P.scale[pidx[j]] : 0.0f;
-            w[j] = (cnt[j] > 0 && P.w) ? P.w[pidx[j]] : 1.0f;
-          }
-          patch_scores_rows<RB, DC, SC>(k == 0 ? s_mx : s_my, k == 0 ? s_fx : s_fy, Wc, rbase, c0, d, stride, fm,
-                                        fs, sc);
-#pragma unroll
-          for (int j = 0; j < RB; ++j)
-            if (cnt[j] > 0 && (!run.weighted || fabsf(w[j]) > 1.0e-6f)) {
-              v[k] = ff_add(v[k], ff_prod((float)cnt[j], (run.weighted ? w[j] : 1.0f) * sc[j]));
-              kept[j] += GRAD ? 0.5f * sc[j] : sc[j];
-            }
-        }
-        if (run.scores)
-#pragma unroll
-          for (int j = 0; j < RB; ++j)
-            if (cnt[j] > 0) run.scores[img * (int64_t)ncr * ncc + pidx[j]] = kept[j];
-      }
-    }
-  } else {
+  {
     const int pr = pr0 + lr;
     if (pr < ncr && pc < ncc) {
       const int64_t pidx = (int64_t)pr * ncc + pc;
@@ -799,6 +693,419 @@ __global__ void __launch_bounds__(kThreads) patch_ncc_kernel(const float* __rest
     double* o = partials + (img * gridDim.x + blockIdx.x) * 2;
     o[0] = t[0];
     o[1] = t[1];
+  }
+}
+
+// ---- patches stacked in a column (the common case) ----
+// A tile is 32 columns of patches by RB rows of them per warp; a thread scores RB patches
+// of one column, so a pixel is read once for all of them and their row sums give
+// every patch's mean.  Two channels run side by side as packed pairs (one
+// instruction for two, each lane rounded as the scalar one): the two gradients of an
+// image, or two images of the plain patch metric.  Per patch two passes as in
+// patch_score: the mean, then the deviations.  Bound by the FP32 pipe (4 operations a
+// pixel, patch and channel) and by 16 warps an SM, which the registers allow.  20
+// images of 768^2, 11 x 11, both gradients: 1175 us one channel at a time, now 667; 24
+// plain images of 384^2: 180 us, now 102; 8 images of 187 x 118 at stride 3, a whole
+// call: 55 us, now 48.
+// Every RB takes the same operations in the same order, patch by patch and up to the
+// partial sums (one for 16 rows of patches), so an image's value does not depend on
+// how many others share the launch.
+// Pixel x of a row lies at (x mod stride) Wp + x / stride, so that the lanes of a
+// read (one patch column each) are neighbours for every stride.
+constexpr int kPartRows = 8;
+
+struct PatchRows {
+  int Wr, Wc, Wp, P;  // the tile's pixels, columns of a residue, pitch (stride Wp)
+  int edge;           // of a patch, as offsets of its columns (four at a time; first in memory)
+  size_t bytes;
+  __host__ __device__ static PatchRows make(int radius, int stride, int grad, bool mask, int rb) {
+    PatchRows L;
+    L.Wc = 31 * stride + 2 * radius + 1;
+    L.Wr = (8 * rb - 1) * stride + 2 * radius + 1;
+    L.Wp = (L.Wc + stride - 1) / stride;
+    L.P = stride * L.Wp;
+    L.edge = (2 * radius + 4) & ~3;
+    const int words = grad ? 4 : (rb > 1 ? 3 : 2);  // the moving side, in pairs but for rb 1, and the fixed one
+    L.bytes = (size_t)L.edge * 4 + (size_t)L.Wr * L.P * 4 * (words + (mask ? 1 : 0));
+    return L;
+  }
+};
+
+typedef unsigned long long u64;
+
+// the same for one channel: the first value
+template <typename V>
+__device__ __forceinline__ V pack2(float a, float b) {
+  if constexpr (sizeof(V) == 4) return a;
+  else {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+  }
+}
+__device__ __forceinline__ float2 unpack2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float add2(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float fma2(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float2 unpack2(u64 r) {
+  float2 v;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
+  return v;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+  u64 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+  u64 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// body(std::integral_constant<int, N>, offsets) for the columns of a patch row, in
+// order, N at a time: all at once where edge and stride (1 or 2) are known, else in fours
+template <int DC, int SC, typename Body>
+__device__ __forceinline__ void patch_columns(int d, int Wp, const int4* __restrict__ offs, Body body) {
+  if constexpr (DC > 0) {
+    int o[DC];
+#pragma unroll
+    for (int c = 0; c < DC; ++c) o[c] = (c % SC) * Wp + c / SC;
+    body(std::integral_constant<int, DC>(), o);
+  } else {
+    int c = 0;
+#pragma unroll 1
+    for (; c + 4 <= d; c += 4) {
+      const int4 q = offs[c >> 2];
+      const int o[4] = {q.x, q.y, q.z, q.w};
+      body(std::integral_constant<int, 4>(), o);
+    }
+    const int4 q = offs[c >> 2];  // d is odd
+    if (d & 2) {
+      const int o[3] = {q.x, q.y, q.z};
+      body(std::integral_constant<int, 3>(), o);
+    } else {
+      const int o[1] = {q.x};
+      body(std::integral_constant<int, 1>(), o);
+    }
+  }
+}
+
+// Scores of RB stacked patches in both channels; their first window starts at m[0]
+// (V: a pair of channels, or one), f[0] (as m, or FS: one value for both), mk[0] (MASK: 1 or 0 per
+// pixel, f zero where it is 0), row pitch P.  DC and SC: the patch edge and stride when
+// known.  scale(j): the patch's 1 / sd of the fixed side, per channel.
+template <typename V, int RB, int DC, int SC, bool MASK, bool FS, typename Scale>
+__device__ __forceinline__ void patch_column_scores(const V* __restrict__ m, const void* __restrict__ f,
+                                                    const float* __restrict__ mk, int P, int Wp, const int4* __restrict__ offs,
+                                                    int d_rt, int stride_rt, const V (&fmean)[RB], Scale scale,
+                                                    float2 (&score)[RB]) {
+  const int d = DC > 0 ? DC : d_rt, stride = DC > 0 ? SC : stride_rt;
+  const int span = (RB - 1) * stride + d;
+  auto fixed = [&](int i) -> V {
+    if constexpr (FS) {
+      const float v = static_cast<const float*>(f)[i];
+      return pack2<V>(v, v);
+    } else {
+      return static_cast<const V*>(f)[i];
+    }
+  };
+  V mu[RB], v[RB], cov[RB];
+#pragma unroll
+  for (int j = 0; j < RB; ++j) mu[j] = v[j] = cov[j] = V(0);
+#pragma unroll 1
+  for (int r = 0; r < span; ++r) {
+    const V* row = m + r * P;
+    V h = V(0);
+    patch_columns<DC, SC>(d, Wp, offs, [&](auto count, auto& o) {
+      V x[count.value];
+#pragma unroll
+      for (int c = 0; c < count.value; ++c) x[c] = row[o[c]];
+#pragma unroll
+      for (int c = 0; c < count.value; ++c) h = add2(h, x[c]);
+    });
+#pragma unroll
+    for (int j = 0; j < RB; ++j)
+      if (r >= j * stride && r < j * stride + d) mu[j] = add2(mu[j], h);
+  }
+  const float n = (float)(d * d);
+#pragma unroll
+  for (int j = 0; j < RB; ++j) {  // negated
+    const float2 t = unpack2(mu[j]);
+    mu[j] = d > 1 ? pack2<V>(-(t.x / n), -(t.y / n)) : pack2<V>(-t.x, -t.y);
+  }
+#pragma unroll 1
+  for (int r = 0; r < span; ++r) {
+    const int row = r * P;
+    patch_columns<DC, SC>(d, Wp, offs, [&](auto count, auto& o) {
+      constexpr int N = count.value;
+      V x[N], y[N], k[N];  // k: the mask twice
+#pragma unroll
+      for (int c = 0; c < N; ++c) {
+        x[c] = m[row + o[c]];
+        y[c] = fixed(row + o[c]);
+        k[c] = MASK ? pack2<V>(mk[row + o[c]], mk[row + o[c]]) : V(0);
+      }
+#pragma unroll
+      for (int j = 0; j < RB; ++j)
+        if (r >= j * stride && r < j * stride + d) {
+#pragma unroll
+          for (int c = 0; c < N; ++c) {
+            const V dm = add2(x[c], mu[j]), e = MASK ? fma2(k[c], fmean[j], y[c]) : add2(y[c], fmean[j]);
+            v[j] = fma2(dm, dm, v[j]);
+            cov[j] = fma2(dm, e, cov[j]);
+          }
+        }
+    });
+  }
+  if constexpr (MASK) {
+    // a masked-out pixel must not count, also where its product with 0 is not 0
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+      const float2 vv = unpack2(v[j]), fm = unpack2(fmean[j]), mj = unpack2(mu[j]);
+      if (isfinite(vv.x) && isfinite(vv.y) && isfinite(fm.x) && isfinite(fm.y)) continue;
+      float2 c2 = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+      for (int r = j * stride; r < j * stride + d; ++r)
+#pragma unroll 1
+        for (int c = 0; c < d; ++c) {
+          const int i = r * P + reinterpret_cast<const int*>(offs)[c];
+          if (mk[i] == 0.0f) continue;
+          const float2 x = unpack2(m[i]), y = unpack2(fixed(i));
+          c2.x = fmaf(x.x + mj.x, y.x + fm.x, c2.x);
+          c2.y = fmaf(x.y + mj.y, y.y + fm.y, c2.y);
+        }
+      cov[j] = pack2<V>(c2.x, c2.y);
+    }
+  }
+  auto value = [&](float vv, float cc, float sc) -> float {
+    float sd = d > 1 ? sqrtf(vv / (n - 1.0f)) : 0.0f;
+    sd = fmaxf(sd, 1.0e-6f);
+    return 1.0f - (cc / sd) * sc;
+  };
+#pragma unroll
+  for (int j = 0; j < RB; ++j) {
+    const float2 vv = unpack2(v[j]), cc = unpack2(cov[j]), fs = scale(j);
+    score[j] = make_float2(value(vv.x, cc.x, fs.x), value(vv.y, cc.y, fs.y));
+  }
+}
+
+// Gradients of the moving image over the tile (top-left pixel x0, y0): a warp goes
+// down 32 columns of a quarter of the rows, horizontal neighbours by shuffles, vertical
+// ones in registers (as gt::grad_tile_moments).
+template <int KR, typename At>
+__device__ __forceinline__ void patch_tile_gradients(const float* __restrict__ src, int rows, int cols, int y0, int x0,
+                                                     const PatchRows& L, At at, float2* __restrict__ s_m) {
+  constexpr int H = KR + 1, kWin = 2 * KR + 1, kOut = 32 - 2 * H;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int strips = (L.Wc + kOut - 1) / kOut, chunk = (L.Wr + 3) / 4;
+  for (int u = warp; u < strips * 4; u += kThreads / 32) {
+    const int c0 = (u % strips) * kOut, r0 = (u / strips) * chunk, r1 = min(r0 + chunk, L.Wr);
+    const int c = c0 - H + lane;
+    const float* pc = src + reflect101(min(x0 + c, cols - 1 + H), cols);
+    const bool owner = lane >= H && lane < 32 - H && c < L.Wc;
+    const int ic = owner ? at(c) : 0;
+    float hb[kWin], bl[3], lf[3], rt[3];
+#pragma unroll
+    for (int i = 0; i < kWin; ++i) hb[i] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) bl[i] = lf[i] = rt[i] = 0.0f;
+    for (int rb = r0 - 2 * H; rb < r1; rb += 8) {  // output rows rb .., from input rows rb + H ..
+      float p[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        p[i] = __ldg(pc + (int64_t)reflect101(min(y0 + rb + i + H, rows - 1 + H), rows) * cols);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float h = p[i];
+        if constexpr (KR == 2)
+          h = gt::blur5(__shfl_up_sync(0xffffffffu, p[i], 2), __shfl_up_sync(0xffffffffu, p[i], 1), p[i],
+                        __shfl_down_sync(0xffffffffu, p[i], 1), __shfl_down_sync(0xffffffffu, p[i], 2));
+        else if constexpr (KR == 1)
+          h = gt::blur3(__shfl_up_sync(0xffffffffu, p[i], 1), p[i], __shfl_down_sync(0xffffffffu, p[i], 1));
+#pragma unroll
+        for (int k = 0; k + 1 < kWin; ++k) hb[k] = hb[k + 1];
+        hb[kWin - 1] = h;
+        bl[0] = bl[1]; bl[1] = bl[2];
+        lf[0] = lf[1]; lf[1] = lf[2];
+        rt[0] = rt[1]; rt[1] = rt[2];
+        if constexpr (KR == 2) bl[2] = gt::blur5(hb[0], hb[1], hb[2], hb[3], hb[4]);
+        else if constexpr (KR == 1) bl[2] = gt::blur3(hb[0], hb[1], hb[2]);
+        else bl[2] = hb[0];
+        lf[2] = __shfl_up_sync(0xffffffffu, bl[2], 1);
+        rt[2] = __shfl_down_sync(0xffffffffu, bl[2], 1);
+        const int r = rb + i;
+        if (owner && r >= r0 && r < r1) {
+          float gx, gy;
+          gt::sobel3(lf[0], bl[0], rt[0], lf[1], rt[1], lf[2], bl[2], rt[2], gx, gy);
+          s_m[r * L.P + ic] = make_float2(gx, gy);
+        }
+      }
+    }
+  }
+}
+
+// Grid: tiles, then images (GRAD, RB 1) or pairs of images; kr: the blur's radius (GRAD).
+// Partials: per image, sums over kPartRows rows by 32 columns of patches, nblk of them.
+template <int GRAD, int RB, int DC, int SC, bool MASK>
+__global__ void __launch_bounds__(kThreads, RB == 1 ? 3 : 2)
+patch_rows_kernel(const float* __restrict__ imgs, int rows, int cols, int64_t nimgs, int kr, int radius, int stride_rt,
+                  int ncr, int ncc, PatchFixed px, PatchFixed py, PatchRun run,
+                  double* __restrict__ partials, int nblk) {
+  constexpr int kWarps = kThreads / 32;
+  constexpr bool kPairs = !GRAD && RB > 1;
+  using V = std::conditional_t<GRAD || kPairs, u64, float>;
+  extern __shared__ int4 smp[];
+  __shared__ FF red[2][kThreads];
+  const int stride = DC > 0 ? SC : stride_rt;
+  const PatchRows L = PatchRows::make(radius, stride, GRAD, MASK, RB);
+  const int size = L.Wr * L.P;
+  int* s_off = reinterpret_cast<int*>(smp);
+  V* s_m = reinterpret_cast<V*>(s_off + L.edge);
+  float2* s_f = reinterpret_cast<float2*>(s_m + size);   // GRAD
+  float* s_f1 = reinterpret_cast<float*>(s_f);           // plain
+  float* s_mk = GRAD ? reinterpret_cast<float*>(s_f + size) : s_f1 + size;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tiles_x = (ncc + 31) / 32;
+  const int tpr = blockIdx.x / tiles_x, tpc = blockIdx.x - tpr * tiles_x;
+  const int pr0 = tpr * kWarps * RB, pc0 = tpc * 32;
+  const int y0 = pr0 * stride, x0 = pc0 * stride;  // top-left pixel of the tile
+  const int64_t npix = (int64_t)rows * cols;
+  const int64_t img = kPairs ? 2 * (int64_t)blockIdx.y : (int64_t)blockIdx.y;
+  const bool pair = kPairs && img + 1 < nimgs;  // a last image alone fills both channels
+  const float* src = imgs + img * npix;
+  auto at = [&](int x) -> int {
+    const int q = x / stride;
+    return (x - q * stride) * L.Wp + q;
+  };
+  if (threadIdx.x < L.edge) s_off[threadIdx.x] = at(threadIdx.x);
+
+  // the fixed side, the mask and (plain patches) the images, 32 pixels of a row per
+  // warp and four such pieces in flight; past the image the last pixel, which only
+  // patches outside the grid read
+  const int pieces = (L.Wc + 31) / 32, units = L.Wr * pieces;
+  for (int u0 = warp; u0 < units; u0 += 4 * kWarps) {
+    float a[4], b[4];
+    bool in[4];
+    int at_i[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int u = u0 + k * kWarps, r = u / pieces, c = (u - r * pieces) * 32 + lane;
+      const int64_t g = (int64_t)min(y0 + r, rows - 1) * cols + min(x0 + c, cols - 1);
+      at_i[k] = (u < units && c < L.Wc) ? r * L.P + at(c) : -1;
+      in[k] = !MASK || run.mask[g];
+      a[k] = __ldg(px.img + g);
+      b[k] = GRAD ? __ldg(py.img + g) : __ldg(src + g);
+      if constexpr (GRAD == 0) {
+        const float b1 = pair ? __ldg(src + npix + g) : b[k];
+        if (at_i[k] >= 0) s_m[at_i[k]] = pack2<V>(b[k], b1);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (at_i[k] < 0) continue;
+      if constexpr (GRAD != 0) s_f[at_i[k]] = in[k] ? make_float2(a[k], b[k]) : make_float2(0.0f, 0.0f);
+      else s_f1[at_i[k]] = in[k] ? a[k] : 0.0f;
+      if constexpr (MASK) s_mk[at_i[k]] = in[k] ? 1.0f : 0.0f;
+    }
+  }
+  if constexpr (GRAD != 0) {
+    if (kr == 2) patch_tile_gradients<2>(src, rows, cols, y0, x0, L, at, reinterpret_cast<float2*>(s_m));
+    else if (kr == 1) patch_tile_gradients<1>(src, rows, cols, y0, x0, L, at, reinterpret_cast<float2*>(s_m));
+    else patch_tile_gradients<0>(src, rows, cols, y0, x0, L, at, reinterpret_cast<float2*>(s_m));
+  }
+  __syncthreads();
+
+  FF v[RB][2];
+#pragma unroll
+  for (int j = 0; j < RB; ++j) v[j][0] = v[j][1] = FF{0.0f, 0.0f};
+  const int pc = pc0 + lane, prw = pr0 + warp * RB;
+  if (pc < ncc && prw < ncr) {
+    int cnt[RB];
+    bool any = false;
+    const int64_t pidx = (int64_t)prw * ncc + pc;
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+      cnt[j] = prw + j < ncr ? (run.cnt ? run.cnt[pidx + (int64_t)j * ncc] : 1) : 0;
+      any = any || cnt[j] > 0;
+    }
+    if (any) {
+      const int o = warp * RB * stride * L.P + lane;
+      V fm[RB];
+      float2 sc[RB];
+      const PatchFixed& p1 = GRAD ? py : px;  // the second channel's fixed side
+#pragma unroll
+      for (int j = 0; j < RB; ++j) {
+        const int64_t i = pidx + (int64_t)j * ncc;
+        fm[j] = cnt[j] > 0 ? pack2<V>(-px.mean[i], -p1.mean[i]) : V(0);
+      }
+      const void* f0 = GRAD ? static_cast<const void*>(s_f + o) : static_cast<const void*>(s_f1 + o);
+      patch_column_scores<V, RB, DC, SC, MASK, GRAD == 0>(
+          s_m + o, f0, s_mk + o, L.P, L.Wp, smp, 2 * radius + 1, stride, fm,
+          [&](int j) -> float2 {
+            const int64_t i = pidx + (int64_t)j * ncc;
+            return prw + j < ncr ? make_float2(px.scale[i], p1.scale[i]) : make_float2(0.0f, 0.0f);
+          },
+          sc);
+#pragma unroll
+      for (int j = 0; j < RB; ++j) {
+        if (prw + j >= ncr) continue;
+        const int64_t i = pidx + (int64_t)j * ncc;
+        const int count = RB > 2 ? (run.cnt ? run.cnt[i] : 1) : cnt[j];
+        if (count <= 0) continue;
+        const float w[2] = {px.w ? px.w[i] : 1.0f, p1.w ? p1.w[i] : 1.0f};
+        const float s2[2] = {sc[j].x, sc[j].y};
+        float kept[2] = {0.0f, 0.0f};  // per-patch score as xReg keeps it (0.5 (s_x + s_y) for GRAD)
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          if (!run.weighted || fabsf(w[k]) > 1.0e-6f) {
+            v[j][k] = ff_prod((float)count, (run.weighted ? w[k] : 1.0f) * s2[k]);
+            kept[GRAD ? 0 : k] += GRAD ? 0.5f * s2[k] : s2[k];
+          }
+        if (run.scores) {
+          const int64_t np = (int64_t)ncr * ncc;
+          run.scores[img * np + i] = kept[0];
+          if (pair) run.scores[(img + 1) * np + i] = kept[1];
+        }
+      }
+    }
+  }
+  // sums by halves: a thread's rows, the warps of a part, the lanes
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+#pragma unroll
+    for (int h = 1; h < RB; h *= 2)
+#pragma unroll
+      for (int j = 0; j < RB; j += 2 * h) v[j][k] = ff_add(v[j][k], v[j + h][k]);
+    red[k][threadIdx.x] = v[0][k];
+  }
+  __syncthreads();
+  constexpr int kPart = kPartRows / RB;  // warps of a part
+  const int part_row = tpr * (kWarps / kPart) + warp;
+  if (warp < kWarps / kPart && part_row * kPartRows < ncr) {
+    double t[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      FF w[kPart];
+#pragma unroll
+      for (int i = 0; i < kPart; ++i) w[i] = red[k][(warp * kPart + i) * 32 + lane];
+#pragma unroll
+      for (int h = 1; h < kPart; h *= 2)
+#pragma unroll
+        for (int i = 0; i < kPart; i += 2 * h) w[i] = ff_add(w[i], w[i + h]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) w[0] = ff_add(w[0], ff_shfl_down(w[0], o));
+      t[k] = (double)w[0].hi + (double)w[0].lo;
+    }
+    if (lane == 0) {
+      double* o = partials + (img * nblk + part_row * tiles_x + tpc) * 2;
+      o[0] = t[0];
+      o[1] = GRAD ? t[1] : 0.0;
+      if (pair) {
+        o += 2 * (int64_t)nblk;
+        o[0] = t[1];
+        o[1] = 0.0;
+      }
+    }
   }
 }
 
@@ -980,49 +1287,110 @@ cudaError_t launch_patch_fixed_stats(const float* img, int rows, int cols, int r
   return cudaGetLastError();
 }
 
-// Patches scored per thread: four stacked in a column when no mask and no
-// moving-variance weight is involved and the taller tile fits, else one.
-constexpr int kPatchRows = 4;
-static int patch_rb(int radius, int stride, int grad, int kr, const PatchRun& run) {
-  if (run.mask || run.mvar) return 1;
-  return PatchLayout::make(radius, stride, grad, kr, kPatchRows).bytes <= 112 * 1024 ? kPatchRows : 1;
+// Patches a thread scores in a column (patch_rows_kernel).  One while a patch a thread
+// does not fill the GPU (1024 threads an SM): more would leave SMs idle (6 images of
+// 311 x 476, 15 x 15 at stride 3, a whole call: 56 us against 81 with four; 16 of 215 x
+// 493, 11 x 11 at stride 2, above the line: 79 against 70).  Eight from two waves of blocks on
+// where the tile fits shared memory twice and no mask takes registers (20 images of
+// 768^2, both gradients: 667 us against 742); else four.  The general kernel with masked
+// statistics, moving-variance weights or tiles too large.
+constexpr size_t kPatchSmem = 200 * 1024;
+
+static size_t patch_rows_bytes(int radius, int stride, int grad, const PatchRun& run, int rb) {
+  return PatchRows::make(radius, stride, grad, run.mask != nullptr, rb).bytes;
 }
 
-static int patch_tiles(int ncr, int ncc, int rb) {
-  return ((ncr + kPC * rb - 1) / (kPC * rb)) * ((ncc + kPC - 1) / kPC);
+static bool patch_general(int radius, int stride, int grad, const PatchRun& run) {
+  return run.mvar || (run.mask && (run.use_mask_stats || !run.mask_in_sums)) ||
+         patch_rows_bytes(radius, stride, grad, run, 1) > kPatchSmem;
 }
 
-int patch_ncc_max_blocks(int ncr, int ncc) { return patch_tiles(ncr, ncc, 1); }
+// tiles of `rows` by 32 patches
+static int patch_tiles(int ncr, int ncc, int rows) { return ((ncr + rows - 1) / rows) * ((ncc + 31) / 32); }
+
+static int patch_general_tiles(int ncr, int ncc) { return ((ncr + kPC - 1) / kPC) * ((ncc + kPC - 1) / kPC); }
+
+static cudaError_t patch_rb(int radius, int stride, int grad, const PatchRun& run, int ncr, int ncc, int64_t nimgs,
+                            int* rb) {
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int64_t pairs = grad ? nimgs : (nimgs + 1) / 2;
+  *rb = 1;
+  if ((int64_t)ncr * ncc * nimgs <= (int64_t)sms * 1024) return e;
+  if (patch_rows_bytes(radius, stride, grad, run, 4) <= kPatchSmem) *rb = 4;
+  if (!run.mask && patch_rows_bytes(radius, stride, grad, run, 8) <= kPatchSmem / 2 &&
+      patch_tiles(ncr, ncc, 64) * pairs >= 4 * sms)
+    *rb = 8;
+  return e;
+}
+
+int patch_ncc_max_blocks(int ncr, int ncc) {
+  return max(patch_general_tiles(ncr, ncc), patch_tiles(ncr, ncc, kPartRows));
+}
+
+template <int GRAD, int RB, int DC, int SC, bool MASK>
+static cudaError_t launch_rows(const float* mov, int rows, int cols, int kr, int radius, int stride, int ncr, int ncc,
+                               int64_t nimgs, const PatchFixed& px, const PatchFixed& py, const PatchRun& run,
+                               double* partials, int nblk, cudaStream_t s) {
+  const size_t bytes = patch_rows_bytes(radius, stride, GRAD, run, RB);
+  const cudaError_t e = set_smem(patch_rows_kernel<GRAD, RB, DC, SC, MASK>, bytes);
+  if (e != cudaSuccess) return e;
+  const dim3 grid(patch_tiles(ncr, ncc, 8 * RB), (unsigned)(!GRAD && RB > 1 ? (nimgs + 1) / 2 : nimgs));
+  patch_rows_kernel<GRAD, RB, DC, SC, MASK><<<grid, kThreads, bytes, s>>>(mov, rows, cols, nimgs, kr, radius, stride, ncr,
+                                                                     ncc, px, py, run, partials, nblk);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_patch_ncc(const float* mov, int rows, int cols, int64_t nimgs, int grad, int smooth_ksize,
                              int radius, int stride, int ncr, int ncc, PatchFixed px, PatchFixed py, PatchRun run,
                              int pass, double* partials, cudaStream_t s, int* nblk_out) {
   const int kr = smooth_ksize == 5 ? 2 : (smooth_ksize == 3 ? 1 : 0);
   if (smooth_ksize != 0 && smooth_ksize != 3 && smooth_ksize != 5) return cudaErrorInvalidValue;
-  const int rb = patch_rb(radius, stride, grad, kr, run);
-  const int tiles = patch_tiles(ncr, ncc, rb);
-  if (nblk_out) *nblk_out = tiles;
+  const bool general = patch_general(radius, stride, grad, run);
+  const int nblk = general ? patch_general_tiles(ncr, ncc) : patch_tiles(ncr, ncc, kPartRows);
+  if (nblk_out) *nblk_out = nblk;
   if (nimgs <= 0 || !partials) return cudaSuccess;
-  if (rb > 1 && pass != 1) return cudaErrorInvalidValue;
-  const PatchLayout L = PatchLayout::make(radius, stride, grad, kr, rb);
-  if (L.bytes > 200 * 1024) return cudaErrorInvalidValue;
-  const dim3 grid(tiles, (unsigned)nimgs);
+  if (!general) {
+    if (pass != 1) return cudaErrorInvalidValue;
+    int rb = 1;
+    const cudaError_t e = patch_rb(radius, stride, grad, run, ncr, ncc, nimgs, &rb);
+    if (e != cudaSuccess) return e;
+    // the columns of xReg's default patches (11 x 11) unroll at strides 1 and 2 (24 masked
+    // images of 384^2 at stride 2, a whole call: 66 us against 95 by fours)
+#define XR_ROWS(G, R, D, S, M) \
+  return launch_rows<G, R, D, S, M>(mov, rows, cols, kr, radius, stride, ncr, ncc, nimgs, px, py, run, partials, nblk, s)
+#define XR_ROWS_R(G, R, M)                                 \
+  if (radius == 5 && stride == 1) XR_ROWS(G, R, 11, 1, M); \
+  if (radius == 5 && stride == 2) XR_ROWS(G, R, 11, 2, M); \
+  XR_ROWS(G, R, 0, 0, M)
+#define XR_ROWS_G(G)                                 \
+  if (run.mask && rb == 1) { XR_ROWS_R(G, 1, true); } \
+  if (run.mask) { XR_ROWS_R(G, 4, true); }            \
+  if (rb == 1) { XR_ROWS_R(G, 1, false); }            \
+  if (rb == 4) { XR_ROWS_R(G, 4, false); }            \
+  XR_ROWS_R(G, 8, false)
+    if (grad) { XR_ROWS_G(1); }
+    XR_ROWS_G(0);
+#undef XR_ROWS_G
+#undef XR_ROWS_R
+#undef XR_ROWS
+  }
+  const dim3 grid(nblk, (unsigned)nimgs);
+  const PatchLayout L = PatchLayout::make(radius, stride, grad, kr);
+  if (L.bytes > kPatchSmem) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
-#define XR_PATCH_R4_11_1 kPatchRows, 11, 1  // xReg's default patches: 11 x 11, stride 1
-#define XR_PATCH_LAUNCH(G, K, P, ...)                                                                        \
-  e = set_smem(patch_ncc_kernel<G, K, P, __VA_ARGS__>, L.bytes);                                            \
-  if (e != cudaSuccess) return e;                                                                            \
-  patch_ncc_kernel<G, K, P, __VA_ARGS__><<<grid, kThreads, L.bytes, s>>>(mov, rows, cols, radius, stride, ncr, ncc, \
-                                                                         px, py, run, partials);
-#define XR_PATCH_PASS(G, K)                                   \
-  if (rb > 1 && radius == 5 && stride == 1) {                 \
-    XR_PATCH_LAUNCH(G, K, 1, XR_PATCH_R4_11_1)                \
-  } else if (rb > 1) {                                        \
-    XR_PATCH_LAUNCH(G, K, 1, kPatchRows)                      \
-  } else if (pass == 0) {                                     \
-    XR_PATCH_LAUNCH(G, K, 0, 1)                               \
-  } else {                                                    \
-    XR_PATCH_LAUNCH(G, K, 1, 1)                               \
+#define XR_PATCH_LAUNCH(G, K, P)                                                                                       \
+  e = set_smem(patch_ncc_kernel<G, K, P>, L.bytes);                                                                    \
+  if (e != cudaSuccess) return e;                                                                                      \
+  patch_ncc_kernel<G, K, P><<<grid, kThreads, L.bytes, s>>>(mov, rows, cols, radius, stride, ncr, ncc, px, py, run,    \
+                                                            partials);
+#define XR_PATCH_PASS(G, K)    \
+  if (pass == 0) {             \
+    XR_PATCH_LAUNCH(G, K, 0)   \
+  } else {                     \
+    XR_PATCH_LAUNCH(G, K, 1)   \
   }
   if (!grad) {
     XR_PATCH_PASS(0, 0)
@@ -1035,7 +1403,6 @@ cudaError_t launch_patch_ncc(const float* mov, int rows, int cols, int64_t nimgs
   }
 #undef XR_PATCH_PASS
 #undef XR_PATCH_LAUNCH
-#undef XR_PATCH_R4_11_1
   return cudaGetLastError();
 }
 
