@@ -39,7 +39,7 @@ def test_hu_to_mu_is_the_double_result(xr):
 
 
 # edges of the build's 32 x 16 x 32 tiles, of 8^3 macro cells and of 1024-voxel row segments
-@pytest.mark.parametrize("size", [(2, 2, 2), (31, 15, 32), (32, 16, 31), (33, 17, 65), (1023, 3, 9), (1033, 9, 10)])
+@pytest.mark.parametrize("size", [(2, 2, 2), (31, 15, 32), (32, 16, 31), (33, 17, 65), (1023, 3, 9), (1033, 9, 10), (516, 9, 17), (1028, 17, 9)])
 @pytest.mark.parametrize("vt,tol", [(0, 1e-4), (1, 2e-3), (2, 2.0 ** -8)])
 def test_sparse_volumes(xr, oracle, size, vt, tol):
     """Few non-zero voxels, corners among them: skipping loses none of them, the

@@ -66,67 +66,103 @@ constexpr int kSegBits = kSegX / 8 + 2;       // macro cells they reach along x,
 constexpr int kSegWords = (kSegBits + 31) / 32;
 
 // A block takes 8 x 8 rows (one macro cell in y and z) of kSegX voxels, a warp a
-// row at a time: the ballot of non-zero voxels gives the macro cells along x, the
-// row's place in its macro cell those along y and z.  A macro cell m is occupied
+// row at a time and a lane four neighbours of every 128: ballots of the lanes with a
+// non-zero voxel (any, the last, one of the first two) give the macro cells along x,
+// the row's place in its macro cell those along y and z.  A macro cell m is occupied
 // when a voxel in [8m - 1, 8m + 9] on every axis is not zero (VolView::occ).  One
 // read of the volume where the largest magnitude, the box and the occupancy took
-// one each (58 + 268 + 372 us for 512 x 512 x 300, now 97).
+// one each (58 + 268 + 372 us for 512 x 512 x 300).  Its reads would take 46 us; with
+// a ballot per 32 voxels it was bound by instructions at 97, with the box's atomics
+// per warp (they all meet in one L2 sector) at 91, now 63.  VEC: rows start on 16 bytes.
+template <bool VEC>
 __global__ void __launch_bounds__(kThreads) volume_stats_kernel(const float* __restrict__ vox, int nx, int ny, int nz,
                                                                 int nxs, int nyb, uint32_t* __restrict__ occ, int nmx,
                                                                 int nmy, int nmz, VolStats* __restrict__ stats) {
   __shared__ uint32_t bits[3][3][kSegWords];  // macro cells (z, y) - 1 .. + 1 around the block's, x from 128 xs - 1
+  __shared__ unsigned int found[7];  // as VolStats: largest magnitude, box
   for (int i = threadIdx.x; i < 9 * kSegWords; i += kThreads) (&bits[0][0][0])[i] = 0u;
+  if (threadIdx.x < 7) found[threadIdx.x] = 0u;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int xs = (int)(blockIdx.x % nxs), yb = (int)(blockIdx.x / nxs % nyb), zb = (int)(blockIdx.x / nxs / nyb);
   const int x0 = xs * kSegX, xe = min(nx, x0 + kSegX);
-  // the chunk's macro cells this lane reports (lanes 0..5: j = lane - 1): voxels 8j - 1 .. 8j + 9 of the chunk
-  const int wl = 8 * (lane - 1) - 1;
-  const uint32_t window = lane > 5 ? 0u : wl >= 0 ? 0x7ffu << wl : 0x7ffu >> -wl;
-  unsigned int mx = 0;
+  float mx = 0.0f;
   int lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {-1, -1, -1};
   for (int r = warp; r < 64; r += kThreads / 32) {
     const int ry = r & 7, rz = r >> 3, y = yb * 8 + ry, z = zb * 8 + rz;
     if (y >= ny || z >= nz) continue;
     const float* row = vox + ((int64_t)z * ny + y) * nx;
-    for (int xc = x0; xc < xe; xc += 256) {
-      float v[8];
+    for (int xc = x0; xc < xe; xc += 512) {
+      float v[4][4];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int x = xc + 32 * k + lane;
-        v[k] = x < xe ? __ldg(row + x) : 0.0f;
+      for (int k = 0; k < 4; ++k) {
+        const int x = xc + 128 * k + 4 * lane;
+        if constexpr (VEC) {
+          const float4 q = x < xe ? __ldg(reinterpret_cast<const float4*>(row + x)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          v[k][0] = q.x; v[k][1] = q.y; v[k][2] = q.z; v[k][3] = q.w;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) v[k][i] = x + i < xe ? __ldg(row + x + i) : 0.0f;
+        }
       }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float a = fabsf(v[k]);
-        if (a == a) mx = max(mx, __float_as_uint(a));
-        const uint32_t m = __ballot_sync(0xffffffffu, v[k] != 0.0f);
-        if (!m) continue;
-        const int xk = xc + 32 * k;
-        lo[0] = min(lo[0], xk + __ffs(m) - 1);
-        hi[0] = max(hi[0], xk + 31 - __clz(m));
+      for (int k = 0; k < 4; ++k) {
+        uint32_t w[4];  // not zero: but for the sign a bit is set (a NaN too)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          mx = fmaxf(mx, fabsf(v[k][i]));  // passes over NaN
+          w[i] = __float_as_uint(v[k][i]);
+        }
+        const bool some = ((w[0] | w[1] | w[2] | w[3]) << 1) != 0u;
+        const uint32_t any = __ballot_sync(0xffffffffu, some);
+        if (!any) continue;
+        const uint32_t last = __ballot_sync(0xffffffffu, (w[3] << 1) != 0u);
+        const uint32_t first2 = __ballot_sync(0xffffffffu, ((w[0] | w[1]) << 1) != 0u);
+        const int xk = xc + 128 * k, x = xk + 4 * lane;
+        if (some && (x < lo[0] || x + 3 > hi[0]))
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if ((w[i] << 1) != 0u) {
+              lo[0] = min(lo[0], x + i);
+              hi[0] = max(hi[0], x + i);
+            }
         lo[1] = min(lo[1], y); hi[1] = max(hi[1], y);
         lo[2] = min(lo[2], z); hi[2] = max(hi[2], z);
-        if (m & window) {
-          const int b = (xk - x0) / 8 + lane;  // bit 0: macro cell 128 xs - 1
-          const uint32_t bit = 1u << (b & 31);
-          for (int dz = rz < 2 ? 0 : 1; dz <= (rz == 7 ? 2 : 1); ++dz)
-            for (int dy = ry < 2 ? 0 : 1; dy <= (ry == 7 ? 2 : 1); ++dy)
-              if (!(bits[dz][dy][b >> 5] & bit)) atomicOr(&bits[dz][dy][b >> 5], bit);
+        // lane j reports the chunk's macro cell j - 1: its lanes 2j - 2 and 2j - 1, the last voxel of
+        // lane 2j - 3 and the first two of lane 2j
+        const int s = 2 * lane - 3;
+        const bool set = lane < 18 && ((((s >= 0 ? any >> s : any << -s) & 6u) | ((s >= 0 ? last >> s : last << -s) & 1u)) != 0u ||
+                                       (lane < 16 && ((first2 >> (2 * lane)) & 1u)));
+        const uint32_t m18 = __ballot_sync(0xffffffffu, set);
+        if (lane < 2) {
+          const int b0 = (xk - x0) / 8;  // bit 0: macro cell 128 xs - 1
+          const uint32_t word = lane == 0 ? m18 << (b0 & 31) : (b0 & 31) ? m18 >> (32 - (b0 & 31)) : 0u;
+          if (word)
+            for (int dz = rz < 2 ? 0 : 1; dz <= (rz == 7 ? 2 : 1); ++dz)
+              for (int dy = ry < 2 ? 0 : 1; dy <= (ry == 7 ? 2 : 1); ++dy)
+                if (word & ~bits[dz][dy][(b0 >> 5) + lane]) atomicOr(&bits[dz][dy][(b0 >> 5) + lane], word);
         }
       }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if (lane == 0) {
-    if (mx) atomicMax(&stats->max_bits, mx);
+  for (int o = 16; o > 0; o >>= 1) {
+    lo[0] = min(lo[0], __shfl_xor_sync(0xffffffffu, lo[0], o));
+    hi[0] = max(hi[0], __shfl_xor_sync(0xffffffffu, hi[0], o));
+  }
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) {  // one atomic per block and value: they all meet in one L2 sector
+    atomicMax(&found[0], __float_as_uint(mx));
     if (hi[0] >= 0)
       for (int k = 0; k < 3; ++k) {
-        atomicMax(&stats->lo[k], 0x7fffffffu - (unsigned int)lo[k]);
-        atomicMax(&stats->hi[k], (unsigned int)hi[k] + 1u);
+        atomicMax(&found[1 + k], 0x7fffffffu - (unsigned int)lo[k]);
+        atomicMax(&found[4 + k], (unsigned int)hi[k] + 1u);
       }
   }
   __syncthreads();
+  if (threadIdx.x < 7 && found[threadIdx.x]) {
+    unsigned int* g = threadIdx.x == 0 ? &stats->max_bits : threadIdx.x < 4 ? &stats->lo[threadIdx.x - 1] : &stats->hi[threadIdx.x - 4];
+    atomicMax(g, found[threadIdx.x]);
+  }
   for (int i = threadIdx.x; i < 9 * kSegBits; i += kThreads) {
     const int d = i / kSegBits, b = i - d * kSegBits;
     if (!((bits[d / 3][d % 3][b >> 5] >> (b & 31)) & 1u)) continue;
@@ -262,8 +298,10 @@ cudaError_t launch_volume_stats(const float* vox, int nx, int ny, int nz, uint32
   if (e == cudaSuccess) e = cudaMemsetAsync(d_stats, 0, sizeof(VolStats), s);
   if (e != cudaSuccess) return e;
   const int64_t nxs = ((int64_t)nx + kSegX - 1) / kSegX, nyb = ((int64_t)ny + 7) / 8, nzb = ((int64_t)nz + 7) / 8;
-  volume_stats_kernel<<<(unsigned)(nxs * nyb * nzb), kThreads, 0, s>>>(vox, nx, ny, nz, (int)nxs, (int)nyb, d_occ, nmx,
-                                                                       nmy, nmz, d_stats);
+  const bool vec = nx % 4 == 0 && reinterpret_cast<uintptr_t>(vox) % 16 == 0;
+  const auto kernel = vec ? volume_stats_kernel<true> : volume_stats_kernel<false>;
+  kernel<<<(unsigned)(nxs * nyb * nzb), kThreads, 0, s>>>(vox, nx, ny, nz, (int)nxs, (int)nyb, d_occ, nmx, nmy, nmz,
+                                                          d_stats);
   return cudaGetLastError();
 }
 
