@@ -1,4 +1,4 @@
-"""Patch metrics at the edges of their tiles (32 columns by 8, 32 or 64 rows of patches,
+"""Patch metrics at the edges of their tiles (32 columns by 8 or 32 rows of patches,
 images in pairs), masked and not, every stride, against the oracle; the same bounds
 as the other metric tests (1e-5)."""
 import numpy as np
@@ -73,7 +73,7 @@ def test_masked_out_pixel_that_is_not_finite(xr, grad, radius, stride, bad):
                                                               ((97, 140), 3, 1, False, 41), ((253, 210), 5, 2, True, 41),
                                                               ((253, 210), 5, 2, False, 41)])
 def test_an_image_alone_or_among_many(xr, grad, shape, radius, stride, masked, nimgs):
-    """Few patches are scored one a thread, many four or eight: the same bits."""
+    """Few patches are scored one a thread, many four: the same bits."""
     import torch
     rng = np.random.default_rng(shape[0])
     fixed = rng.random(shape).astype(np.float32)

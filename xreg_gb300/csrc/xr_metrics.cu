@@ -703,10 +703,11 @@ __global__ void __launch_bounds__(kThreads) patch_ncc_kernel(const float* __rest
 // instruction for two, each lane rounded as the scalar one): the two gradients of an
 // image, or two images of the plain patch metric.  Per patch two passes as in
 // patch_score: the mean, then the deviations.  Bound by the FP32 pipe (4 operations a
-// pixel, patch and channel) and by 16 warps an SM, which the registers allow.  20
-// images of 768^2, 11 x 11, both gradients: 1175 us one channel at a time, now 667; 24
-// plain images of 384^2: 180 us, now 102; 8 images of 187 x 118 at stride 3, a whole
-// call: 55 us, now 48.
+// pixel, patch and channel) at 24 warps an SM, for which the columns of a row are taken
+// in two parts and a mask is kept in bytes (at 16 warps eight patches a thread were
+// needed: masked calls and strides of 2 were 5 to 12 % slower).  20 images of 768^2, 11
+// x 11, both gradients: 1175 us one channel at a time, now 669; 24 plain images of 384^2:
+// 180 us, now 99; 8 images of 187 x 118 at stride 3, a whole call: 55 us, now 47.
 // Every RB takes the same operations in the same order, patch by patch and up to the
 // partial sums (one for 16 rows of patches), so an image's value does not depend on
 // how many others share the launch.
@@ -726,7 +727,7 @@ struct PatchRows {
     L.P = stride * L.Wp;
     L.edge = (2 * radius + 4) & ~3;
     const int words = grad ? 4 : (rb > 1 ? 3 : 2);  // the moving side, in pairs but for rb 1, and the fixed one
-    L.bytes = (size_t)L.edge * 4 + (size_t)L.Wr * L.P * 4 * (words + (mask ? 1 : 0));
+    L.bytes = (size_t)L.edge * 4 + (size_t)L.Wr * L.P * (4 * words + (mask ? 1 : 0));
     return L;
   }
 };
@@ -763,14 +764,23 @@ __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
 }
 
 // body(std::integral_constant<int, N>, offsets) for the columns of a patch row, in
-// order, N at a time: all at once where edge and stride (1 or 2) are known, else in fours
-template <int DC, int SC, typename Body>
+// order, N at a time: all at once (HALVES: in two parts) where edge and stride (1 or 2)
+// are known, else in fours
+template <int DC, int SC, bool HALVES, typename Body>
 __device__ __forceinline__ void patch_columns(int d, int Wp, const int4* __restrict__ offs, Body body) {
   if constexpr (DC > 0) {
     int o[DC];
 #pragma unroll
     for (int c = 0; c < DC; ++c) o[c] = (c % SC) * Wp + c / SC;
-    body(std::integral_constant<int, DC>(), o);
+    if constexpr (HALVES) {
+      body(std::integral_constant<int, DC - DC / 2>(), o);
+      int o2[DC / 2];
+#pragma unroll
+      for (int c = 0; c < DC / 2; ++c) o2[c] = o[DC - DC / 2 + c];
+      body(std::integral_constant<int, DC / 2>(), o2);
+    } else {
+      body(std::integral_constant<int, DC>(), o);
+    }
   } else {
     int c = 0;
 #pragma unroll 1
@@ -790,13 +800,20 @@ __device__ __forceinline__ void patch_columns(int d, int Wp, const int4* __restr
   }
 }
 
+// a mask byte (-1 or 0) as 1 or 0 in every channel
+template <typename V>
+__device__ __forceinline__ V patch_mask(int m) {
+  const float k = __uint_as_float((unsigned int)m & 0x3f800000u);
+  return pack2<V>(k, k);
+}
+
 // Scores of RB stacked patches in both channels; their first window starts at m[0]
-// (V: a pair of channels, or one), f[0] (as m, or FS: one value for both), mk[0] (MASK: 1 or 0 per
+// (V: a pair of channels, or one), f[0] (as m, or FS: one value for both), mk[0] (MASK: -1 or 0 per
 // pixel, f zero where it is 0), row pitch P.  DC and SC: the patch edge and stride when
 // known.  scale(j): the patch's 1 / sd of the fixed side, per channel.
 template <typename V, int RB, int DC, int SC, bool MASK, bool FS, typename Scale>
 __device__ __forceinline__ void patch_column_scores(const V* __restrict__ m, const void* __restrict__ f,
-                                                    const float* __restrict__ mk, int P, int Wp, const int4* __restrict__ offs,
+                                                    const int8_t* __restrict__ mk, int P, int Wp, const int4* __restrict__ offs,
                                                     int d_rt, int stride_rt, const V (&fmean)[RB], Scale scale,
                                                     float2 (&score)[RB]) {
   const int d = DC > 0 ? DC : d_rt, stride = DC > 0 ? SC : stride_rt;
@@ -816,7 +833,7 @@ __device__ __forceinline__ void patch_column_scores(const V* __restrict__ m, con
   for (int r = 0; r < span; ++r) {
     const V* row = m + r * P;
     V h = V(0);
-    patch_columns<DC, SC>(d, Wp, offs, [&](auto count, auto& o) {
+    patch_columns<DC, SC, RB == 4>(d, Wp, offs, [&](auto count, auto& o) {
       V x[count.value];
 #pragma unroll
       for (int c = 0; c < count.value; ++c) x[c] = row[o[c]];
@@ -836,14 +853,14 @@ __device__ __forceinline__ void patch_column_scores(const V* __restrict__ m, con
 #pragma unroll 1
   for (int r = 0; r < span; ++r) {
     const int row = r * P;
-    patch_columns<DC, SC>(d, Wp, offs, [&](auto count, auto& o) {
+    patch_columns<DC, SC, RB == 4>(d, Wp, offs, [&](auto count, auto& o) {
       constexpr int N = count.value;
       V x[N], y[N], k[N];  // k: the mask twice
 #pragma unroll
       for (int c = 0; c < N; ++c) {
         x[c] = m[row + o[c]];
         y[c] = fixed(row + o[c]);
-        k[c] = MASK ? pack2<V>(mk[row + o[c]], mk[row + o[c]]) : V(0);
+        k[c] = MASK ? patch_mask<V>(mk[row + o[c]]) : V(0);
       }
 #pragma unroll
       for (int j = 0; j < RB; ++j)
@@ -869,7 +886,7 @@ __device__ __forceinline__ void patch_column_scores(const V* __restrict__ m, con
 #pragma unroll 1
         for (int c = 0; c < d; ++c) {
           const int i = r * P + reinterpret_cast<const int*>(offs)[c];
-          if (mk[i] == 0.0f) continue;
+          if (mk[i] == 0) continue;
           const float2 x = unpack2(m[i]), y = unpack2(fixed(i));
           c2.x = fmaf(x.x + mj.x, y.x + fm.x, c2.x);
           c2.y = fmaf(x.y + mj.y, y.y + fm.y, c2.y);
@@ -947,7 +964,7 @@ __device__ __forceinline__ void patch_tile_gradients(const float* __restrict__ s
 // Grid: tiles, then images (GRAD, RB 1) or pairs of images; kr: the blur's radius (GRAD).
 // Partials: per image, sums over kPartRows rows by 32 columns of patches, nblk of them.
 template <int GRAD, int RB, int DC, int SC, bool MASK>
-__global__ void __launch_bounds__(kThreads, RB == 1 ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, 3)
 patch_rows_kernel(const float* __restrict__ imgs, int rows, int cols, int64_t nimgs, int kr, int radius, int stride_rt,
                   int ncr, int ncc, PatchFixed px, PatchFixed py, PatchRun run,
                   double* __restrict__ partials, int nblk) {
@@ -963,7 +980,7 @@ patch_rows_kernel(const float* __restrict__ imgs, int rows, int cols, int64_t ni
   V* s_m = reinterpret_cast<V*>(s_off + L.edge);
   float2* s_f = reinterpret_cast<float2*>(s_m + size);   // GRAD
   float* s_f1 = reinterpret_cast<float*>(s_f);           // plain
-  float* s_mk = GRAD ? reinterpret_cast<float*>(s_f + size) : s_f1 + size;
+  int8_t* s_mk = reinterpret_cast<int8_t*>(GRAD ? reinterpret_cast<float*>(s_f + size) : s_f1 + size);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tiles_x = (ncc + 31) / 32;
   const int tpr = blockIdx.x / tiles_x, tpc = blockIdx.x - tpr * tiles_x;
@@ -1005,7 +1022,7 @@ patch_rows_kernel(const float* __restrict__ imgs, int rows, int cols, int64_t ni
       if (at_i[k] < 0) continue;
       if constexpr (GRAD != 0) s_f[at_i[k]] = in[k] ? make_float2(a[k], b[k]) : make_float2(0.0f, 0.0f);
       else s_f1[at_i[k]] = in[k] ? a[k] : 0.0f;
-      if constexpr (MASK) s_mk[at_i[k]] = in[k] ? 1.0f : 0.0f;
+      if constexpr (MASK) s_mk[at_i[k]] = in[k] ? -1 : 0;
     }
   }
   if constexpr (GRAD != 0) {
@@ -1288,12 +1305,10 @@ cudaError_t launch_patch_fixed_stats(const float* img, int rows, int cols, int r
 }
 
 // Patches a thread scores in a column (patch_rows_kernel).  One while a patch a thread
-// does not fill the GPU (1024 threads an SM): more would leave SMs idle (6 images of
+// does not fill the GPU (1024 threads an SM): four would leave SMs idle (6 images of
 // 311 x 476, 15 x 15 at stride 3, a whole call: 56 us against 81 with four; 16 of 215 x
-// 493, 11 x 11 at stride 2, above the line: 79 against 70).  Eight from two waves of blocks on
-// where the tile fits shared memory twice and no mask takes registers (20 images of
-// 768^2, both gradients: 667 us against 742); else four.  The general kernel with masked
-// statistics, moving-variance weights or tiles too large.
+// 493, 11 x 11 at stride 2, above the line: 79 against 60).  The general kernel with
+// masked statistics, moving-variance weights or tiles too large.
 constexpr size_t kPatchSmem = 200 * 1024;
 
 static size_t patch_rows_bytes(int radius, int stride, int grad, const PatchRun& run, int rb) {
@@ -1316,13 +1331,8 @@ static cudaError_t patch_rb(int radius, int stride, int grad, const PatchRun& ru
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  const int64_t pairs = grad ? nimgs : (nimgs + 1) / 2;
-  *rb = 1;
-  if ((int64_t)ncr * ncc * nimgs <= (int64_t)sms * 1024) return e;
-  if (patch_rows_bytes(radius, stride, grad, run, 4) <= kPatchSmem) *rb = 4;
-  if (!run.mask && patch_rows_bytes(radius, stride, grad, run, 8) <= kPatchSmem / 2 &&
-      patch_tiles(ncr, ncc, 64) * pairs >= 4 * sms)
-    *rb = 8;
+  const bool many = (int64_t)ncr * ncc * nimgs > (int64_t)sms * 1024;
+  *rb = many && patch_rows_bytes(radius, stride, grad, run, 4) <= kPatchSmem ? 4 : 1;
   return e;
 }
 
@@ -1358,7 +1368,7 @@ cudaError_t launch_patch_ncc(const float* mov, int rows, int cols, int64_t nimgs
     const cudaError_t e = patch_rb(radius, stride, grad, run, ncr, ncc, nimgs, &rb);
     if (e != cudaSuccess) return e;
     // the columns of xReg's default patches (11 x 11) unroll at strides 1 and 2 (24 masked
-    // images of 384^2 at stride 2, a whole call: 66 us against 95 by fours)
+    // images of 384^2 at stride 2, a whole call: 63 us against 95 by fours)
 #define XR_ROWS(G, R, D, S, M) \
   return launch_rows<G, R, D, S, M>(mov, rows, cols, kr, radius, stride, ncr, ncc, nimgs, px, py, run, partials, nblk, s)
 #define XR_ROWS_R(G, R, M)                                 \
@@ -1369,8 +1379,7 @@ cudaError_t launch_patch_ncc(const float* mov, int rows, int cols, int64_t nimgs
   if (run.mask && rb == 1) { XR_ROWS_R(G, 1, true); } \
   if (run.mask) { XR_ROWS_R(G, 4, true); }            \
   if (rb == 1) { XR_ROWS_R(G, 1, false); }            \
-  if (rb == 4) { XR_ROWS_R(G, 4, false); }            \
-  XR_ROWS_R(G, 8, false)
+  XR_ROWS_R(G, 4, false)
     if (grad) { XR_ROWS_G(1); }
     XR_ROWS_G(0);
 #undef XR_ROWS_G
