@@ -706,8 +706,8 @@ __global__ void __launch_bounds__(kThreads) patch_ncc_kernel(const float* __rest
 // pixel, patch and channel) at 24 warps an SM, for which the columns of a row are taken
 // in two parts and a mask is kept in bytes (at 16 warps eight patches a thread were
 // needed: masked calls and strides of 2 were 5 to 12 % slower).  20 images of 768^2, 11
-// x 11, both gradients: 1175 us one channel at a time, now 669; 24 plain images of 384^2:
-// 180 us, now 99; 8 images of 187 x 118 at stride 3, a whole call: 55 us, now 47.
+// x 11, both gradients: 1175 us one channel at a time, now 632; 24 plain images of 384^2:
+// 180 us, now 98; 8 images of 187 x 118 at stride 3, a whole call: 55 us, now 47.
 // Every RB takes the same operations in the same order, patch by patch and up to the
 // partial sums (one for 16 rows of patches), so an image's value does not depend on
 // how many others share the launch.
@@ -926,13 +926,20 @@ __device__ __forceinline__ void patch_tile_gradients(const float* __restrict__ s
     for (int i = 0; i < kWin; ++i) hb[i] = 0.0f;
 #pragma unroll
     for (int i = 0; i < 3; ++i) bl[i] = lf[i] = rt[i] = 0.0f;
-    for (int rb = r0 - 2 * H; rb < r1; rb += 8) {  // output rows rb .., from input rows rb + H ..
-      float p[8];
+    constexpr int kGroup = 6;  // rows in flight; 11 or 17 rows a warp at the default radius (8: 645 us for 632)
+    for (int rb = r0 - 2 * H; rb < r1; rb += kGroup) {  // output rows rb .., from input rows rb + H ..
+      float p[kGroup];
+      if (y0 + rb + H >= 0 && y0 + rb + H + kGroup <= rows) {  // no row to reflect
+        const float* q = pc + (int64_t)(y0 + rb + H) * cols;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        p[i] = __ldg(pc + (int64_t)reflect101(min(y0 + rb + i + H, rows - 1 + H), rows) * cols);
+        for (int i = 0; i < kGroup; ++i) p[i] = __ldg(q + (int64_t)i * cols);
+      } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < kGroup; ++i)
+          p[i] = __ldg(pc + (int64_t)reflect101(min(y0 + rb + i + H, rows - 1 + H), rows) * cols);
+      }
+#pragma unroll
+      for (int i = 0; i < kGroup; ++i) {
         float h = p[i];
         if constexpr (KR == 2)
           h = gt::blur5(__shfl_up_sync(0xffffffffu, p[i], 2), __shfl_up_sync(0xffffffffu, p[i], 1), p[i],
@@ -996,33 +1003,35 @@ patch_rows_kernel(const float* __restrict__ imgs, int rows, int cols, int64_t ni
   };
   if (threadIdx.x < L.edge) s_off[threadIdx.x] = at(threadIdx.x);
 
-  // the fixed side, the mask and (plain patches) the images, 32 pixels of a row per
-  // warp and four such pieces in flight; past the image the last pixel, which only
-  // patches outside the grid read
-  const int pieces = (L.Wc + 31) / 32, units = L.Wr * pieces;
-  for (int u0 = warp; u0 < units; u0 += 4 * kWarps) {
-    float a[4], b[4];
-    bool in[4];
-    int at_i[4];
+  // the fixed side, the mask and (plain patches) the images: a lane goes down a column,
+  // four of its rows in flight; past the image the last pixel, which only patches outside
+  // the grid read
+  for (int c = lane; c < L.Wc; c += 32) {
+    const int to = at(c);
+    const int64_t gc = min(x0 + c, cols - 1);
+    for (int r0 = warp; r0 < L.Wr; r0 += 4 * kWarps) {
+      float a[4], b[4], b1[4];
+      bool in[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int u = u0 + k * kWarps, r = u / pieces, c = (u - r * pieces) * 32 + lane;
-      const int64_t g = (int64_t)min(y0 + r, rows - 1) * cols + min(x0 + c, cols - 1);
-      at_i[k] = (u < units && c < L.Wc) ? r * L.P + at(c) : -1;
-      in[k] = !MASK || run.mask[g];
-      a[k] = __ldg(px.img + g);
-      b[k] = GRAD ? __ldg(py.img + g) : __ldg(src + g);
-      if constexpr (GRAD == 0) {
-        const float b1 = pair ? __ldg(src + npix + g) : b[k];
-        if (at_i[k] >= 0) s_m[at_i[k]] = pack2<V>(b[k], b1);
+      for (int k = 0; k < 4; ++k) {
+        const int64_t g = (int64_t)min(y0 + r0 + k * kWarps, rows - 1) * cols + gc;
+        in[k] = !MASK || run.mask[g];
+        a[k] = __ldg(px.img + g);
+        b[k] = GRAD ? __ldg(py.img + g) : __ldg(src + g);
+        b1[k] = pair ? __ldg(src + npix + g) : b[k];
       }
-    }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (at_i[k] < 0) continue;
-      if constexpr (GRAD != 0) s_f[at_i[k]] = in[k] ? make_float2(a[k], b[k]) : make_float2(0.0f, 0.0f);
-      else s_f1[at_i[k]] = in[k] ? a[k] : 0.0f;
-      if constexpr (MASK) s_mk[at_i[k]] = in[k] ? -1 : 0;
+      for (int k = 0; k < 4; ++k) {
+        const int r = r0 + k * kWarps, i = r * L.P + to;
+        if (r >= L.Wr) break;
+        if constexpr (GRAD != 0) {
+          s_f[i] = in[k] ? make_float2(a[k], b[k]) : make_float2(0.0f, 0.0f);
+        } else {
+          s_m[i] = pack2<V>(b[k], b1[k]);
+          s_f1[i] = in[k] ? a[k] : 0.0f;
+        }
+        if constexpr (MASK) s_mk[i] = in[k] ? -1 : 0;
+      }
     }
   }
   if constexpr (GRAD != 0) {
