@@ -59,6 +59,20 @@ def test_values_up_to_the_faces(xr, oracle, size, vt):
     assert zero == 0.0 and rel <= TOL[vt], rel
 
 
+def test_subnormal_bf16_voxels(xr):
+    """Rays that meet only voxels below 2^-126: every layout gives the same bits."""
+    rng = np.random.default_rng(11)
+    v = np.zeros((40, 36, 33), np.float32)
+    v[6:34, 6:30, 6:15] = rng.uniform(0.5, 1.0, (28, 24, 9))
+    v[6:34, 6:30, 15:27] = rng.uniform(0.0, 1.0, (28, 24, 12)) * 1e-38
+    vol = api.Volume(v, spacing=(1.5, 1.5, 1.5))
+    cam, poses = small_camera((45, 37), 4.0), _poses(vol, 5)
+    imgs = _images(xr, vol, cam, poses, 2)
+    assert np.any((imgs[0] > 0) & (imgs[0] < 1e-30))
+    for img in imgs[1:]:
+        np.testing.assert_array_equal(img, imgs[0])
+
+
 @pytest.mark.parametrize("vt", [0, 2])
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 1e38])
 def test_values_without_finite_differences(xr, oracle, value, vt):
