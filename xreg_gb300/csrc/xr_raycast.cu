@@ -952,7 +952,7 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
       if (use) {
         const int total = W * H * Dz;
         for (int i = tid; i < total; i += kThreads) {
-          const int x = lo[0] + i % W, y = lo[1] + (i / W) % H, zz = lo[2] + i / (W * H);
+          const int zz = lo[2] + i % Dz, x = lo[0] + (i / Dz) % W, y = lo[1] + i / (Dz * W);  // as cells lie
           const int64_t c = (int64_t)x * vol.cs[0] + (int64_t)y * vol.cs[1] + zz;
           s_cells[2 * i] = __ldg(cells + 2 * c);
           s_cells[2 * i + 1] = __ldg(cells + 2 * c + 1);
@@ -969,7 +969,7 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
           const bool in = use && c[0] >= lo[0] && c[0] <= hi[0] && c[1] >= lo[1] && c[1] <= hi[1] && c[2] >= lo[2] &&
                           c[2] <= hi[2];
           if (in) {
-            const int i = (c[0] - lo[0]) + W * ((c[1] - lo[1]) + H * (c[2] - lo[2]));
+            const int i = (c[2] - lo[2]) + Dz * ((c[0] - lo[0]) + W * (c[1] - lo[1]));
             const float4 q0 = s_cells[2 * i], q1 = s_cells[2 * i + 1];
             v[0] = q0.x; v[1] = q0.y; v[2] = q0.z; v[3] = q0.w;
             v[4] = q1.x; v[5] = q1.y; v[6] = q1.z; v[7] = q1.w;
