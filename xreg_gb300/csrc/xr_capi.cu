@@ -1,6 +1,7 @@
 // xr_capi.cu -- the extern "C" boundary: handles, validation, device buffers,
 // stream ordering and CUDA-graph capture of the population objective.
 // Nothing here throws across the ABI; every entry point returns an xr_status.
+#include "xr_cells.h"
 #include "xr_internal.h"
 #include "xr_posespread.h"
 #include "xreg_gb300_regi.h"

@@ -109,12 +109,6 @@ struct MultiJobDrr {
 // grouped: every job's pose_group is 4 (otherwise every job's is 0).
 cudaError_t launch_drr_jobs(const MultiJobDrr* d_jobs, int njobs, long long total_items, int32_t voxel_type,
                             int32_t layout, bool grouped, cudaStream_t s);
-// Bytes of the CELL8 copy of a volume (cells numbered z fastest, then x, then y: VolView::cs).
-size_t cell_layout_bytes(int64_t nx, int64_t ny, int64_t nz, int32_t voxel_type);
-// The x and y cell strides of that order (VolView::cs).
-void cell_strides(int64_t nx, int64_t ny, int64_t nz, int32_t cs[2]);
-// VolView::kfl and cell_bytes of a volume; zeros in kfl where there are none.
-void cell_floor_constants(int64_t nx, int64_t ny, int64_t nz, int32_t voxel_type, float kfl[3], int32_t* bytes);
 
 // ---- launchers (xr_volume.cu) ----
 // HUToLinAtt of n values.

@@ -34,8 +34,9 @@
 //           border cells (index -1 and n-1) are constant along their axis: a
 //           position that rounding carries past a face of the volume reads the
 //           face's values with no clamp in the sample loop.
-#include "xr_internal.h"
+#include "xr_cells.h"
 #include "xr_gradtile.cuh"
+#include "xr_internal.h"
 
 #include <algorithm>
 #include <atomic>
@@ -236,7 +237,6 @@ __device__ __forceinline__ unsigned int h2_pack(float g, float f) {
   asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(f), "f"(g));
   return d;
 }
-constexpr float kH16 = 32768.0f;  // scale of the x and y weights
 // w: (v000, v001) (v100, v101) (v010, v011) (v110, v111), low half z = 0; fx, fy:
 // the fractions times kH16 (the cell walk's positions carry that scale, so the
 // four weights take two subtractions and two conversions; with the x weights
@@ -667,19 +667,15 @@ __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, co
           }
         }
       }
-      // The exact ray lies in [0, n-1], so positions without drift beyond an eighth
-      // of a voxel stay in [-1, n): march_cells.  On the LINEAR layout rays whose
-      // first and last loaded samples lie a quarter voxel inside (the segment is
-      // straight) run the sampler without clamps.
+      // With both ends within three quarters of a voxel of [0, n-1] (the segment is
+      // straight) and a drift below an eighth, every position stays in [-1, n):
+      // march_cells, whose loads no clamp bounds.  Rays of ordinary frames all lie
+      // there; a NaN or infinite start or step does not, nor one that a focal point
+      // millions of voxels away rounds off the volume: those take the clamped
+      // sampler.  On the LINEAR layout rays a quarter voxel inside run without clamps.
       bool unclamped = drift_ok && (LAYOUT == XR_LAYOUT_LINEAR || p.vol.kfl[0] > 0.0f);
-      if (LAYOUT == XR_LAYOUT_LINEAR && unclamped) {
-        const float p0[3] = {px, py, pz}, st[3] = {sx, sy, sz};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const float a = p0[k] + (float)first * st[k], b = p0[k] + (float)last * st[k];
-          unclamped = unclamped && fminf(a, b) >= 0.25f && fmaxf(a, b) <= maxb[k] - 0.25f;
-        }
-      }
+      if (unclamped)
+        unclamped = xf::samples_within(st0, stv, first, last, maxb, LAYOUT == XR_LAYOUT_LINEAR ? -0.25f : 0.75f);
       if (hit) {
         // advance to sample `first` (four additions per trip: the skipped samples
         // are a large part of a trimmed ray); x and y as one packed pair, whose
@@ -1452,49 +1448,6 @@ cudaError_t launch_drr_jobs(const MultiJobDrr* d_jobs, int njobs, long long tota
     default: return cudaErrorInvalidValue;
   }
 #undef XR_JOBS
-}
-
-size_t cell_layout_bytes(int64_t nx, int64_t ny, int64_t nz, int32_t voxel_type) {
-  int32_t cs[2];
-  cell_strides(nx, ny, nz, cs);
-  const size_t ncell = (size_t)cs[1] * (size_t)(ny + 1);
-  return ncell * (voxel_type == XR_VOXEL_F32 ? 32 : 16);
-}
-
-// Strides of 2 modulo 8.  The L1 serves a cell load in passes of 4 lanes
-// (32-byte cells) or 8 lanes (16-byte cells), one wavefront per pass unless two of
-// its cells share a bank group, i.e. a cell number modulo 4 or 8; with these
-// strides the cells of a pass's 2 x 2 or 4 x 2 pixel block (lane_pixel) mostly
-// differ there.  Measured against unpadded strides, and 4 x 1 and 4 x 2 blocks, on
-// the launches of march_cells: float32 5409 -> 5130 us (9.8 -> 8.9 wavefronts per
-// load, 8 is the least), FP16 2994 -> 2871 (12.4 -> 11.5), BF16 unchanged.
-void cell_strides(int64_t nx, int64_t ny, int64_t nz, int32_t cs[2]) {
-  (void)ny;
-  auto pad = [](int64_t n) { return (int32_t)(n + ((2 - n) & 7)); };  // the next number that is 2 modulo 8
-  cs[0] = pad(nz + 1);
-  cs[1] = pad((int64_t)cs[0] * (nx + 1));
-}
-
-// Whole numbers 1 <= m <= 2^22 that turn bias + m + floor(p) per axis into the
-// cell (floor(p) + 1 per axis, in strides of cs[0] u, cs[1] u and u bytes or, with
-// u 1, cells) modulo 2^32: the sum of the biases, negated, in the mixed base of the
-// strides, plus one each.  m_y <= 2^32 / (cs[1] u), m_x and m_z stay within a slab's
-// cells; a slab below 2^10 (bytes or cells) would need a larger m_y: none then.
-void cell_floor_constants(int64_t nx, int64_t ny, int64_t nz, int32_t voxel_type, float kfl[3], int32_t* bytes) {
-  int32_t cs[2];
-  cell_strides(nx, ny, nz, cs);
-  *bytes = cell_layout_bytes(nx, ny, nz, voxel_type) < (size_t(1) << 32) ? 1 : 0;
-  const uint32_t u = !*bytes ? 1u : (voxel_type == XR_VOXEL_F32 ? 32u : 16u);
-  const uint32_t sx = (uint32_t)cs[0] * u, sy = (uint32_t)cs[1] * u;
-  for (int k = 0; k < 3; ++k) kfl[k] = 0.0f;
-  if (sy <= 1024) return;
-  const float scale = voxel_type == XR_VOXEL_F16 ? kH16 : 1.0f;  // of the x and y positions
-  const uint32_t bias_xy = voxel_type == XR_VOXEL_F16 ? 0x52800000u : 0x4B000000u;  // bits of 2^23 scale
-  const uint32_t t = 0u - bias_xy * (sx + sy) - 0x4B000000u * u;
-  const uint32_t my = t / sy, mx = (t % sy) / sx, mz = (t % sy) % sx / u;
-  kfl[0] = (8388609.0f + (float)mx) * scale;
-  kfl[1] = (8388609.0f + (float)my) * scale;
-  kfl[2] = 8388609.0f + (float)mz;
 }
 
 }  // namespace xr

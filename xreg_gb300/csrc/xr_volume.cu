@@ -1,6 +1,7 @@
 // xr_volume.cu -- volume set-up: HU to attenuation, the statistics of a volume
 // (largest magnitude, support box, macro-cell occupancy) in one pass, and its
 // cell copy and 16-bit voxels in another.  All bound by HBM.
+#include "xr_cells.h"
 #include "xr_internal.h"
 
 #include <algorithm>
