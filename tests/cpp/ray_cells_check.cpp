@@ -8,6 +8,7 @@
 #include <cfenv>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -89,6 +90,17 @@ Counts run(const int32_t n[3], int vt, float step, int rows, int cols, const xr:
 }  // namespace
 
 int main(int argc, char** argv) {
+  if (argc == 6) {  // nx ny nz voxel type, "numbering": strides, bytes, constants
+    const int64_t n[3] = {std::atoll(argv[1]), std::atoll(argv[2]), std::atoll(argv[3])};
+    const int vt = std::atoi(argv[4]);
+    int32_t cs[2], bytes;
+    float kfl[3];
+    xr::cell_strides(n[0], n[1], n[2], cs);
+    xr::cell_floor_constants(n[0], n[1], n[2], vt, kfl, &bytes);
+    std::printf("%d %d %d %llu %d %.1f %.1f %.1f\n", xr::cells_numbered(n[0], n[1], n[2]) ? 1 : 0, cs[0], cs[1],
+                (unsigned long long)xr::cell_layout_bytes(n[0], n[1], n[2], vt), bytes, kfl[0], kfl[1], kfl[2]);
+    return 0;
+  }
   if (argc != 3) return 2;
   std::FILE* f = std::fopen(argv[1], "rb");
   std::FILE* o = std::fopen(argv[2], "wb");

@@ -113,3 +113,36 @@ def test_focal_points_far_away(exe, tmp_path, vt):
         if far <= 1e6:
             assert np.all(c["guarded"] == 0)
     assert seen > 0
+
+
+def _numbering(exe, n, vt):
+    out = subprocess.run([str(exe), *map(str, n), str(vt), "numbering"], check=True, capture_output=True, text=True).stdout.split()
+    return bool(int(out[0])), (int(out[1]), int(out[2])), int(out[3]), int(out[4]), tuple(map(float, out[5:]))
+
+
+# full volumes, stacks of few slices on each axis, axes as long as 2^31 voxels allow
+@pytest.mark.parametrize("n", [(256, 256, 256), (512, 512, 300), (1290, 1290, 1290), (512, 512, 4), (4, 512, 512), (512, 4, 512),
+                               (2, 2, 2), (55, 9, 55), (56, 9, 54), (20000, 20000, 4), (32768, 32767, 2), (2, 32768, 32767),
+                               (4194303, 2, 2), (2, 4194303, 2), (2, 2, 4194303), (440000000, 2, 2), (2, 440000000, 2),
+                               (2, 2, 440000000), (536870911, 2, 2), (2, 536870911, 2), (2, 2, 536870911), (4194303, 255, 2)])
+@pytest.mark.parametrize("vt", [F32, F16, BF16])
+def test_cell_numbers_fit_their_32_bits(exe, n, vt):
+    numbered, (sx, sy), nbytes, in_bytes, kfl = _numbering(exe, n, vt)
+    cell = 32 if vt == F32 else 16
+    least = (n[0] + 1) * (n[1] + 1) * (n[2] + 1)
+    if not numbered:
+        assert least >= 2 ** 32 and (sx, sy, nbytes) == (0, 0, 0) and kfl == (0.0, 0.0, 0.0)
+        return
+    assert sx >= n[2] + 1 and sy >= sx * (n[0] + 1) and nbytes == sy * (n[1] + 1) * cell < 2 ** 32 * cell
+    assert nbytes <= 1.27 * least * cell  # an eighth on either stride
+    assert in_bytes == (nbytes < 2 ** 32)
+    if kfl != (0.0, 0.0, 0.0):
+        unit, s = (cell if in_bytes else 1), (32768.0 if vt == F16 else 1.0)
+        for k in range(3):
+            one = s if k < 2 else 1.0
+            m = kfl[k] / one - 2.0 ** 23
+            assert m == int(m) and 1 <= m and m + n[k] < 2 ** 23  # 2^23 + m + floor(p) stays below 2^24
+        b = [0x52800000 if vt == F16 else 0x4B000000] * 2 + [0x4B000000]
+        at = [b[k] + int(kfl[k] / (s if k < 2 else 1.0) - 2.0 ** 23) for k in range(3)]  # of position 0: cell 1
+        got = (at[1] * sy * unit + at[0] * sx * unit + at[2] * unit) % 2 ** 32
+        assert got == (sy + sx + 1) * unit % 2 ** 32
