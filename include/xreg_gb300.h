@@ -223,8 +223,8 @@ XR_API xr_status xr_rc_set_count_samples(xr_raycaster rc, int32_t enable);
  * the autotuner time the block shapes on the first compute of each shape (volume
  * size, voxel type, detector, projection count) and cache the fastest for the
  * process; the cell copy, one load per sample, and loop 4 are always its choice.
- * A volume that holds an infinity or a value above 2^126 is read in the LINEAR
- * layout whatever is asked for.  No xReg counterpart (xReg's OpenCL caster has a fixed NDRange). */
+ * A volume with more than 2^32 cells (about 2^31 voxels, two very short axes) is
+ * read in the LINEAR layout whatever is asked for.  No xReg counterpart (xReg's OpenCL caster has a fixed NDRange). */
 XR_API xr_status xr_rc_set_launch_config(xr_raycaster rc, int32_t layout, int32_t block_warps_x, int32_t unroll);
 /* The configuration the last compute used. */
 XR_API xr_status xr_rc_get_launch_config(xr_raycaster rc, int32_t* layout, int32_t* block_warps_x, int32_t* unroll);

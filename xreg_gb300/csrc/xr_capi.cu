@@ -498,11 +498,11 @@ static xr_status rc_set_volumes_impl(xr_raycaster rc, int32_t n, const xr_volume
       v->inv_scale = 1.0f / sc;
     }
     // Differences of corners must be finite for the blends of float32 and BF16
-    // volumes; a volume where they might not be is read as it lies (VolView::weighted).
+    // volumes; a volume where they might not be takes the weighted ones (VolView::weighted).
     v->weighted = vt != XR_VOXEL_F16 && !(mx * sc <= 0x1p126f);
     vol_support(*v, st);
     v->linear_only = rc->build_cells && !cells_numbered(d.n[0], d.n[1], d.n[2]);
-    const bool cells = rc->build_cells && !v->weighted && !v->linear_only;
+    const bool cells = rc->build_cells && !v->linear_only;
     const size_t cell_bytes = cells ? cell_layout_bytes(d.n[0], d.n[1], d.n[2], vt) : 0;
     // One volume in place of one of the same or a larger size: its buffers are
     // written over (allocating and freeing them took 1.4 ms of the 5.1 ms of
@@ -533,7 +533,7 @@ static xr_status rc_set_volumes_impl(xr_raycaster rc, int32_t n, const xr_volume
     }
     if (cells) {
       XR_CUDA_TRY(v->cells.reserve(cell_bytes));
-      XR_CUDA_TRY(launch_build_cells(src, nx, ny, nz, vt, sc, v->cells.p, own_vox, s));
+      XR_CUDA_TRY(launch_build_cells(src, nx, ny, nz, vt, sc, v->weighted, v->cells.p, own_vox, s));
     } else if (own_vox && vt == XR_VOXEL_F32) {
       XR_CUDA_TRY(cudaMemcpyAsync(own_vox, src, vox_bytes, cudaMemcpyDeviceToDevice, s));
     } else if (own_vox) {
@@ -945,15 +945,14 @@ static int32_t best_layout(const xr_raycaster_s::Vol& vol) {
 static xr_status rc_choose_config(xr_raycaster rc, const xr_raycaster_s::Vol& vol, DrrParams& p, cudaStream_t s,
                                   int32_t* loop) {
   if (rc->cfg_layout != XR_LAYOUT_AUTO) {
-    const bool has_cells = vol.cells.p != nullptr || vol.weighted || vol.linear_only;
+    const bool has_cells = vol.cells.p != nullptr || vol.linear_only;
     if (rc->cfg_layout != XR_LAYOUT_LINEAR && !has_cells)
       return fail(XR_ERR_INVALID_ARG, "compute: CELL8 layout requested but the volume has no cell copy");
     if (rc->cfg_layout == 2 && vol.type != XR_VOXEL_F32)
       return fail(XR_ERR_INVALID_ARG, "compute: the 256-bit CELL8 read needs a float32 volume");
     if (rc->cfg_layout == 3 && (vol.type != XR_VOXEL_F32 || p.kernel_id != XR_LINE_INT_SUM))
       return fail(XR_ERR_INVALID_ARG, "compute: the brick-staged layout needs a float32 volume and the sum kernel");
-    // only LINEAR has the weighted blend
-    p.vol.layout = vol.weighted || vol.linear_only ? XR_LAYOUT_LINEAR : rc->cfg_layout;
+    p.vol.layout = vol.linear_only ? XR_LAYOUT_LINEAR : rc->cfg_layout;
     p.block_warps_x = rc->cfg_bw;
     p.warp_tall = rc->cfg_warp_rows == 8 ? 1 : 0;
     *loop = rc->cfg_unroll;

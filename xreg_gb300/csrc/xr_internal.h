@@ -37,8 +37,8 @@ struct VolView {
   float kfl[3];
   int32_t cell_bytes;
   // 1: the voxels hold infinities or values above 2^126, so the trilinear takes
-  // the weighted form on the LINEAR layout (differences of corners would not be
-  // finite); such a volume has no cells.
+  // the weighted form (differences of corners would not be finite): float32 cells
+  // hold their corners, and rays along the faces take the clamped sampler.
   int32_t weighted;
   // Support box: every sample whose continuous index lies outside
   // (sup_lo, sup_hi) on some axis interpolates only zero voxels.  has_support 0
@@ -124,10 +124,11 @@ struct VolStats {
 // VolView::occ; d_occ holds ceil(nmx * nmy * nmz / 32) words).
 cudaError_t launch_volume_stats(const float* vox_f32, int nx, int ny, int nz, uint32_t* d_occ, int nmx, int nmy, int nmz,
                                 VolStats* d_stats, cudaStream_t s);
-// The CELL8 copy from float32 voxels, scaled by `scale` for the 16-bit types, and,
+// The CELL8 copy from float32 voxels, scaled by `scale` for the 16-bit types (of a
+// float32 volume with the x differences, or with the corners when `weighted`), and,
 // unless out_vox is nullptr, the voxels in the volume's own type.
 cudaError_t launch_build_cells(const float* vox_f32, int nx, int ny, int nz, int32_t voxel_type, float scale,
-                               void* out, void* out_vox, cudaStream_t s);
+                               bool weighted, void* out, void* out_vox, cudaStream_t s);
 // The voxels in a 16-bit type alone.
 cudaError_t launch_convert_voxels(const float* vox_f32, int64_t n, int32_t voxel_type, float scale, void* out,
                                   cudaStream_t s);

@@ -29,7 +29,8 @@
 //           It spends 8x the voxel bytes of HBM to cut L1 requests per sample
 //           from 8 to 1-2; the linear kernel is bound by exactly those requests.
 //           Float32 cells hold, in place of the x + 1 corners, their differences
-//           to the x corners (v1yz - v0yz), the first blend's slope.
+//           to the x corners (v1yz - v0yz), the first blend's slope (but for
+//           VolView::weighted volumes, which hold the corners).
 //           Cells are numbered z fastest, then x, then y (VolView::cs).  The
 //           border cells (index -1 and n-1) are constant along their axis: a
 //           position that rounding carries past a face of the volume reads the
@@ -309,20 +310,39 @@ struct CellData {
     static_assert(VT == XR_VOXEL_BF16, "");
     return interp8_pairs(w, f.xy, f.z);
   }
+  // of a volume with VolView::weighted, whose float32 cells hold their corners
+  __device__ __forceinline__ float weighted_value(const Frac21& f) const {
+    Frac3 g;
+    upk2(f.xy, g.x, g.y);
+    g.z = f.z;
+    return weighted_value(g);
+  }
+  __device__ __forceinline__ float weighted_value(const Frac3& f) const {
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if constexpr (VT == XR_VOXEL_F32) v[k] = __uint_as_float(w[k]);
+      else v[k] = __uint_as_float((k & 1) ? (w[k >> 1] & 0xffff0000u) : (w[k >> 1] << 16));
+    }
+    return interp8_weighted(v, f.x, f.y, f.z);
+  }
 };
 
 // Trilinear sample at index position (px, py, pz) with ITK's boundary rule:
 // positions past a face take the face's values.  The cell is floor(position)
 // clamped to [-1, n-1], the fraction saturated to [0, 1] (a NaN position reads
 // cell 0 with fraction 0).  INSIDE (LINEAR only): the caller has shown that the
-// position lies in [0, n-1) on every axis, where no clamp changes anything.
+// position lies in [0, n-1) on every axis, where no clamp changes anything.  A
+// weighted volume's cells end at n-2 (fraction 1 on the last voxel), without the
+// border's: there a corner of weight 0 decides whether an infinity makes a NaN.
 template <int VT, int LAYOUT, bool INSIDE = false>
 __device__ __forceinline__ float sample(const VolView& vol, const void* data, float px, float py, float pz) {
   int ix = __float2int_rd(px), iy = __float2int_rd(py), iz = __float2int_rd(pz);
   if (!INSIDE) {
-    ix = clampi(ix, -1, vol.nx - 1);
-    iy = clampi(iy, -1, vol.ny - 1);
-    iz = clampi(iz, -1, vol.nz - 1);
+    const int b = VT != XR_VOXEL_F16 && vol.weighted ? 1 : 0;
+    ix = clampi(ix, b - 1, vol.nx - 1 - b);
+    iy = clampi(iy, b - 1, vol.ny - 1 - b);
+    iz = clampi(iz, b - 1, vol.nz - 1 - b);
   }
   float fx = px - (float)ix, fy = py - (float)iy, fz = pz - (float)iz;
   if (!INSIDE) {
@@ -365,6 +385,8 @@ __device__ __forceinline__ float sample(const VolView& vol, const void* data, fl
                            (unsigned int)(iy + 1) * (unsigned int)vol.cs[1] + (unsigned int)(iz + 1);
     CellData<VT, LAYOUT> q;
     q.load(data, c);
+    if constexpr (VT != XR_VOXEL_F16)
+      if (vol.weighted) return q.weighted_value(Frac3{fx, fy, fz});
     constexpr float kS = VT == XR_VOXEL_F16 ? kH16 : 1.0f;
     return q.value(Frac3{fx * kS, fy * kS, fz});
   }
@@ -484,7 +506,8 @@ struct CellWalk<XR_VOXEL_BF16, BYTES> {
 // scalar batches of four 5144 / 2873 / 1726, packed batches - / 3025 / 1690,
 // packed reload 7029 / 3464 / 1613 (the reload form spills at float32's and
 // FP16's register need), scalar reload of three 5317 / - / -.
-template <int VT, int KERNEL, int LAYOUT, bool BYTES, bool DEEP>
+// WEIGHTED: of a VolView::weighted volume, by weights (no DEEP).
+template <int VT, int KERNEL, int LAYOUT, bool BYTES, bool DEEP, bool WEIGHTED>
 __device__ __forceinline__ float march_cells(const VolView& vol, float px, float py, float pz, float sx, float sy,
                                              float sz, unsigned int n, float sum) {
   using Cell = CellData<VT, LAYOUT>;
@@ -492,6 +515,10 @@ __device__ __forceinline__ float march_cells(const VolView& vol, float px, float
   using Frac = typename Walk::Frac;
   const void* data = vol.cells;
   Walk walk(vol, px, py, pz, sx, sy, sz);
+  auto value = [](const Cell& q, const Frac& f) {
+    if constexpr (WEIGHTED) return q.weighted_value(f);
+    else return q.value(f);
+  };
   if constexpr (DEEP) {  // batches of eight, the last one masked
     constexpr unsigned int kDeep = 8;
     unsigned int c = 0;
@@ -507,14 +534,14 @@ __device__ __forceinline__ float march_cells(const VolView& vol, float px, float
       }
 #pragma unroll
       for (unsigned int k = 0; k < kDeep; ++k) {
-        const float v = fold<KERNEL>(sum, q[k].value(f[k]));
+        const float v = fold<KERNEL>(sum, value(q[k], f[k]));
         sum = k < m ? v : sum;
       }
       n -= m;
     }
     return sum;
   }
-  if constexpr (VT == XR_VOXEL_BF16) {
+  if constexpr (VT == XR_VOXEL_BF16 && !WEIGHTED) {
     if (n >= 4) {
       Frac f[4];
       Cell q[4];
@@ -523,12 +550,12 @@ __device__ __forceinline__ float march_cells(const VolView& vol, float px, float
       for (n -= 4; n >= 4; n -= 4) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          sum = fold<KERNEL>(sum, q[k].value(f[k]));
+          sum = fold<KERNEL>(sum, value(q[k], f[k]));
           q[k].template load<BYTES>(data, walk.next(f[k]));
         }
       }
 #pragma unroll
-      for (int k = 0; k < 4; ++k) sum = fold<KERNEL>(sum, q[k].value(f[k]));
+      for (int k = 0; k < 4; ++k) sum = fold<KERNEL>(sum, value(q[k], f[k]));
     }
   } else {
     for (; n >= 4; n -= 4) {
@@ -537,14 +564,14 @@ __device__ __forceinline__ float march_cells(const VolView& vol, float px, float
 #pragma unroll
       for (int k = 0; k < 4; ++k) q[k].template load<BYTES>(data, walk.next(f[k]));
 #pragma unroll
-      for (int k = 0; k < 4; ++k) sum = fold<KERNEL>(sum, q[k].value(f[k]));
+      for (int k = 0; k < 4; ++k) sum = fold<KERNEL>(sum, value(q[k], f[k]));
     }
   }
   for (; n > 0; --n) {
     Frac f;
     Cell q;
     q.template load<BYTES>(data, walk.next(f));
-    sum = fold<KERNEL>(sum, q.value(f));
+    sum = fold<KERNEL>(sum, value(q, f));
   }
   return sum;
 }
@@ -554,14 +581,12 @@ __device__ __forceinline__ float march_cells(const VolView& vol, float px, float
 template <int VT, int KERNEL, int LAYOUT, bool INSIDE>
 __device__ __forceinline__ float march_samples(const VolView& vol, const void* data, float px, float py, float pz,
                                                float sx, float sy, float sz, unsigned int n, float sum) {
-  if (LAYOUT == XR_LAYOUT_LINEAR) {
-    for (; n >= 2; n -= 2) {
-      const float v0 = sample<VT, LAYOUT, INSIDE>(vol, data, px, py, pz);
-      px = __fadd_rn(px, sx); py = __fadd_rn(py, sy); pz = __fadd_rn(pz, sz);
-      const float v1 = sample<VT, LAYOUT, INSIDE>(vol, data, px, py, pz);
-      px = __fadd_rn(px, sx); py = __fadd_rn(py, sy); pz = __fadd_rn(pz, sz);
-      sum = fold<KERNEL>(fold<KERNEL>(sum, v0), v1);
-    }
+  for (; n >= 2; n -= 2) {
+    const float v0 = sample<VT, LAYOUT, INSIDE>(vol, data, px, py, pz);
+    px = __fadd_rn(px, sx); py = __fadd_rn(py, sy); pz = __fadd_rn(pz, sz);
+    const float v1 = sample<VT, LAYOUT, INSIDE>(vol, data, px, py, pz);
+    px = __fadd_rn(px, sx); py = __fadd_rn(py, sy); pz = __fadd_rn(pz, sz);
+    sum = fold<KERNEL>(fold<KERNEL>(sum, v0), v1);
   }
   for (; n > 0; --n) {
     const float v0 = sample<VT, LAYOUT, INSIDE>(vol, data, px, py, pz);
@@ -575,7 +600,7 @@ __device__ __forceinline__ float march_samples(const VolView& vol, const void* d
 // (the caller checks that the pixel exists).  Returns the number of samples of
 // the reference step rule; *loaded receives how many of them were loaded (the
 // others were proven zero and skipped).
-template <int VT, int KERNEL, int LAYOUT, bool DEEP = false>
+template <int VT, int KERNEL, int LAYOUT, bool DEEP = false, bool WEIGHTED = false>
 __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, const int64_t proj, const int row,
                                                           const int col, unsigned int* loaded) {
   float sum = (KERNEL == XR_LINE_INT_MAX) ? -FLT_MAX : 0.0f;
@@ -672,10 +697,12 @@ __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, co
       // march_cells, whose loads no clamp bounds.  Rays of ordinary frames all lie
       // there; a NaN or infinite start or step does not, nor one that a focal point
       // millions of voxels away rounds off the volume: those take the clamped
-      // sampler.  On the LINEAR layout rays a quarter voxel inside run without clamps.
-      bool unclamped = drift_ok && (LAYOUT == XR_LAYOUT_LINEAR || p.vol.kfl[0] > 0.0f);
-      if (unclamped)
-        unclamped = xf::samples_within(st0, stv, first, last, maxb, LAYOUT == XR_LAYOUT_LINEAR ? -0.25f : 0.75f);
+      // sampler.  On the LINEAR layout, and of weighted volumes, rays a quarter voxel
+      // inside run without clamps.
+      constexpr bool kInside = LAYOUT == XR_LAYOUT_LINEAR || WEIGHTED;
+      bool unclamped =
+          drift_ok && (LAYOUT == XR_LAYOUT_LINEAR || (p.vol.kfl[0] > 0.0f && (WEIGHTED || !p.vol.weighted)));
+      if (unclamped) unclamped = xf::samples_within(st0, stv, first, last, maxb, kInside ? -0.25f : 0.75f);
       if (hit) {
         // advance to sample `first` (four additions per trip: the skipped samples
         // are a large part of a trimmed ray); x and y as one packed pair, whose
@@ -703,8 +730,8 @@ __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, co
             sum = march_samples<VT, KERNEL, LAYOUT, true>(p.vol, data, px, py, pz, sx, sy, sz, n, sum);
           else
             sum = p.vol.cell_bytes
-                      ? march_cells<VT, KERNEL, LAYOUT, true, DEEP>(p.vol, px, py, pz, sx, sy, sz, n, sum)
-                      : march_cells<VT, KERNEL, LAYOUT, false, DEEP>(p.vol, px, py, pz, sx, sy, sz, n, sum);
+                      ? march_cells<VT, KERNEL, LAYOUT, true, DEEP, WEIGHTED>(p.vol, px, py, pz, sx, sy, sz, n, sum)
+                      : march_cells<VT, KERNEL, LAYOUT, false, DEEP, WEIGHTED>(p.vol, px, py, pz, sx, sy, sz, n, sum);
         } else {
           sum = march_samples<VT, KERNEL, LAYOUT, false>(p.vol, data, px, py, pz, sx, sy, sz, n, sum);
         }
@@ -734,7 +761,7 @@ __device__ __forceinline__ void lane_pixel(int lane, int wl, int& col, int& row)
   row = ((lane >> 1) & 1) + ((lane >> (wl + 1)) << 1);
 }
 
-template <int VT, int KERNEL, int LAYOUT, bool DEEP>
+template <int VT, int KERNEL, int LAYOUT, bool DEEP, bool WEIGHTED>
 __global__ void __launch_bounds__(32 * kWarps, DEEP ? kDeepBlocksPerSM : kMinBlocksPerSM * 8 / kWarps)
 drr_kernel(const DrrParams p, const int64_t proj_base) {
   // Each warp covers an 8 x 4 (or, tall, 4 x 8) patch of pixels so its 32 rays
@@ -752,7 +779,7 @@ drr_kernel(const DrrParams p, const int64_t proj_base) {
   const int64_t proj = proj_base + blockIdx.x;
   unsigned long long ns = 0;
   unsigned int nl = 0;
-  if (col < p.cols && row < p.rows) ns = trace_pixel<VT, KERNEL, LAYOUT, DEEP>(p, proj, row, col, &nl);
+  if (col < p.cols && row < p.rows) ns = trace_pixel<VT, KERNEL, LAYOUT, DEEP, WEIGHTED>(p, proj, row, col, &nl);
   if (p.sample_counter) {
     unsigned long long nlw = nl;
     for (int o = 16; o > 0; o >>= 1) {
@@ -783,10 +810,15 @@ __device__ __forceinline__ void cell3(const VolView& vol, const float pos[3], in
   const int n[3] = {vol.nx, vol.ny, vol.nz};
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const int i = clampi(__float2int_rd(pos[a]), -1, n[a] - 1);
+    const int b = vol.weighted ? 1 : 0;
+    const int i = clampi(__float2int_rd(pos[a]), b - 1, n[a] - 1 - b);
     f[a] = __saturatef(pos[a] - (float)i);
     c[a] = i + 1;
   }
+}
+
+__device__ __forceinline__ float brick_value(const VolView& vol, const float v[8], const float f[3]) {
+  return vol.weighted ? interp8_weighted(v, f[0], f[1], f[2]) : interp8<true>(v, f[0], f[1], f[2]);
 }
 
 // The ray's remaining samples k..last from global memory, in order.
@@ -797,7 +829,7 @@ __device__ __forceinline__ float brick_march_global(const VolView& vol, float po
     float f[3], v[8];
     cell3(vol, pos, c, f);
     Vox<XR_VOXEL_F32>::cell_wide(vol.cells, (unsigned int)c[0] * vol.cs[0] + (unsigned int)c[1] * vol.cs[1] + (unsigned int)c[2], v);
-    sum = __fadd_rn(sum, interp8<true>(v, f[0], f[1], f[2]));
+    sum = __fadd_rn(sum, brick_value(vol, v, f));
     pos[0] = __fadd_rn(pos[0], st[0]);
     pos[1] = __fadd_rn(pos[1], st[1]);
     pos[2] = __fadd_rn(pos[2], st[2]);
@@ -972,7 +1004,7 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
           } else {
             Vox<XR_VOXEL_F32>::cell_wide(vol.cells, (unsigned int)c[0] * vol.cs[0] + (unsigned int)c[1] * vol.cs[1] + (unsigned int)c[2], v);
           }
-          sum = __fadd_rn(sum, interp8<true>(v, f[0], f[1], f[2]));
+          sum = __fadd_rn(sum, brick_value(vol, v, f));
           pos[0] = __fadd_rn(pos[0], st[0]);
           pos[1] = __fadd_rn(pos[1], st[1]);
           pos[2] = __fadd_rn(pos[2], st[2]);
@@ -1312,7 +1344,7 @@ cudaError_t launch_jobs_t(const MultiJobDrr* d_jobs, int njobs, long long total,
                  : launch_jobs_g<VT, LAYOUT, false>(d_jobs, njobs, total, s);
 }
 
-template <int VT, int KERNEL, int LAYOUT, bool DEEP>
+template <int VT, int KERNEL, int LAYOUT, bool DEEP, bool WEIGHTED = false>
 cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
   // The kernel uses no shared memory: ask for the largest L1 (the gathers hit
   // it), once per device (a preference; setting it twice is harmless).
@@ -1320,7 +1352,7 @@ cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
       !carveout_set[dev].load(std::memory_order_relaxed)) {
-    cudaFuncSetAttribute(drr_kernel<VT, KERNEL, LAYOUT, DEEP>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(drr_kernel<VT, KERNEL, LAYOUT, DEEP, WEIGHTED>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxL1);
     carveout_set[dev].store(true, std::memory_order_relaxed);
   }
@@ -1331,7 +1363,7 @@ cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
   for (int64_t base = 0; base < p.num_projs; base += max_x) {
     const int64_t n = (p.num_projs - base) < max_x ? (p.num_projs - base) : max_x;
     const dim3 grid((unsigned)n, (p.cols + tx - 1) / tx, (p.rows + ty - 1) / ty);
-    drr_kernel<VT, KERNEL, LAYOUT, DEEP><<<grid, 32 * kWarps, 0, s>>>(p, base);
+    drr_kernel<VT, KERNEL, LAYOUT, DEEP, WEIGHTED><<<grid, 32 * kWarps, 0, s>>>(p, base);
   }
   return cudaGetLastError();
 }
@@ -1347,6 +1379,10 @@ cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
 template <int VT, int KERNEL, int LAYOUT>
 cudaError_t launch_t(const DrrParams& p, cudaStream_t s) {
   if constexpr (LAYOUT != XR_LAYOUT_LINEAR) {
+    // Volumes with an infinity have a march of their own, four by weights (20 images
+    // of 256^2 of a 256 x 256 x 200 float32 volume: 616 us through the clamped sampler).
+    if constexpr (VT != XR_VOXEL_F16)
+      if (p.vol.weighted) return launch_depth<VT, KERNEL, LAYOUT, false, true>(p, s);
     static std::atomic<int> cached[kMaxDevices];  // SMs per device; zero = not known yet
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {

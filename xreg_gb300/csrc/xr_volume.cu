@@ -198,8 +198,9 @@ constexpr int kBuildY = 16, kTile = 32, kPlane = kTile + 1;
 
 template <int VT>
 __global__ void __launch_bounds__(kThreads) build_cells_kernel(const float* __restrict__ vox, int nx, int ny, int nz,
-                                                               float scale, int32_t csx, int32_t csy, int tx, int tz,
-                                                               void* __restrict__ out, void* __restrict__ out_vox) {
+                                                               float scale, bool weighted, int32_t csx, int32_t csy,
+                                                               int tx, int tz, void* __restrict__ out,
+                                                               void* __restrict__ out_vox) {
   __shared__ float plane[2][kPlane * kPlane];  // [y parity][z][x], odd pitch: columns are free of bank conflicts
   const int bx = (int)(blockIdx.x % tx), bz = (int)(blockIdx.x / tx % tz), by = (int)(blockIdx.x / tx / tz);
   const int cx0 = bx * kTile, cz0 = bz * kTile, cy0 = by * kBuildY;  // first cell (index + 1)
@@ -246,9 +247,14 @@ __global__ void __launch_bounds__(kThreads) build_cells_kernel(const float* __re
         const int64_t cell = (int64_t)(cx0 + xi) * csx + (int64_t)cy * csy + cz0 + lane;
         if constexpr (VT == XR_VOXEL_F32) {
           float* q = static_cast<float*>(out) + 8 * cell;
-          asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(q), "f"(c[0]), "f"(c[1]),
-                       "f"(__fsub_rn(c[2], c[0])), "f"(__fsub_rn(c[3], c[1])), "f"(c[4]), "f"(c[5]),
-                       "f"(__fsub_rn(c[6], c[4])), "f"(__fsub_rn(c[7], c[5]))
+          float d[4];  // the x + 1 corners, as cells hold them
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int k0 = (i & 1) + 4 * (i >> 1);
+            d[i] = weighted ? c[k0 + 2] : __fsub_rn(c[k0 + 2], c[k0]);
+          }
+          asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(q), "f"(c[0]), "f"(c[1]), "f"(d[0]),
+                       "f"(d[1]), "f"(c[4]), "f"(c[5]), "f"(d[2]), "f"(d[3])
                        : "memory");
         } else {
           static_cast<uint4*>(out)[cell] = make_uint4(half_pair<VT>(c[0], c[1]), half_pair<VT>(c[2], c[3]),
@@ -307,7 +313,7 @@ cudaError_t launch_volume_stats(const float* vox, int nx, int ny, int nz, uint32
 }
 
 cudaError_t launch_build_cells(const float* vox_f32, int nx, int ny, int nz, int32_t voxel_type, float scale,
-                               void* out, void* out_vox, cudaStream_t s) {
+                               bool weighted, void* out, void* out_vox, cudaStream_t s) {
   int32_t cs[2];
   cell_strides(nx, ny, nz, cs);
   const int64_t tx = (nx + (int64_t)kTile) / kTile, tz = (nz + (int64_t)kTile) / kTile,
@@ -315,15 +321,15 @@ cudaError_t launch_build_cells(const float* vox_f32, int nx, int ny, int nz, int
   const unsigned blocks = (unsigned)(tx * ty * tz);
   switch (voxel_type) {
     case XR_VOXEL_F32:
-      build_cells_kernel<XR_VOXEL_F32><<<blocks, kThreads, 0, s>>>(vox_f32, nx, ny, nz, 1.0f, cs[0], cs[1], (int)tx,
+      build_cells_kernel<XR_VOXEL_F32><<<blocks, kThreads, 0, s>>>(vox_f32, nx, ny, nz, 1.0f, weighted, cs[0], cs[1], (int)tx,
                                                                    (int)tz, out, out_vox);
       break;
     case XR_VOXEL_F16:
-      build_cells_kernel<XR_VOXEL_F16><<<blocks, kThreads, 0, s>>>(vox_f32, nx, ny, nz, scale, cs[0], cs[1], (int)tx,
+      build_cells_kernel<XR_VOXEL_F16><<<blocks, kThreads, 0, s>>>(vox_f32, nx, ny, nz, scale, weighted, cs[0], cs[1], (int)tx,
                                                                    (int)tz, out, out_vox);
       break;
     case XR_VOXEL_BF16:
-      build_cells_kernel<XR_VOXEL_BF16><<<blocks, kThreads, 0, s>>>(vox_f32, nx, ny, nz, scale, cs[0], cs[1], (int)tx,
+      build_cells_kernel<XR_VOXEL_BF16><<<blocks, kThreads, 0, s>>>(vox_f32, nx, ny, nz, scale, weighted, cs[0], cs[1], (int)tx,
                                                                     (int)tz, out, out_vox);
       break;
     default: return cudaErrorInvalidValue;
