@@ -1316,9 +1316,14 @@ cudaError_t launch_patch_fixed_stats(const float* img, int rows, int cols, int r
 // Patches a thread scores in a column (patch_rows_kernel).  One while a patch a thread
 // does not fill the GPU (1024 threads an SM): four would leave SMs idle (6 images of
 // 311 x 476, 15 x 15 at stride 3, a whole call: 56 us against 81 with four; 16 of 215 x
-// 493, 11 x 11 at stride 2, above the line: 79 against 60).  The general kernel with
-// masked statistics, moving-variance weights or tiles too large.
+// 493, 11 x 11 at stride 2, above the line: 79 against 60).  Four while two blocks' tiles
+// fit an SM (228 KB, 4 KB of static and 1 KB of reserved memory a block): one block of 8
+// warps cannot hide its own staging (24 images of 384^2 at stride 3, 7 x 7, 11 x 11 and
+// 15 x 15, masked: 88, 104, 125 us with four, 62, 79, 104 with one; at stride 2, 15 x 15,
+// both gradients, 96 KB: 179 with four, 234 with one).  The general kernel with masked
+// statistics, moving-variance weights or tiles too large.
 constexpr size_t kPatchSmem = 200 * 1024;
+constexpr size_t kPatchSmemFour = 109 * 1024;
 
 static size_t patch_rows_bytes(int radius, int stride, int grad, const PatchRun& run, int rb) {
   return PatchRows::make(radius, stride, grad, run.mask != nullptr, rb).bytes;
@@ -1341,7 +1346,7 @@ static cudaError_t patch_rb(int radius, int stride, int grad, const PatchRun& ru
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   const bool many = (int64_t)ncr * ncc * nimgs > (int64_t)sms * 1024;
-  *rb = many && patch_rows_bytes(radius, stride, grad, run, 4) <= kPatchSmem ? 4 : 1;
+  *rb = many && patch_rows_bytes(radius, stride, grad, run, 4) <= kPatchSmemFour ? 4 : 1;
   return e;
 }
 
