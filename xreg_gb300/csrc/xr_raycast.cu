@@ -1131,8 +1131,12 @@ __device__ __noinline__ void fused_metric_image(const FusedJob& J, int64_t proj,
   }
 }
 
+// Resident blocks per SM: 48 registers, but for BF16, whose reload form spills in this
+// kernel at 48 (3 views of 250 x 240 under 57 poses 4158 us, at 64 registers 2804).
+constexpr int fused_blocks(int vt) { return vt == XR_VOXEL_BF16 ? kMinBlocksPerSM - 1 : kMinBlocksPerSM; }
+
 template <int VT, int LAYOUT>
-__global__ void __launch_bounds__(kThreads, kMinBlocksPerSM)
+__global__ void __launch_bounds__(kThreads, fused_blocks(VT))
 eval_fused_kernel(const FusedJob* __restrict__ jobs, int njobs, long long total, unsigned long long* counter) {
   // under 1 KB of shared memory: the SM's unified L1 stays with the DRR gathers
   __shared__ long long s_item;
@@ -1302,7 +1306,7 @@ cudaError_t launch_fused_t(const FusedJob* d_jobs, int njobs, long long total, u
     cudaError_t e = cudaFuncGetAttributes(&fa, eval_fused_kernel<VT, LAYOUT>);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     if (e != cudaSuccess) return e;
-    const double need = (double)(fa.sharedSizeBytes + 1024) * kMinBlocksPerSM;
+    const double need = (double)(fa.sharedSizeBytes + 1024) * fused_blocks(VT);
     const int pct = std::min(100, (int)std::ceil(100.0 * need / (double)std::max(smem_sm, 1)) + 1);
     e = cudaFuncSetAttribute(eval_fused_kernel<VT, LAYOUT>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
     if (e != cudaSuccess) return e;
