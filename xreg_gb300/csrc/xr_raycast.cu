@@ -1268,8 +1268,10 @@ drr_jobs_kernel(const MultiJobDrr* __restrict__ jobs, int njobs, long long item0
       row = ty * 8 + (warp >> 2) * 4 + ((lane & 7) >> 1);
     } else {
       q = warp >> 1;
-      col = tx * 8 + (lane & 7);
-      row = ty * 8 + (warp & 1) * 4 + (lane >> 3);
+      int lc, lr;
+      lane_pixel(lane, 3, lc, lr);
+      col = tx * 8 + lc;
+      row = ty * 8 + (warp & 1) * 4 + lr;
     }
     proj = p0 + q;
     if (proj >= nproj) return;
