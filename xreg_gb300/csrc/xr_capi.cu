@@ -2234,12 +2234,16 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
                                    rc->d_geo.as<ProjGeom>(), s));
       ++tuning_launches;
     }
+    // the macro-cell trim runs whatever loop the caster's own computes are set to
     int32_t loop = 0;
+    const uint32_t* occ = P.vol.occ;
     if ((st = rc_choose_config(rc, vol, P, s, &loop)) != XR_OK) return st;
+    P.vol.occ = occ;
+    loop = std::max(loop, 3);
     P.vol.layout = best_layout(vol);
-    rc->last_bw = P.block_warps_x;
     const int warps = fused ? 8 : kDrrWarps;
     P.block_warps_x = std::min(P.block_warps_x, warps);
+    rc->last_bw = P.block_warps_x;
     const int wc = P.warp_tall ? 4 : 8, tw = wc * P.block_warps_x, th = (warps / P.block_warps_x) * (32 / wc);
     J.d.tiles_x = (int32_t)((P.cols + tw - 1) / tw);
     J.d.tiles_y = (int32_t)((P.rows + th - 1) / th);
