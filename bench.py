@@ -445,11 +445,12 @@ def run_ours(a, rank, world, local):
     lname = {0: "linear", 1: "cell8", 2: "cell8-256bit"}.get(layout, str(layout))
     wcols = 32 // wrows
     wshape = "" if wrows == 4 else f"-warp{wcols}x{wrows}"
-    block = f"{wcols * bw}x{(8 // bw) * wrows}"
+    block = f"{wcols * bw}x{max(4 // bw, 1) * wrows}"  # 4 warps a block, or the 8 across
     tag = f"batched-256^3-384^2-pop100-{a.voxel}-{lname}-loop{unroll}{wshape}"
     l2_peak = xr.measure_l2_read_bandwidth(dev)
     roofline = _roofline(vt, layout, drr_ms, samples, loaded, l2_peak, tag)
-    roofline["kernel"] = f"drr_kernel<{a.voxel},sum,{lname},unroll{unroll}> block {block}, warps {wcols}x{wrows}"
+    trim = "trimmed" if unroll >= 3 else "untrimmed"
+    roofline["kernel"] = f"drr_kernel<{a.voxel},sum,{lname},{trim}> block {block}, warps {wcols}x{wrows}"
 
     extras = {}
     if not a.no_extras and rank == 0:

@@ -214,8 +214,9 @@ XR_API xr_status xr_rc_set_count_samples(xr_raycaster rc, int32_t enable);
  * axis copied to shared memory and sampled from there; float32 volumes and the
  * sum kernel; identical values, measured 3-4x slower than the gather, never
  * autotuned; block shape and loop are ignored), warps
- * across a block (1, 2, 4 or 8, at most the warps of a block: 4, or 8 in the
- * fused evaluation; each warp covers 8x4 pixels) and
+ * across a block (1, 2, 4 or 8; each warp covers 8x4 pixels, a block is 4 warps,
+ * or the 8 across; job steps run 4 across at most, the fused evaluation has
+ * blocks of 8) and
  * the loop number: 1 and 2 sample from the support box on, 3 to 6 after each ray
  * is trimmed to its first and last occupied macro cell (sum kernel with
  * empty-space skipping on; otherwise as 2).  layout

@@ -53,7 +53,7 @@ struct VolView {
 };
 constexpr int kMacroShift = 3;  // macro cells of 8 x 8 x 8 trilinear cells
 
-constexpr int kDrrWarps = 4;    // warps per block of the DRR kernels (the fused evaluation's: 8)
+constexpr int kDrrWarps = 4;    // warps per block of the DRR kernels (the fused evaluation's, and of 8 across: 8)
 
 // Launch parameters of a DRR kernel.
 struct DrrParams {
@@ -72,7 +72,8 @@ struct DrrParams {
   float default_bg;
   int32_t kernel_id;      // XR_LINE_INT_SUM / MAX
   int32_t store;          // XR_PROJ_STORE_REPLACE / ACCUM
-  int32_t block_warps_x;  // warps across a block (1, 2, 4, 8; at most the block's)
+  int32_t block_warps_x;  // warps across a block (1, 2, 4, 8)
+  int32_t block_warps_y;  // warps down a block of drr_kernel (set by launch_drr)
   int32_t warp_tall;      // 0: each warp covers 8x4 pixels (cols x rows); 1: 4x8
 };
 

@@ -103,6 +103,7 @@ constexpr int kMinBlocksPerSM = 5;
 // faster than 8 (population 4867 -> 4785 us, FP16 coarse 2837 -> 2718, BF16 1570 ->
 // 1521), 2 or 1 mixed (4749 / 2728 / 1545, 5178 / 2710 / 1497).
 constexpr int kWarps = kDrrWarps;
+constexpr int kMaxWarps = 8;  // of a drr_kernel block: 8 warps across where the caller asks for them
 constexpr int kDeepBlocksPerSM = 4;  // of the deep march (launch_t): 128 registers
 // CELL8 data read with one 256-bit load per sample (float32 volumes only).
 constexpr int kLayoutCell8Wide = 2;
@@ -762,10 +763,10 @@ __device__ __forceinline__ void lane_pixel(int lane, int wl, int& col, int& row)
 }
 
 template <int VT, int KERNEL, int LAYOUT, bool DEEP, bool WEIGHTED>
-__global__ void __launch_bounds__(32 * kWarps, DEEP ? kDeepBlocksPerSM : kMinBlocksPerSM * 8 / kWarps)
+__global__ void __launch_bounds__(32 * kMaxWarps, (DEEP ? kDeepBlocksPerSM : kMinBlocksPerSM * 8 / kWarps) * kWarps / kMaxWarps)
 drr_kernel(const DrrParams p, const int64_t proj_base) {
   // Each warp covers an 8 x 4 (or, tall, 4 x 8) patch of pixels so its 32 rays
-  // stay close inside the volume; a block is bw x (kWarps / bw) warps.  The
+  // stay close inside the volume; a block is bw x bh warps, kWarps or bw of them.  The
   // projection is the fastest grid index: blocks resident at the same time trace
   // the same detector tile for many nearby poses, whose footprints overlap in L2.
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -775,7 +776,7 @@ drr_kernel(const DrrParams p, const int64_t proj_base) {
   int lc, lr;
   lane_pixel(lane, wl, lc, lr);
   const int col = blockIdx.y * (wc * bw) + (warp % bw) * wc + lc;
-  const int row = blockIdx.z * ((kWarps / bw) * wr) + (warp / bw) * wr + lr;
+  const int row = blockIdx.z * (p.block_warps_y * wr) + (warp / bw) * wr + lr;
   const int64_t proj = proj_base + blockIdx.x;
   unsigned long long ns = 0;
   unsigned int nl = 0;
@@ -1364,12 +1365,12 @@ cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
   }
   const int bw = p.block_warps_x;
   const int wc = p.warp_tall ? 4 : 8;
-  const int tx = wc * bw, ty = (kWarps / bw) * (32 / wc);
+  const int tx = wc * bw, ty = p.block_warps_y * (32 / wc);
   const int64_t max_x = 0x7fffffff;
   for (int64_t base = 0; base < p.num_projs; base += max_x) {
     const int64_t n = (p.num_projs - base) < max_x ? (p.num_projs - base) : max_x;
     const dim3 grid((unsigned)n, (p.cols + tx - 1) / tx, (p.rows + ty - 1) / ty);
-    drr_kernel<VT, KERNEL, LAYOUT, DEEP, WEIGHTED><<<grid, 32 * kWarps, 0, s>>>(p, base);
+    drr_kernel<VT, KERNEL, LAYOUT, DEEP, WEIGHTED><<<grid, 32 * bw * p.block_warps_y, 0, s>>>(p, base);
   }
   return cudaGetLastError();
 }
@@ -1441,11 +1442,11 @@ cudaError_t launch_brick(const DrrParams& p, cudaStream_t s) {
 
 cudaError_t launch_drr(const DrrParams& params, cudaStream_t s) {
   DrrParams p = params;
-  p.block_warps_x = std::min(p.block_warps_x, kWarps);
   if (p.num_projs <= 0) return cudaSuccess;
   if (p.vol.layout == kLayoutBrick) return launch_brick(p, s);
-  if (!(p.block_warps_x == 1 || p.block_warps_x == 2 || p.block_warps_x == 4))
+  if (!(p.block_warps_x == 1 || p.block_warps_x == 2 || p.block_warps_x == 4 || p.block_warps_x == 8))
     return cudaErrorInvalidValue;
+  p.block_warps_y = std::max(kWarps / p.block_warps_x, 1);
   if (p.warp_tall != 0 && p.warp_tall != 1) return cudaErrorInvalidValue;
   if (p.vol.layout != XR_LAYOUT_LINEAR && !p.vol.cells) return cudaErrorInvalidValue;
   if (p.vol.layout == kLayoutCell8Wide && p.vol.voxel_type != XR_VOXEL_F32) return cudaErrorInvalidValue;
