@@ -146,3 +146,18 @@ def test_cell_numbers_fit_their_32_bits(exe, n, vt):
         at = [b[k] + int(kfl[k] / (s if k < 2 else 1.0) - 2.0 ** 23) for k in range(3)]  # of position 0: cell 1
         got = (at[1] * sy * unit + at[0] * sx * unit + at[2] * unit) % 2 ** 32
         assert got == (sy + sx + 1) * unit % 2 ** 32
+
+
+@pytest.mark.parametrize("n", [(512, 512, 300), (256, 256, 256), (512, 512, 4), (4, 512, 512), (33, 40, 55), (20000, 20000, 4),
+                               (440000000, 2, 2), (2, 2, 536870911)])
+@pytest.mark.parametrize("vt", [F32, F16, BF16])
+def test_the_servers_budget_counts_the_copy(exe, n, vt):
+    from types import SimpleNamespace
+
+    from xreg_gb300.regi import Registration, RegiLevel, cell_copy_bytes
+    numbered, _, nbytes, _, _ = _numbering(exe, n, vt)
+    assert cell_copy_bytes(n, vt) == nbytes
+    job = Registration.__new__(Registration)
+    job.vol, job.voxel_type = SimpleNamespace(size=n), vt
+    job.levels = [RegiLevel([_camera()], [np.zeros((21, 19), np.float32)])]
+    assert job.footprint_bytes() >= n[0] * n[1] * n[2] * (4 if vt == F32 else 2) + nbytes

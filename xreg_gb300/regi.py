@@ -42,6 +42,20 @@ METRICS = {
 DEFAULT_SIGMA = np.array([np.radians(10.0)] * 3 + [20.0] * 3)
 
 
+def cell_copy_bytes(size, voxel_type: int) -> int:
+    """Device bytes of a volume's cell copy (cell_layout_bytes, csrc/xr_cells.h): bordered
+    cells of 32 bytes (float32) or 16, long strides padded to 2 modulo 8; none where
+    their number does not fit 32 bits."""
+    def pad(n):
+        return n if n < 56 else n + (2 - n) % 8
+
+    nx, ny, nz = size
+    slab = pad(pad(nz + 1) * (nx + 1))
+    if slab > 0x7FFFFFFF or slab * (ny + 1) >= 2 ** 32:
+        return 0
+    return slab * (ny + 1) * (32 if voxel_type == 0 else 16)
+
+
 @dataclass
 class RegiLevel:
     cams: list                      # CameraModel per view
@@ -119,8 +133,7 @@ class Registration:
     def footprint_bytes(self) -> int:
         """Device memory the job holds while active (volume copies + the largest level's buffers)."""
         nx, ny, nz = self.vol.size
-        bvox = 4 if self.voxel_type == 0 else 2
-        vol = nx * ny * nz * bvox + (nx - 1) * (ny - 1) * (nz - 1) * bvox * 8
+        vol = nx * ny * nz * (4 if self.voxel_type == 0 else 2) + cell_copy_bytes((nx, ny, nz), self.voxel_type)
         lev = 0
         for L in self.levels:
             r, c = L.cams[0].num_det_rows, L.cams[0].num_det_cols
