@@ -175,11 +175,17 @@ __global__ void widen_kernel(const float* __restrict__ in, int64_t n, double* __
     out[i] = (double)in[i];
 }
 
-// Cubic B-spline prefilter of a line of `len` samples, `stride` apart, in place.
-// z = the pole, gain = (1 - z)(1 - 1/z), horizon = terms of the causal start.
+// Cubic B-spline prefilter of a line of `len` samples, `stride` apart, into v (from
+// src, where given, else in place).  z = the pole, gain = (1 - z)(1 - 1/z), horizon =
+// terms of the causal start.
 __device__ void bspline_prefilter_line(double* __restrict__ v, int len, int64_t stride, double z, double gain,
-                                       int horizon) {
-  for (int n = 0; n < len; ++n) v[n * stride] = __dmul_rn(v[n * stride], gain);
+                                       int horizon, const float* __restrict__ src = nullptr) {
+  if (src) {
+#pragma unroll 8
+    for (int n = 0; n < len; ++n) v[n * stride] = __dmul_rn((double)__ldg(src + n * stride), gain);
+  } else {
+    for (int n = 0; n < len; ++n) v[n * stride] = __dmul_rn(v[n * stride], gain);
+  }
   // causal initialisation (mirror boundaries)
   {
     double zn = z, sum;
@@ -269,21 +275,33 @@ __global__ void bspline_resample_kernel(const double* __restrict__ coef, int row
                    (int64_t)gridDim.x * blockDim.x, out);
 }
 
-// The whole spline in double by one block, for an image with values that
-// float-float does not carry (*beyond); otherwise it returns at once.
-__global__ void __launch_bounds__(1024) spline_double_kernel(const float* __restrict__ img, int rows, int cols,
-                                                             double factor, int orows, int ocols, double z,
-                                                             double gain, int horizon, const int* __restrict__ beyond,
-                                                             double* __restrict__ coef, float* __restrict__ out) {
+// What spline_kernel does in double for an image with values that float-float does
+// not carry (*beyond): its first pass widens and prefilters the rows, its second the
+// columns, one thread a line over all blocks, and spline_double_kernel interpolates.
+struct SplineDouble {
+  const float* img;
+  int rows, cols;
+  double* coef;
+};
+
+__device__ __noinline__ void spline_lines_double(const SplineDouble& d, bool columns, double z, double gain,
+                                                 int horizon) {
+  const int threads = gridDim.x * gridDim.y * blockDim.x;
+  const int first = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+  if (columns) {
+    for (int c = first; c < d.cols; c += threads)
+      bspline_prefilter_line(d.coef + c, d.rows, d.cols, z, gain, horizon);
+    return;
+  }
+  for (int r = first; r < d.rows; r += threads)
+    bspline_prefilter_line(d.coef + (int64_t)r * d.cols, d.cols, 1, z, gain, horizon, d.img + (int64_t)r * d.cols);
+}
+
+__global__ void spline_double_kernel(const double* __restrict__ coef, int rows, int cols, double factor, int orows,
+                                     int ocols, const int* __restrict__ beyond, float* __restrict__ out) {
   if (!*beyond) return;
-  for (int64_t i = threadIdx.x; i < (int64_t)rows * cols; i += blockDim.x) coef[i] = (double)img[i];
-  __syncthreads();
-  for (int r = threadIdx.x; r < rows; r += blockDim.x)
-    bspline_prefilter_line(coef + (int64_t)r * cols, cols, 1, z, gain, horizon);
-  __syncthreads();
-  for (int c = threadIdx.x; c < cols; c += blockDim.x) bspline_prefilter_line(coef + c, rows, cols, z, gain, horizon);
-  __syncthreads();
-  bspline_resample(coef, rows, cols, factor, orows, ocols, threadIdx.x, blockDim.x, out);
+  bspline_resample(coef, rows, cols, factor, orows, ocols, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                   (int64_t)gridDim.x * blockDim.x, out);
 }
 
 // The spline along one axis, prefilter and interpolation together, in float-float:
@@ -303,12 +321,17 @@ constexpr int kOuts = kChunk + 8;              // candidate outputs of a chunk (
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(32) spline_kernel(const TIn* __restrict__ in, int lines, int len, double factor,
                                                     int outs, double z_d, double gain_d, int horizon,
-                                                    const int* __restrict__ beyond, TOut* __restrict__ out) {
+                                                    const int* __restrict__ beyond, const SplineDouble dbl,
+                                                    TOut* __restrict__ out) {
   __shared__ float hi[kSpan][33], lo[kSpan][33];
   __shared__ FF w[kOuts][4];
   __shared__ int first[kOuts];  // index of an output's second coefficient, -1: outside the image
-  if (*beyond) return;
+  if (*beyond) {
+    spline_lines_double(dbl, sizeof(TOut) == sizeof(float), z_d, gain_d, horizon);
+    return;
+  }
   const int lane = threadIdx.x, l0 = blockIdx.y * 32;
+  if (l0 >= lines) return;  // a block for the double columns alone
   const int start = blockIdx.x * kChunk;  // this chunk's outputs have floor(position) in [start, start + kChunk)
   const int k0 = max(start - 1 - kWarm, 0), k1 = min(start + kChunk + 2 + kWarm, len);
   for (int k = k0 + lane; k < k1; k += 32) {
@@ -533,12 +556,16 @@ extern "C" XR_API xr_status xr_downsample_image(const float* d_src, int64_t rows
     auto grid = [](int64_t len, int64_t lines) {
       return dim3((unsigned)((len + kChunk - 1) / kChunk), (unsigned)((lines + 31) / 32));
     };
+    // an image with values beyond float-float: the coefficients lie where x_out does
+    const SplineDouble dbl{smooth, (int)rows, (int)cols, a};
     spline_kernel<float, float2><<<grid(cols, rows), 32, 0, s>>>(smooth, (int)rows, (int)cols, factor, (int)ocols, p.z,
-                                                                 p.gain, p.horizon, beyond, x_out);
-    spline_kernel<float2, float><<<grid(rows, ocols), 32, 0, s>>>(x_out, (int)ocols, (int)rows, factor, (int)orows, p.z,
-                                                                  p.gain, p.horizon, beyond, d_dst);
-    spline_double_kernel<<<1, 1024, 0, s>>>(smooth, (int)rows, (int)cols, factor, (int)orows, (int)ocols, p.z, p.gain,
-                                            p.horizon, beyond, a, d_dst);
+                                                                 p.gain, p.horizon, beyond, dbl, x_out);
+    dim3 columns = grid(rows, ocols);  // a thread for each column in the double case
+    columns.y = std::max(columns.y, (unsigned)((cols + 32 * columns.x - 1) / (32 * columns.x)));
+    spline_kernel<float2, float><<<columns, 32, 0, s>>>(x_out, (int)ocols, (int)rows, factor, (int)orows, p.z, p.gain,
+                                                        p.horizon, beyond, dbl, d_dst);
+    spline_double_kernel<<<std::min<unsigned>(grid_for(orows * ocols), 256), 256, 0, s>>>(
+        a, (int)rows, (int)cols, factor, (int)orows, (int)ocols, beyond, d_dst);
     XR_CUDA_TRY(cudaGetLastError());
     return XR_OK;
   }
