@@ -266,14 +266,15 @@ XF_HD bool ray_setup(const RayFrame& g, float col, float row, const float maxb[3
 }
 
 // Whether samples first..last of a ray, at start + k step, lie within [0, maxb]
-// widened by `margin` on every axis.  Every comparison is one that a NaN fails.
+// widened by `margin` on every axis, as distances from its middle (two instructions
+// an end and axis).  Every comparison is one that a NaN fails.
 XF_HD bool samples_within(const float start[3], const float stepv[3], uint32_t first, uint32_t last,
                           const float maxb[3], float margin) {
+  const float f = (float)first, l = (float)last;
   bool in = true;
   for (int k = 0; k < 3; ++k) {
-    const float a = add(start[k], mul((float)first, stepv[k])), b = add(start[k], mul((float)last, stepv[k]));
-    const float hi = add(maxb[k], margin);
-    in = in && a >= -margin && a <= hi && b >= -margin && b <= hi;
+    const float mid = 0.5f * maxb[k], reach = mid + margin, q = start[k] - mid;
+    in = in && fabsf(q + f * stepv[k]) <= reach && fabsf(q + l * stepv[k]) <= reach;
   }
   return in;
 }
