@@ -66,7 +66,7 @@ def _args():
     p.add_argument("--serving-rates", default=",".join(str(r) for r in SERVING_RATES),
                    help="Poisson arrival rates (per second) of the serving measurement")
     p.add_argument("--launch-config", default="auto",
-                   help="DRR kernel configuration 'layout,block_warps_x,unroll[,warp_rows]' (layout 0 linear, "
+                   help="DRR kernel configuration 'layout,block_warps_x,loop[,warp_rows]' (layout 0 linear, "
                         "1 cell8, 2 cell8 256-bit; warp_rows 4 = 8x4-pixel warps, 8 = 4x8) instead of the "
                         "autotuner's choice")
     return p.parse_args()

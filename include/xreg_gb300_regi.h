@@ -161,7 +161,7 @@ XR_API xr_status xr_log_remap(const float* d_src, int64_t rows, int64_t cols, in
 /* Job set: evaluates one population for each of several registrations (each an
  * xr_objective with its own volume, cameras, fixed images and population size)
  * with ONE DRR launch over all their (tile, projection) work items (each job
- * in its autotuned block shape and sample loop), followed by one batched
+ * in its autotuned block shape), followed by one batched
  * grad-NCC launch over every job's images.  This is the multi-job batching of many
  * concurrent Intensity2D3DRegiCMAES runs (each calls obj_fn per iteration,
  * xregIntensity2D3DRegi.cpp:571-742); xReg itself has no counterpart and runs

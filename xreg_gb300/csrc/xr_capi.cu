@@ -860,8 +860,8 @@ extern "C" XR_API xr_status xr_rc_set_count_samples(xr_raycaster rc, int32_t ena
 }
 
 // ------------------------------------------------------------- autotuner
-// Candidates differ only in speed (layout, block shape, unroll give bit-identical
-// results), so the fastest measured one is cached per shape for the process.
+// Block shapes differ only in speed (they give bit-identical results), so the
+// fastest measured one is cached per shape for the process.
 namespace {
 struct TuneKey {
   int64_t nx, ny, nz, rows, cols, projs_pow2;
@@ -2286,9 +2286,7 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
       else cu.push_back(CmaUpdateJob{cma[i].state, obj->d_sims.as<float>(), d_report + i});
     }
     fj.push_back(J);
-    // one launch per (voxel type, layout, pose-grouped or not): the DRR job kernel
-    // runs each job's loop, the fused kernel the group's first job's (every loop
-    // gives the same bits)
+    // one launch per (voxel type, layout, pose-grouped or not)
     key.push_back((vol.type * 4 + J.d.p.vol.layout) * 2 + (J.d.pose_group ? 1 : 0));
   }
   // jobs ordered by group; item numbering restarts in each group

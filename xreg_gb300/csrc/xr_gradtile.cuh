@@ -61,7 +61,7 @@ __device__ __forceinline__ FF ff_shfl_down(FF v, int o) {
 }
 
 // Blur and Sobel arithmetic with every rounding explicit (no contraction), so
-// the shared-memory and the register forms of the tile give the same bits.
+// every kernel that forms gradients gives the same bits.
 __device__ __forceinline__ float blur5(float a, float b, float c, float d, float e) {
   return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(0.0625f, a), __fmul_rn(0.25f, b)), __fmul_rn(0.375f, c)),
                              __fmul_rn(0.25f, d)),

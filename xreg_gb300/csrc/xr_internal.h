@@ -153,8 +153,8 @@ struct FusedView {
   double* partials;       // [pop][metric tiles][6]
   float* sims;            // [pop]
 };
-// A job of a fused evaluation launch: its DRR work items (16x16-pixel tiles,
-// projection fastest), and when `metric` is 1 the grad-NCC of every image
+// A job of a fused evaluation launch: its DRR work items (tiles of
+// its block shape, projection fastest), and when `metric` is 1 the grad-NCC of every image
 // computed tile by tile as soon as the DRR pixels a 64x52-pixel metric tile reads are
 // written, then each image's value, then each pose's mean over views.
 // Counters live in `cnt` (zero between launches; the block that completes a

@@ -13,10 +13,11 @@
 // reflect-extended input, which equals the reflect-extended blurred image because
 // the kernels are symmetric.
 //
-// Patch NCC (xregImgSimMetric2DPatchNCCCPU.cpp:205-287,558-619): one thread per
-// patch centre, two-pass mean / sample std dev over the (2r+1)^2 window from a
-// shared-memory tile, score 1 - sum((m - mu_m)/sd_m * fhat), unit weights, mean
-// over patches.  The fixed side (per-patch mean and 1/(sd n)) is pre-computed once.
+// Patch NCC (xregImgSimMetric2DPatchNCCCPU.cpp:205-287,558-619): a thread scores
+// one or four patches of a column, two-pass mean / sample std dev over the (2r+1)^2
+// window from a shared-memory tile, score 1 - sum((m - mu_m)/sd_m * fhat), mean over
+// patches, weighted where asked.  The fixed side (per-patch mean and 1/(sd n)) is
+// pre-computed once.
 #include "xr_cmaes_core.h"
 #include "xr_gradtile.cuh"
 
@@ -709,7 +710,7 @@ __global__ void __launch_bounds__(kThreads) patch_ncc_kernel(const float* __rest
 // x 11, both gradients: 1175 us one channel at a time, now 632; 24 plain images of 384^2:
 // 180 us, now 98; 8 images of 187 x 118 at stride 3, a whole call: 55 us, now 47.
 // Every RB takes the same operations in the same order, patch by patch and up to the
-// partial sums (one for 16 rows of patches), so an image's value does not depend on
+// partial sums (one for 8 rows of patches), so an image's value does not depend on
 // how many others share the launch.
 // Pixel x of a row lies at (x mod stride) Wp + x / stride, so that the lanes of a
 // read (one patch column each) are neighbours for every stride.

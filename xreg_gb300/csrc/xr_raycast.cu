@@ -1043,7 +1043,7 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
 // Fused evaluation: a persistent multi-job DRR loop (every block takes the
 // next (job, tile, projection) item from a global counter; projections are
 // the fastest index within a job), with each job's grad-NCC (5x5 smoothing) computed inside the same launch.
-// No block ever waits for another.  After a block writes a 16x16 DRR tile it
+// No block ever waits for another.  After a block writes a DRR tile it
 // counts the tile towards every 64x52 metric tile whose input (the tile with
 // its 3-pixel blur + Sobel halo, clipped to the image) the tile overlaps; the
 // block whose count completes a metric tile computes that tile's moments at
