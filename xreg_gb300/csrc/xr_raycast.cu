@@ -329,6 +329,14 @@ struct CellData {
   }
 };
 
+// How a kernel blends a volume's corners: the cells' kernels know it (their volume is
+// weighted or not), the others ask the volume.
+enum class Blend { kDifferences, kWeights, kVolume };
+template <int VT, Blend BLEND>
+__device__ __forceinline__ bool by_weights(const VolView& vol) {
+  return VT != XR_VOXEL_F16 && (BLEND == Blend::kWeights || (BLEND == Blend::kVolume && vol.weighted));
+}
+
 // Trilinear sample at index position (px, py, pz) with ITK's boundary rule:
 // positions past a face take the face's values.  The cell is floor(position)
 // clamped to [-1, n-1], the fraction saturated to [0, 1] (a NaN position reads
@@ -336,11 +344,12 @@ struct CellData {
 // position lies in [0, n-1) on every axis, where no clamp changes anything.  A
 // weighted volume's cells end at n-2 (fraction 1 on the last voxel), without the
 // border's: there a corner of weight 0 decides whether an infinity makes a NaN.
-template <int VT, int LAYOUT, bool INSIDE = false>
+template <int VT, int LAYOUT, bool INSIDE, Blend BLEND>
 __device__ __forceinline__ float sample(const VolView& vol, const void* data, float px, float py, float pz) {
+  const bool weighted = by_weights<VT, BLEND>(vol);
   int ix = __float2int_rd(px), iy = __float2int_rd(py), iz = __float2int_rd(pz);
   if (!INSIDE) {
-    const int b = VT != XR_VOXEL_F16 && vol.weighted ? 1 : 0;
+    const int b = weighted ? 1 : 0;
     ix = clampi(ix, b - 1, vol.nx - 1 - b);
     iy = clampi(iy, b - 1, vol.ny - 1 - b);
     iz = clampi(iz, b - 1, vol.nz - 1 - b);
@@ -379,15 +388,15 @@ __device__ __forceinline__ float sample(const VolView& vol, const void* data, fl
       v[5] = Vox<VT>::ld(data, b + sz + sy);
       v[6] = Vox<VT>::ld(data, b + sy + sx);
       v[7] = Vox<VT>::ld(data, b + sz + sy + sx);
-      return vol.weighted ? interp8_weighted(v, fx, fy, fz) : interp8<false>(v, fx, fy, fz);
+      return weighted ? interp8_weighted(v, fx, fy, fz) : interp8<false>(v, fx, fy, fz);
     }
   } else {
     const unsigned int c = (unsigned int)(ix + 1) * (unsigned int)vol.cs[0] +
                            (unsigned int)(iy + 1) * (unsigned int)vol.cs[1] + (unsigned int)(iz + 1);
     CellData<VT, LAYOUT> q;
     q.load(data, c);
-    if constexpr (VT != XR_VOXEL_F16)
-      if (vol.weighted) return q.weighted_value(Frac3{fx, fy, fz});
+    if constexpr (VT != XR_VOXEL_F16 && BLEND != Blend::kDifferences)
+      if (weighted) return q.weighted_value(Frac3{fx, fy, fz});
     constexpr float kS = VT == XR_VOXEL_F16 ? kH16 : 1.0f;
     return q.value(Frac3{fx * kS, fy * kS, fz});
   }
@@ -579,18 +588,20 @@ __device__ __forceinline__ float march_cells(const VolView& vol, float px, float
 
 // The same through sample(): the LINEAR layout, and rays that march_cells does
 // not take.
-template <int VT, int KERNEL, int LAYOUT, bool INSIDE>
+template <int VT, int KERNEL, int LAYOUT, bool INSIDE, Blend BLEND>
 __device__ __forceinline__ float march_samples(const VolView& vol, const void* data, float px, float py, float pz,
                                                float sx, float sy, float sz, unsigned int n, float sum) {
-  for (; n >= 2; n -= 2) {
-    const float v0 = sample<VT, LAYOUT, INSIDE>(vol, data, px, py, pz);
-    px = __fadd_rn(px, sx); py = __fadd_rn(py, sy); pz = __fadd_rn(pz, sz);
-    const float v1 = sample<VT, LAYOUT, INSIDE>(vol, data, px, py, pz);
-    px = __fadd_rn(px, sx); py = __fadd_rn(py, sy); pz = __fadd_rn(pz, sz);
-    sum = fold<KERNEL>(fold<KERNEL>(sum, v0), v1);
+  if (LAYOUT == XR_LAYOUT_LINEAR || BLEND != Blend::kDifferences) {
+    for (; n >= 2; n -= 2) {
+      const float v0 = sample<VT, LAYOUT, INSIDE, BLEND>(vol, data, px, py, pz);
+      px = __fadd_rn(px, sx); py = __fadd_rn(py, sy); pz = __fadd_rn(pz, sz);
+      const float v1 = sample<VT, LAYOUT, INSIDE, BLEND>(vol, data, px, py, pz);
+      px = __fadd_rn(px, sx); py = __fadd_rn(py, sy); pz = __fadd_rn(pz, sz);
+      sum = fold<KERNEL>(fold<KERNEL>(sum, v0), v1);
+    }
   }
   for (; n > 0; --n) {
-    const float v0 = sample<VT, LAYOUT, INSIDE>(vol, data, px, py, pz);
+    const float v0 = sample<VT, LAYOUT, INSIDE, BLEND>(vol, data, px, py, pz);
     px = __fadd_rn(px, sx); py = __fadd_rn(py, sy); pz = __fadd_rn(pz, sz);
     sum = fold<KERNEL>(sum, v0);
   }
@@ -601,7 +612,7 @@ __device__ __forceinline__ float march_samples(const VolView& vol, const void* d
 // (the caller checks that the pixel exists).  Returns the number of samples of
 // the reference step rule; *loaded receives how many of them were loaded (the
 // others were proven zero and skipped).
-template <int VT, int KERNEL, int LAYOUT, bool DEEP = false, bool WEIGHTED = false>
+template <int VT, int KERNEL, int LAYOUT, bool DEEP = false, Blend BLEND = Blend::kVolume>
 __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, const int64_t proj, const int row,
                                                           const int col, unsigned int* loaded) {
   float sum = (KERNEL == XR_LINE_INT_MAX) ? -FLT_MAX : 0.0f;
@@ -700,9 +711,9 @@ __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, co
       // millions of voxels away rounds off the volume: those take the clamped
       // sampler.  On the LINEAR layout, and of weighted volumes, rays a quarter voxel
       // inside run without clamps.
-      constexpr bool kInside = LAYOUT == XR_LAYOUT_LINEAR || WEIGHTED;
-      bool unclamped =
-          drift_ok && (LAYOUT == XR_LAYOUT_LINEAR || (p.vol.kfl[0] > 0.0f && (WEIGHTED || !p.vol.weighted)));
+      constexpr bool kWeights = BLEND == Blend::kWeights, kInside = LAYOUT == XR_LAYOUT_LINEAR || kWeights;
+      bool unclamped = drift_ok && (LAYOUT == XR_LAYOUT_LINEAR ||
+                                    (p.vol.kfl[0] > 0.0f && (kWeights || !by_weights<VT, BLEND>(p.vol))));
       if (unclamped) unclamped = xf::samples_within(st0, stv, first, last, maxb, kInside ? -0.25f : 0.75f);
       if (hit) {
         // advance to sample `first` (four additions per trip: the skipped samples
@@ -728,13 +739,13 @@ __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, co
         *loaded = n;
         if (unclamped) {
           if constexpr (LAYOUT == XR_LAYOUT_LINEAR)
-            sum = march_samples<VT, KERNEL, LAYOUT, true>(p.vol, data, px, py, pz, sx, sy, sz, n, sum);
+            sum = march_samples<VT, KERNEL, LAYOUT, true, BLEND>(p.vol, data, px, py, pz, sx, sy, sz, n, sum);
           else
             sum = p.vol.cell_bytes
-                      ? march_cells<VT, KERNEL, LAYOUT, true, DEEP, WEIGHTED>(p.vol, px, py, pz, sx, sy, sz, n, sum)
-                      : march_cells<VT, KERNEL, LAYOUT, false, DEEP, WEIGHTED>(p.vol, px, py, pz, sx, sy, sz, n, sum);
+                      ? march_cells<VT, KERNEL, LAYOUT, true, DEEP, kWeights>(p.vol, px, py, pz, sx, sy, sz, n, sum)
+                      : march_cells<VT, KERNEL, LAYOUT, false, DEEP, kWeights>(p.vol, px, py, pz, sx, sy, sz, n, sum);
         } else {
-          sum = march_samples<VT, KERNEL, LAYOUT, false>(p.vol, data, px, py, pz, sx, sy, sz, n, sum);
+          sum = march_samples<VT, KERNEL, LAYOUT, false, BLEND>(p.vol, data, px, py, pz, sx, sy, sz, n, sum);
         }
         sum = __fmul_rn(sum, p.step);
         if (VT != XR_VOXEL_F32) sum = __fmul_rn(sum, p.vol.inv_scale);
@@ -762,7 +773,7 @@ __device__ __forceinline__ void lane_pixel(int lane, int wl, int& col, int& row)
   row = ((lane >> 1) & 1) + ((lane >> (wl + 1)) << 1);
 }
 
-template <int VT, int KERNEL, int LAYOUT, bool DEEP, bool WEIGHTED>
+template <int VT, int KERNEL, int LAYOUT, bool DEEP, Blend BLEND>
 __global__ void __launch_bounds__(32 * kMaxWarps, (DEEP ? kDeepBlocksPerSM : kMinBlocksPerSM * 8 / kWarps) * kWarps / kMaxWarps)
 drr_kernel(const DrrParams p, const int64_t proj_base) {
   // Each warp covers an 8 x 4 (or, tall, 4 x 8) patch of pixels so its 32 rays
@@ -780,7 +791,7 @@ drr_kernel(const DrrParams p, const int64_t proj_base) {
   const int64_t proj = proj_base + blockIdx.x;
   unsigned long long ns = 0;
   unsigned int nl = 0;
-  if (col < p.cols && row < p.rows) ns = trace_pixel<VT, KERNEL, LAYOUT, DEEP, WEIGHTED>(p, proj, row, col, &nl);
+  if (col < p.cols && row < p.rows) ns = trace_pixel<VT, KERNEL, LAYOUT, DEEP, BLEND>(p, proj, row, col, &nl);
   if (p.sample_counter) {
     unsigned long long nlw = nl;
     for (int o = 16; o > 0; o >>= 1) {
@@ -1351,7 +1362,7 @@ cudaError_t launch_jobs_t(const MultiJobDrr* d_jobs, int njobs, long long total,
                  : launch_jobs_g<VT, LAYOUT, false>(d_jobs, njobs, total, s);
 }
 
-template <int VT, int KERNEL, int LAYOUT, bool DEEP, bool WEIGHTED = false>
+template <int VT, int KERNEL, int LAYOUT, bool DEEP, Blend BLEND>
 cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
   // The kernel uses no shared memory: ask for the largest L1 (the gathers hit
   // it), once per device (a preference; setting it twice is harmless).
@@ -1359,7 +1370,7 @@ cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
       !carveout_set[dev].load(std::memory_order_relaxed)) {
-    cudaFuncSetAttribute(drr_kernel<VT, KERNEL, LAYOUT, DEEP, WEIGHTED>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(drr_kernel<VT, KERNEL, LAYOUT, DEEP, BLEND>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxL1);
     carveout_set[dev].store(true, std::memory_order_relaxed);
   }
@@ -1370,7 +1381,7 @@ cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
   for (int64_t base = 0; base < p.num_projs; base += max_x) {
     const int64_t n = (p.num_projs - base) < max_x ? (p.num_projs - base) : max_x;
     const dim3 grid((unsigned)n, (p.cols + tx - 1) / tx, (p.rows + ty - 1) / ty);
-    drr_kernel<VT, KERNEL, LAYOUT, DEEP, WEIGHTED><<<grid, 32 * bw * p.block_warps_y, 0, s>>>(p, base);
+    drr_kernel<VT, KERNEL, LAYOUT, DEEP, BLEND><<<grid, 32 * bw * p.block_warps_y, 0, s>>>(p, base);
   }
   return cudaGetLastError();
 }
@@ -1385,11 +1396,13 @@ cudaError_t launch_depth(const DrrParams& p, cudaStream_t s) {
 // (156,000 rays) 97 / 98; FP16, two views of 384^2 (294,912 rays) 148 / 150.
 template <int VT, int KERNEL, int LAYOUT>
 cudaError_t launch_t(const DrrParams& p, cudaStream_t s) {
-  if constexpr (LAYOUT != XR_LAYOUT_LINEAR) {
+  if constexpr (LAYOUT == XR_LAYOUT_LINEAR) {
+    return launch_depth<VT, KERNEL, LAYOUT, false, Blend::kVolume>(p, s);
+  } else {
     // Volumes with an infinity have a march of their own, four by weights (20 images
     // of 256^2 of a 256 x 256 x 200 float32 volume: 616 us through the clamped sampler).
     if constexpr (VT != XR_VOXEL_F16)
-      if (p.vol.weighted) return launch_depth<VT, KERNEL, LAYOUT, false, true>(p, s);
+      if (p.vol.weighted) return launch_depth<VT, KERNEL, LAYOUT, false, Blend::kWeights>(p, s);
     static std::atomic<int> cached[kMaxDevices];  // SMs per device; zero = not known yet
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
@@ -1398,9 +1411,9 @@ cudaError_t launch_t(const DrrParams& p, cudaStream_t s) {
         cached[dev].store(sms, std::memory_order_relaxed);
     }
     if (p.num_projs * p.rows * p.cols <= 2 * (int64_t)sms * kDeepBlocksPerSM * 32 * kWarps)
-      return launch_depth<VT, KERNEL, LAYOUT, true>(p, s);
+      return launch_depth<VT, KERNEL, LAYOUT, true, Blend::kDifferences>(p, s);
+    return launch_depth<VT, KERNEL, LAYOUT, false, Blend::kDifferences>(p, s);
   }
-  return launch_depth<VT, KERNEL, LAYOUT, false>(p, s);
 }
 
 template <int VT, int KERNEL>
