@@ -818,30 +818,33 @@ constexpr int kBrickCells = 1400;  // 43.75 KB of 32-byte cells
 constexpr int kBrickDepth = 16;    // cells per slab along the dominant axis
 
 // Cell (numbered from 0: floor + 1) and fractions of a position, clamped as sample() does.
+template <Blend BLEND>
 __device__ __forceinline__ void cell3(const VolView& vol, const float pos[3], int c[3], float f[3]) {
   const int n[3] = {vol.nx, vol.ny, vol.nz};
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const int b = vol.weighted ? 1 : 0;
+    const int b = BLEND == Blend::kWeights ? 1 : 0;
     const int i = clampi(__float2int_rd(pos[a]), b - 1, n[a] - 1 - b);
     f[a] = __saturatef(pos[a] - (float)i);
     c[a] = i + 1;
   }
 }
 
-__device__ __forceinline__ float brick_value(const VolView& vol, const float v[8], const float f[3]) {
-  return vol.weighted ? interp8_weighted(v, f[0], f[1], f[2]) : interp8<true>(v, f[0], f[1], f[2]);
+template <Blend BLEND>
+__device__ __forceinline__ float brick_value(const float v[8], const float f[3]) {
+  return BLEND == Blend::kWeights ? interp8_weighted(v, f[0], f[1], f[2]) : interp8<true>(v, f[0], f[1], f[2]);
 }
 
 // The ray's remaining samples k..last from global memory, in order.
+template <Blend BLEND>
 __device__ __forceinline__ float brick_march_global(const VolView& vol, float pos[3], const float st[3],
                                                     unsigned int& k, unsigned int last, float sum) {
   for (; k <= last; ++k) {
     int c[3];
     float f[3], v[8];
-    cell3(vol, pos, c, f);
+    cell3<BLEND>(vol, pos, c, f);
     Vox<XR_VOXEL_F32>::cell_wide(vol.cells, (unsigned int)c[0] * vol.cs[0] + (unsigned int)c[1] * vol.cs[1] + (unsigned int)c[2], v);
-    sum = __fadd_rn(sum, brick_value(vol, v, f));
+    sum = __fadd_rn(sum, brick_value<BLEND>(v, f));
     pos[0] = __fadd_rn(pos[0], st[0]);
     pos[1] = __fadd_rn(pos[1], st[1]);
     pos[2] = __fadd_rn(pos[2], st[2]);
@@ -849,6 +852,7 @@ __device__ __forceinline__ float brick_march_global(const VolView& vol, float po
   return sum;
 }
 
+template <Blend BLEND>
 __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams p, const int64_t proj_base) {
   __shared__ float4 s_cells[2 * kBrickCells];
   __shared__ int s_code, s_amin, s_amax, s_lo[3], s_hi[3];
@@ -930,14 +934,14 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
   __syncthreads();
   const int bcode = s_code, ax = bcode >> 1, dir = (bcode & 1) ? 1 : -1;
   const bool staged = k <= last && bcode >= 0 && code == bcode;
-  if (k <= last && !staged) sum = brick_march_global(vol, pos, st, k, last, sum);  // another axis: global reads
+  if (k <= last && !staged) sum = brick_march_global<BLEND>(vol, pos, st, k, last, sum);  // another axis: global reads
   if (staged) {  // the cells of this ray's first and (about) last samples along the axis
     int c0[3], c1[3];
     float f[3];
-    cell3(vol, pos, c0, f);
+    cell3<BLEND>(vol, pos, c0, f);
     const float e = (float)(last - k);
     const float pe[3] = {pos[0] + e * st[0], pos[1] + e * st[1], pos[2] + e * st[2]};
-    cell3(vol, pe, c1, f);
+    cell3<BLEND>(vol, pe, c1, f);
     atomicMin(&s_amin, min(c0[ax], c1[ax]) - 1);
     atomicMax(&s_amax, max(c0[ax], c1[ax]) + 1);
   }
@@ -955,11 +959,11 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
       if (staged && k <= last) {
         int ce[3], cx[3];
         float f[3];
-        cell3(vol, pos, ce, f);
+        cell3<BLEND>(vol, pos, ce, f);
         float m = ((float)zfar - pos[ax]) / st[ax];  // samples to the slab's far side, about
         m = fminf(fmaxf(m, 0.0f), (float)(last - k));
         const float pe[3] = {pos[0] + m * st[0], pos[1] + m * st[1], pos[2] + m * st[2]};
-        cell3(vol, pe, cx, f);
+        cell3<BLEND>(vol, pe, cx, f);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           if (a == ax) continue;
@@ -1004,7 +1008,7 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
         for (; k <= last; ++k) {
           int c[3];
           float f[3], v[8];
-          cell3(vol, pos, c, f);
+          cell3<BLEND>(vol, pos, c, f);
           if (dir > 0 ? c[ax] >= zend : c[ax] <= zend) break;
           const bool in = use && c[0] >= lo[0] && c[0] <= hi[0] && c[1] >= lo[1] && c[1] <= hi[1] && c[2] >= lo[2] &&
                           c[2] <= hi[2];
@@ -1016,7 +1020,7 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
           } else {
             Vox<XR_VOXEL_F32>::cell_wide(vol.cells, (unsigned int)c[0] * vol.cs[0] + (unsigned int)c[1] * vol.cs[1] + (unsigned int)c[2], v);
           }
-          sum = __fadd_rn(sum, brick_value(vol, v, f));
+          sum = __fadd_rn(sum, brick_value<BLEND>(v, f));
           pos[0] = __fadd_rn(pos[0], st[0]);
           pos[1] = __fadd_rn(pos[1], st[1]);
           pos[2] = __fadd_rn(pos[2], st[2]);
@@ -1026,7 +1030,7 @@ __global__ void __launch_bounds__(kThreads, 4) drr_brick_kernel(const DrrParams 
       z = zend;
     }
   }
-  if (k <= last) sum = brick_march_global(vol, pos, st, k, last, sum);  // past the estimated range
+  if (k <= last) sum = brick_march_global<BLEND>(vol, pos, st, k, last, sum);  // past the estimated range
   if (pixel) {
     sum = __fmul_rn(sum, p.step);
     const float aa = __fadd_rn(0.0f, sum);
@@ -1434,23 +1438,28 @@ cudaError_t launch_kernel_id(const DrrParams& p, cudaStream_t s) {
 
 }  // namespace
 
-cudaError_t launch_brick(const DrrParams& p, cudaStream_t s) {
-  if (p.vol.voxel_type != XR_VOXEL_F32 || !p.vol.cells || p.kernel_id != XR_LINE_INT_SUM) return cudaErrorInvalidValue;
+template <Blend BLEND>
+cudaError_t launch_brick_t(const DrrParams& p, cudaStream_t s) {
   static std::atomic<bool> carveout_set[kMaxDevices];
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
       !carveout_set[dev].load(std::memory_order_relaxed)) {
     // four resident blocks of 44 KB each, the rest of the SM's unified L1 for the global reads
-    cudaFuncSetAttribute(drr_brick_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 80);
+    cudaFuncSetAttribute(drr_brick_kernel<BLEND>, cudaFuncAttributePreferredSharedMemoryCarveout, 80);
     carveout_set[dev].store(true, std::memory_order_relaxed);
   }
   const int64_t max_x = 0x7fffffff;
   for (int64_t base = 0; base < p.num_projs; base += max_x) {
     const int64_t n = (p.num_projs - base) < max_x ? (p.num_projs - base) : max_x;
     const dim3 grid((unsigned)n, (p.cols + 15) / 16, (p.rows + 15) / 16);
-    drr_brick_kernel<<<grid, kThreads, 0, s>>>(p, base);
+    drr_brick_kernel<BLEND><<<grid, kThreads, 0, s>>>(p, base);
   }
   return cudaGetLastError();
+}
+
+cudaError_t launch_brick(const DrrParams& p, cudaStream_t s) {
+  if (p.vol.voxel_type != XR_VOXEL_F32 || !p.vol.cells || p.kernel_id != XR_LINE_INT_SUM) return cudaErrorInvalidValue;
+  return p.vol.weighted ? launch_brick_t<Blend::kWeights>(p, s) : launch_brick_t<Blend::kDifferences>(p, s);
 }
 
 cudaError_t launch_drr(const DrrParams& params, cudaStream_t s) {
