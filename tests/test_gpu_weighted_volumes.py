@@ -57,3 +57,34 @@ def test_cells_of_weighted_volumes(xr, oracle, vt, value, at):
     np.testing.assert_array_equal(np.isfinite(linear), ok)
     rel, zero = drr_rel_err(np.where(ok, linear, 0.0), np.where(ok, ref, 0.0))
     assert zero == 0.0 and rel <= TOL[vt], rel
+
+
+def test_job_sets_of_weighted_and_other_volumes(xr):
+    """Job steps, fused and not, pose-grouped or not: every job's values and images are
+    those of its objective alone."""
+    rng = np.random.default_rng(11)
+    cam, jobs = small_camera((45, 37), 4.0), []
+    for vt, value in ((0, np.inf), (0, 1.0), (2, 2.0 ** 127), (2, 1.0), (1, 1.0), (0, 2.0 ** 127)):
+        v = rng.uniform(0.5, 1.0, (33, 36, 40)).astype(np.float32)
+        v[14, 20, 18] = value
+        vol = api.Volume(v, spacing=(1.5, 1.5, 1.5))
+        rc = xr.RayCasterLineIntCUDA()
+        rc.set_volume(vol, vt)
+        rc.set_camera_model(cam)
+        rc.set_ray_step_size(0.5)
+        m = xr.ImgSimMetric2DGradNCCCUDA()
+        m.set_fixed_image(rng.random((45, 37)).astype(np.float32))
+        jobs.append((rc, m, xr.PopulationObjective(rc, [m], 5), _poses(vol)))
+    alone, images = [], []
+    for rc, _, obj, poses in jobs:
+        alone.append(obj.eval(poses))
+        images.append(rc.projs())
+    assert sum(np.isnan(i).any() or np.isinf(i).any() or i.max() > 1e30 for i in images) == 3
+    for mode in ("split", "groups", "fused"):
+        js = xr.JobSet()
+        js.set_fused(mode == "fused")
+        js.set_pose_groups(2 if mode == "groups" else 0)
+        got = js.eval([j[2] for j in jobs], [j[3] for j in jobs])
+        for (rc, _, _, _), g, a, i in zip(jobs, got, alone, images):
+            np.testing.assert_array_equal(g, a)
+            np.testing.assert_array_equal(rc.projs(), i)

@@ -2286,8 +2286,8 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
       else cu.push_back(CmaUpdateJob{cma[i].state, obj->d_sims.as<float>(), d_report + i});
     }
     fj.push_back(J);
-    // one launch per (voxel type, layout, pose-grouped or not)
-    key.push_back((vol.type * 4 + J.d.p.vol.layout) * 2 + (J.d.pose_group ? 1 : 0));
+    // one launch per (voxel type, layout, blend, pose-grouped or not)
+    key.push_back((vol.type * 4 + J.d.p.vol.layout) * 4 + J.d.p.vol.weighted * 2 + (J.d.pose_group ? 1 : 0));
   }
   // jobs ordered by group; item numbering restarts in each group
   std::vector<int32_t> keys(key);
@@ -2354,12 +2354,13 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
     if (fused)
       XR_CUDA_TRY(launch_eval_fused(reinterpret_cast<const FusedJob*>(d + off_f) + ranges[gi].first,
                                     (int)(ranges[gi].second - ranges[gi].first), group_items[gi],
-                                    f0.d.p.vol.voxel_type, f0.d.p.vol.layout,
+                                    f0.d.p.vol.voxel_type, f0.d.p.vol.layout, f0.d.p.vol.weighted != 0,
                                     fw.d_counter.as<unsigned long long>(), &blocks, s));
     else {
       XR_CUDA_TRY(launch_drr_jobs(reinterpret_cast<const MultiJobDrr*>(d + off_m) + ranges[gi].first,
                                   (int)(ranges[gi].second - ranges[gi].first), group_items[gi],
-                                  f0.d.p.vol.voxel_type, f0.d.p.vol.layout, f0.d.pose_group != 0, s));
+                                  f0.d.p.vol.voxel_type, f0.d.p.vol.layout, f0.d.p.vol.weighted != 0,
+                                  f0.d.pose_group != 0, s));
       blocks = (int)std::min<long long>(group_items[gi], 0x7fffffff);
     }
     fw.items += group_items[gi];

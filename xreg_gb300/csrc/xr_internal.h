@@ -106,10 +106,10 @@ struct MultiJobDrr {
   }
 };
 // One launch whose grid covers the (tile, projection) items of jobs sharing a
-// voxel type and layout (no work counter: one block per item).
+// voxel type, layout and (VolView::weighted) blend (no work counter: one block per item).
 // grouped: every job's pose_group is 4 (otherwise every job's is 0).
 cudaError_t launch_drr_jobs(const MultiJobDrr* d_jobs, int njobs, long long total_items, int32_t voxel_type,
-                            int32_t layout, bool grouped, cudaStream_t s);
+                            int32_t layout, bool weighted, bool grouped, cudaStream_t s);
 
 // ---- launchers (xr_volume.cu) ----
 // HUToLinAtt of n values.
@@ -175,9 +175,10 @@ struct FusedJob {
   void* cma;              // CMA-ES state updated by the batched grad-NCC launch once every pose has its value
   CmaReport* report;      // where that update reports its termination code
 };
-// One persistent launch over the jobs of one (voxel type, layout) group.
+// One persistent launch over the jobs of one (voxel type, layout, blend) group.
 cudaError_t launch_eval_fused(const FusedJob* d_jobs, int njobs, long long total_items, int32_t voxel_type,
-                              int32_t layout, unsigned long long* d_counter, int* blocks_out, cudaStream_t s);
+                              int32_t layout, bool weighted, unsigned long long* d_counter, int* blocks_out,
+                              cudaStream_t s);
 // Grad-NCC (5x5 smoothing) of every image of the jobs with `metric` set, their
 // DRRs already written: one launch over all their tiles (the split
 // path's tile code), each image's FP64 combine by the block that completes its

@@ -329,8 +329,8 @@ struct CellData {
   }
 };
 
-// How a kernel blends a volume's corners: the cells' kernels know it (their volume is
-// weighted or not), the others ask the volume.
+// How a kernel blends a volume's corners: the cells' kernels know it (their volumes are
+// weighted or not), those of the LINEAR layout ask the volume.
 enum class Blend { kDifferences, kWeights, kVolume };
 template <int VT, Blend BLEND>
 __device__ __forceinline__ bool by_weights(const VolView& vol) {
@@ -395,10 +395,9 @@ __device__ __forceinline__ float sample(const VolView& vol, const void* data, fl
                            (unsigned int)(iy + 1) * (unsigned int)vol.cs[1] + (unsigned int)(iz + 1);
     CellData<VT, LAYOUT> q;
     q.load(data, c);
-    if constexpr (VT != XR_VOXEL_F16 && BLEND != Blend::kDifferences)
-      if (weighted) return q.weighted_value(Frac3{fx, fy, fz});
     constexpr float kS = VT == XR_VOXEL_F16 ? kH16 : 1.0f;
-    return q.value(Frac3{fx * kS, fy * kS, fz});
+    if constexpr (BLEND == Blend::kWeights) return q.weighted_value(Frac3{fx, fy, fz});
+    else return q.value(Frac3{fx * kS, fy * kS, fz});
   }
 }
 
@@ -612,7 +611,7 @@ __device__ __forceinline__ float march_samples(const VolView& vol, const void* d
 // (the caller checks that the pixel exists).  Returns the number of samples of
 // the reference step rule; *loaded receives how many of them were loaded (the
 // others were proven zero and skipped).
-template <int VT, int KERNEL, int LAYOUT, bool DEEP = false, Blend BLEND = Blend::kVolume>
+template <int VT, int KERNEL, int LAYOUT, bool DEEP, Blend BLEND>
 __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, const int64_t proj, const int row,
                                                           const int col, unsigned int* loaded) {
   float sum = (KERNEL == XR_LINE_INT_MAX) ? -FLT_MAX : 0.0f;
@@ -712,8 +711,7 @@ __device__ __forceinline__ unsigned long long trace_pixel(const DrrParams& p, co
       // sampler.  On the LINEAR layout, and of weighted volumes, rays a quarter voxel
       // inside run without clamps.
       constexpr bool kWeights = BLEND == Blend::kWeights, kInside = LAYOUT == XR_LAYOUT_LINEAR || kWeights;
-      bool unclamped = drift_ok && (LAYOUT == XR_LAYOUT_LINEAR ||
-                                    (p.vol.kfl[0] > 0.0f && (kWeights || !by_weights<VT, BLEND>(p.vol))));
+      bool unclamped = drift_ok && (LAYOUT == XR_LAYOUT_LINEAR || p.vol.kfl[0] > 0.0f);
       if (unclamped) unclamped = xf::samples_within(st0, stv, first, last, maxb, kInside ? -0.25f : 0.75f);
       if (hit) {
         // advance to sample `first` (four additions per trip: the skipped samples
@@ -1151,7 +1149,7 @@ __device__ __noinline__ void fused_metric_image(const FusedJob& J, int64_t proj,
 // kernel at 48 (3 views of 250 x 240 under 57 poses 4158 us, at 64 registers 2804).
 constexpr int fused_blocks(int vt) { return vt == XR_VOXEL_BF16 ? kMinBlocksPerSM - 1 : kMinBlocksPerSM; }
 
-template <int VT, int LAYOUT>
+template <int VT, int LAYOUT, Blend BLEND>
 __global__ void __launch_bounds__(kThreads, fused_blocks(VT))
 eval_fused_kernel(const FusedJob* __restrict__ jobs, int njobs, long long total, unsigned long long* counter) {
   // under 1 KB of shared memory: the SM's unified L1 stays with the DRR gathers
@@ -1184,7 +1182,7 @@ eval_fused_kernel(const FusedJob* __restrict__ jobs, int njobs, long long total,
     const int col = tx * tw + (warp % bw) * wc + lc;
     const int row = ty * th + (warp / bw) * wr + lr;
     unsigned int nl;
-    if (col < P.cols && row < P.rows) trace_pixel<VT, XR_LINE_INT_SUM, LAYOUT>(P, proj, row, col, &nl);
+    if (col < P.cols && row < P.rows) trace_pixel<VT, XR_LINE_INT_SUM, LAYOUT, false, BLEND>(P, proj, row, col, &nl);
     if (!J.metric) continue;
     __threadfence();  // this block's DRR pixels, visible device-wide before they are counted
     __syncthreads();
@@ -1214,7 +1212,7 @@ eval_fused_kernel(const FusedJob* __restrict__ jobs, int njobs, long long total,
 // GROUPED: every job's items are pose groups (MultiJobDrr::pose_group); a
 // separate instantiation, so the per-projection kernels keep their registers.
 constexpr int jobs_threads(bool grouped) { return grouped ? kThreads : 32 * kWarps; }
-template <int VT, int LAYOUT, bool GROUPED>
+template <int VT, int LAYOUT, bool GROUPED, Blend BLEND>
 __global__ void __launch_bounds__(jobs_threads(GROUPED), (kMinBlocksPerSM - 1) * kThreads / jobs_threads(GROUPED))
 drr_jobs_kernel(const MultiJobDrr* __restrict__ jobs, int njobs, long long item0) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1304,12 +1302,12 @@ drr_jobs_kernel(const MultiJobDrr* __restrict__ jobs, int njobs, long long item0
   }
   if (col >= J.p.cols || row >= J.p.rows) return;
   unsigned int nl;
-  trace_pixel<VT, XR_LINE_INT_SUM, LAYOUT>(J.p, proj, row, col, &nl);
+  trace_pixel<VT, XR_LINE_INT_SUM, LAYOUT, false, BLEND>(J.p, proj, row, col, &nl);
 }
 
 constexpr int kMaxDevices = 64;
 
-template <int VT, int LAYOUT>
+template <int VT, int LAYOUT, Blend BLEND>
 cudaError_t launch_fused_t(const FusedJob* d_jobs, int njobs, long long total, unsigned long long* d_counter,
                            int* blocks_out, cudaStream_t s) {
   static std::atomic<int> cached[kMaxDevices];  // blocks per device; zero = not known yet
@@ -1321,16 +1319,16 @@ cudaError_t launch_fused_t(const FusedJob* d_jobs, int njobs, long long total, u
     // every resident block leaves the rest of the SM's unified L1 to the gathers
     cudaFuncAttributes fa{};
     int smem_sm = 0;
-    cudaError_t e = cudaFuncGetAttributes(&fa, eval_fused_kernel<VT, LAYOUT>);
+    cudaError_t e = cudaFuncGetAttributes(&fa, eval_fused_kernel<VT, LAYOUT, BLEND>);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     if (e != cudaSuccess) return e;
     const double need = (double)(fa.sharedSizeBytes + 1024) * fused_blocks(VT);
     const int pct = std::min(100, (int)std::ceil(100.0 * need / (double)std::max(smem_sm, 1)) + 1);
-    e = cudaFuncSetAttribute(eval_fused_kernel<VT, LAYOUT>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+    e = cudaFuncSetAttribute(eval_fused_kernel<VT, LAYOUT, BLEND>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eval_fused_kernel<VT, LAYOUT>, kThreads, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eval_fused_kernel<VT, LAYOUT, BLEND>, kThreads, 0);
     if (e != cudaSuccess) return e;
     blocks = sms * (per_sm > 0 ? per_sm : 1);
     cached[dev].store(blocks, std::memory_order_relaxed);
@@ -1338,32 +1336,32 @@ cudaError_t launch_fused_t(const FusedJob* d_jobs, int njobs, long long total, u
   *blocks_out = blocks;
   cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  eval_fused_kernel<VT, LAYOUT><<<blocks, kThreads, 0, s>>>(d_jobs, njobs, total, d_counter);
+  eval_fused_kernel<VT, LAYOUT, BLEND><<<blocks, kThreads, 0, s>>>(d_jobs, njobs, total, d_counter);
   return cudaGetLastError();
 }
 
-template <int VT, int LAYOUT, bool GROUPED>
+template <int VT, int LAYOUT, bool GROUPED, Blend BLEND>
 cudaError_t launch_jobs_g(const MultiJobDrr* d_jobs, int njobs, long long total, cudaStream_t s) {
   static std::atomic<bool> carveout_set[kMaxDevices];
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
       !carveout_set[dev].load(std::memory_order_relaxed)) {
-    cudaFuncSetAttribute(drr_jobs_kernel<VT, LAYOUT, GROUPED>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(drr_jobs_kernel<VT, LAYOUT, GROUPED, BLEND>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxL1);
     carveout_set[dev].store(true, std::memory_order_relaxed);
   }
   const long long max_x = 0x7fffffff;
   for (long long base = 0; base < total; base += max_x) {
     const long long n = (total - base) < max_x ? (total - base) : max_x;
-    drr_jobs_kernel<VT, LAYOUT, GROUPED><<<(unsigned)n, jobs_threads(GROUPED), 0, s>>>(d_jobs, njobs, base);
+    drr_jobs_kernel<VT, LAYOUT, GROUPED, BLEND><<<(unsigned)n, jobs_threads(GROUPED), 0, s>>>(d_jobs, njobs, base);
   }
   return cudaGetLastError();
 }
 
-template <int VT, int LAYOUT>
+template <int VT, int LAYOUT, Blend BLEND>
 cudaError_t launch_jobs_t(const MultiJobDrr* d_jobs, int njobs, long long total, bool grouped, cudaStream_t s) {
-  return grouped ? launch_jobs_g<VT, LAYOUT, true>(d_jobs, njobs, total, s)
-                 : launch_jobs_g<VT, LAYOUT, false>(d_jobs, njobs, total, s);
+  return grouped ? launch_jobs_g<VT, LAYOUT, true, BLEND>(d_jobs, njobs, total, s)
+                 : launch_jobs_g<VT, LAYOUT, false, BLEND>(d_jobs, njobs, total, s);
 }
 
 template <int VT, int KERNEL, int LAYOUT, bool DEEP, Blend BLEND>
@@ -1480,39 +1478,39 @@ cudaError_t launch_drr(const DrrParams& params, cudaStream_t s) {
   }
 }
 
+// CALL(voxel type, layout, blend) for the jobs' voxel type and layout: the cell layouts
+// by their blend, LINEAR by each volume's own.
+#define XR_BY_VOLUME(CALL)                                                                                        \
+  switch (voxel_type * 4 + layout) {                                                                              \
+    case XR_VOXEL_F32 * 4 + XR_LAYOUT_LINEAR: return CALL(XR_VOXEL_F32, XR_LAYOUT_LINEAR, Blend::kVolume);        \
+    case XR_VOXEL_F32 * 4 + kLayoutCell8Wide:                                                                     \
+      return weighted ? CALL(XR_VOXEL_F32, kLayoutCell8Wide, Blend::kWeights)                                     \
+                      : CALL(XR_VOXEL_F32, kLayoutCell8Wide, Blend::kDifferences);                                \
+    case XR_VOXEL_F16 * 4 + XR_LAYOUT_LINEAR: return CALL(XR_VOXEL_F16, XR_LAYOUT_LINEAR, Blend::kVolume);        \
+    case XR_VOXEL_F16 * 4 + XR_LAYOUT_CELL8: return CALL(XR_VOXEL_F16, XR_LAYOUT_CELL8, Blend::kDifferences);     \
+    case XR_VOXEL_BF16 * 4 + XR_LAYOUT_LINEAR: return CALL(XR_VOXEL_BF16, XR_LAYOUT_LINEAR, Blend::kVolume);      \
+    case XR_VOXEL_BF16 * 4 + XR_LAYOUT_CELL8:                                                                     \
+      return weighted ? CALL(XR_VOXEL_BF16, XR_LAYOUT_CELL8, Blend::kWeights)                                     \
+                      : CALL(XR_VOXEL_BF16, XR_LAYOUT_CELL8, Blend::kDifferences);                                \
+    default: return cudaErrorInvalidValue;                                                                        \
+  }
+
 cudaError_t launch_eval_fused(const FusedJob* d_jobs, int njobs, long long total, int32_t voxel_type, int32_t layout,
-                              unsigned long long* d_counter, int* blocks_out, cudaStream_t s) {
+                              bool weighted, unsigned long long* d_counter, int* blocks_out, cudaStream_t s) {
   *blocks_out = 0;
   if (total <= 0) return cudaSuccess;
-#define XR_FUSED(V, L) \
-  case V * 4 + L: return launch_fused_t<V, L>(d_jobs, njobs, total, d_counter, blocks_out, s)
-  switch (voxel_type * 4 + layout) {
-    XR_FUSED(XR_VOXEL_F32, XR_LAYOUT_LINEAR);
-    XR_FUSED(XR_VOXEL_F32, kLayoutCell8Wide);
-    XR_FUSED(XR_VOXEL_F16, XR_LAYOUT_LINEAR);
-    XR_FUSED(XR_VOXEL_F16, XR_LAYOUT_CELL8);
-    XR_FUSED(XR_VOXEL_BF16, XR_LAYOUT_LINEAR);
-    XR_FUSED(XR_VOXEL_BF16, XR_LAYOUT_CELL8);
-    default: return cudaErrorInvalidValue;
-  }
+#define XR_FUSED(V, L, B) launch_fused_t<V, L, B>(d_jobs, njobs, total, d_counter, blocks_out, s)
+  XR_BY_VOLUME(XR_FUSED)
 #undef XR_FUSED
 }
 
 cudaError_t launch_drr_jobs(const MultiJobDrr* d_jobs, int njobs, long long total, int32_t voxel_type, int32_t layout,
-                            bool grouped, cudaStream_t s) {
+                            bool weighted, bool grouped, cudaStream_t s) {
   if (total <= 0) return cudaSuccess;
-#define XR_JOBS(V, L) \
-  case V * 4 + L: return launch_jobs_t<V, L>(d_jobs, njobs, total, grouped, s)
-  switch (voxel_type * 4 + layout) {
-    XR_JOBS(XR_VOXEL_F32, XR_LAYOUT_LINEAR);
-    XR_JOBS(XR_VOXEL_F32, kLayoutCell8Wide);
-    XR_JOBS(XR_VOXEL_F16, XR_LAYOUT_LINEAR);
-    XR_JOBS(XR_VOXEL_F16, XR_LAYOUT_CELL8);
-    XR_JOBS(XR_VOXEL_BF16, XR_LAYOUT_LINEAR);
-    XR_JOBS(XR_VOXEL_BF16, XR_LAYOUT_CELL8);
-    default: return cudaErrorInvalidValue;
-  }
+#define XR_JOBS(V, L, B) launch_jobs_t<V, L, B>(d_jobs, njobs, total, grouped, s)
+  XR_BY_VOLUME(XR_JOBS)
 #undef XR_JOBS
 }
+#undef XR_BY_VOLUME
 
 }  // namespace xr
