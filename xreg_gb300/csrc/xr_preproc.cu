@@ -284,17 +284,15 @@ struct SplineDouble {
   double* coef;
 };
 
-__device__ __noinline__ void spline_lines_double(const SplineDouble& d, bool columns, double z, double gain,
-                                                 int horizon) {
+template <bool COLUMNS>
+__device__ __noinline__ void spline_lines_double(const float* __restrict__ img, int rows, int cols,
+                                                 double* __restrict__ coef, double z, double gain, int horizon) {
   const int threads = gridDim.x * gridDim.y * blockDim.x;
   const int first = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
-  if (columns) {
-    for (int c = first; c < d.cols; c += threads)
-      bspline_prefilter_line(d.coef + c, d.rows, d.cols, z, gain, horizon);
-    return;
+  for (int l = first; l < (COLUMNS ? cols : rows); l += threads) {
+    if constexpr (COLUMNS) bspline_prefilter_line(coef + l, rows, cols, z, gain, horizon);
+    else bspline_prefilter_line(coef + (int64_t)l * cols, cols, 1, z, gain, horizon, img + (int64_t)l * cols);
   }
-  for (int r = first; r < d.rows; r += threads)
-    bspline_prefilter_line(d.coef + (int64_t)r * d.cols, d.cols, 1, z, gain, horizon, d.img + (int64_t)r * d.cols);
 }
 
 __global__ void spline_double_kernel(const double* __restrict__ coef, int rows, int cols, double factor, int orows,
@@ -327,7 +325,7 @@ __global__ void __launch_bounds__(32) spline_kernel(const TIn* __restrict__ in, 
   __shared__ FF w[kOuts][4];
   __shared__ int first[kOuts];  // index of an output's second coefficient, -1: outside the image
   if (*beyond) {
-    spline_lines_double(dbl, sizeof(TOut) == sizeof(float), z_d, gain_d, horizon);
+    spline_lines_double<sizeof(TOut) == sizeof(float)>(dbl.img, dbl.rows, dbl.cols, dbl.coef, z_d, gain_d, horizon);
     return;
   }
   const int lane = threadIdx.x, l0 = blockIdx.y * 32;
