@@ -38,3 +38,30 @@ def test_alone_and_among_many(xr, oracle, grad, radius, stride, masked):
     f = oracle.patch_grad_ncc_ex if grad else oracle.patch_ncc_ex
     ref = f(fixed, movs[[0, -1]], radius=radius, stride=stride, mask=mask)
     np.testing.assert_allclose(got[0][[0, -1]], ref, atol=1e-5, rtol=0)
+
+
+@pytest.mark.parametrize("masked,nimgs", [(False, 1), (False, 60), (True, 1), (True, 60)])
+def test_the_largest_windows_are_refused_alike(xr, masked, nimgs):
+    """Both gradients' tile of 16 x 16 patches must fit 200 KB, whatever kernel runs."""
+    import torch
+    from xreg_gb300 import XRegError
+    shape = (150, 170)
+    rng = np.random.default_rng(4)
+    d = torch.from_numpy(rng.random((nimgs,) + shape).astype(np.float32)).cuda()
+    torch.cuda.synchronize()
+    for radius, stride, ok in [(10, 4, True), (11, 4, False), (12, 4, False), (16, 3, True), (16, 4, False)]:
+        m = xr.ImgSimMetric2DPatchGradNCCCUDA()
+        m.set_fixed_image(rng.random(shape).astype(np.float32))
+        if masked:
+            m.set_mask((rng.random(shape) < 0.7).astype(np.uint8))
+        m.set_patch_radius(radius)
+        m.set_patch_stride(stride)
+        m.set_num_moving_images(nimgs)
+        m.set_mov_imgs_device_buf(d.data_ptr())
+        m.allocate_resources()
+        if ok:
+            m.compute()
+            assert np.all(np.isfinite(m.sim_vals()))
+        else:
+            with pytest.raises(XRegError):
+                m.compute()

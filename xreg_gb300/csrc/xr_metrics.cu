@@ -1377,6 +1377,10 @@ cudaError_t launch_patch_ncc(const float* mov, int rows, int cols, int64_t nimgs
   const int nblk = general ? patch_general_tiles(ncr, ncc) : patch_tiles(ncr, ncc, kPartRows);
   if (nblk_out) *nblk_out = nblk;
   if (nimgs <= 0 || !partials) return cudaSuccess;
+  // One limit of radius and stride for every form, the general kernel's: options and the
+  // number of images do not decide what is refused.
+  const PatchLayout L = PatchLayout::make(radius, stride, grad, kr);
+  if (L.bytes > kPatchSmem) return cudaErrorInvalidValue;
   if (!general) {
     if (pass != 1) return cudaErrorInvalidValue;
     int rb = 1;
@@ -1402,8 +1406,6 @@ cudaError_t launch_patch_ncc(const float* mov, int rows, int cols, int64_t nimgs
 #undef XR_ROWS
   }
   const dim3 grid(nblk, (unsigned)nimgs);
-  const PatchLayout L = PatchLayout::make(radius, stride, grad, kr);
-  if (L.bytes > kPatchSmem) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
 #define XR_PATCH_LAUNCH(G, K, P)                                                                                       \
   e = set_smem(patch_ncc_kernel<G, K, P>, L.bytes);                                                                    \
