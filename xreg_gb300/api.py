@@ -463,9 +463,6 @@ class ImgSimMetric2DCUDA:
         call("xr_sm_fixed_image", self._h, 0, None, C.byref(r), C.byref(c))
         return out.reshape(r.value, c.value)
 
-    def num_moving_images(self) -> int:
-        return self._n
-
     def set_mov_imgs_buf_from_ray_caster(self, rc: RayCasterLineIntCUDA, proj_offset: int = 0) -> None:
         call("xr_sm_set_mov_imgs_buf_from_ray_caster", self._h, rc.handle, int(proj_offset))
         self._rc_ref = rc  # keep the ray caster alive at least as long as this metric
@@ -487,7 +484,7 @@ class ImgSimMetric2DCUDA:
         call("xr_sm_compute", self._h)
 
     def sim_vals(self) -> np.ndarray:
-        out = np.empty(self._n, dtype=np.float32)
+        out = np.empty(self.num_moving_images(), dtype=np.float32)  # an objective sets it too
         call("xr_sm_sim_vals", self._h, _ptr(out))
         return out
 

@@ -1866,6 +1866,24 @@ extern "C" XR_API xr_status xr_sm_allocate_resources(xr_simmetric sm) {
 
 static xr_status sm_enqueue_compute_on(xr_simmetric sm, cudaStream_t s);
 
+// A metric's buffers for `n` moving images: an objective's population may exceed the
+// number its metric was allocated again for.  Captured launches that hold the old
+// buffers are not valid any more (generation).
+static xr_status sm_reserve_images(xr_simmetric sm, int64_t n) {
+  const void* const held[4] = {sm->d_partials.p, sm->d_sims.p, sm->d_pscores.p, sm->d_mvar_sum.p};
+  const bool patch = sm->kind == XR_SIM_PATCH_NCC || sm->kind == XR_SIM_PATCH_GRAD_NCC;
+  const size_t sums = patch ? 2 : (sm->kind == XR_SIM_GRAD_NCC ? 6 : 3);
+  XR_CUDA_TRY(sm->d_partials.reserve((size_t)n * sm->nblk * sums * 8));
+  XR_CUDA_TRY(sm->d_sims.reserve((size_t)n * 4));
+  if (patch && sm->popt.save_all_per_patch_scores)
+    XR_CUDA_TRY(sm->d_pscores.reserve((size_t)n * (size_t)sm->ncr * (size_t)sm->ncc * 4));
+  if (patch && sm->mvar_mode) XR_CUDA_TRY(sm->d_mvar_sum.reserve((size_t)n * 2 * 8));
+  if (held[0] != sm->d_partials.p || held[1] != sm->d_sims.p || held[2] != sm->d_pscores.p ||
+      held[3] != sm->d_mvar_sum.p)
+    sm->generation++;
+  return XR_OK;
+}
+
 static xr_status sm_enqueue_compute(xr_simmetric sm) {
   XR_CHECK_ARG(sm, "compute: NULL handle");
   return sm_enqueue_compute_on(sm, sm->stream());
@@ -1875,6 +1893,10 @@ static xr_status sm_enqueue_compute(xr_simmetric sm) {
 static xr_status sm_enqueue_compute_on(xr_simmetric sm, cudaStream_t s) {
   XR_CHECK_ARG(sm, "compute: NULL handle");
   if (!sm->allocated) return fail(XR_ERR_NOT_ALLOCATED, "compute: allocate_resources has not been called");
+  if (sm->num_mov > sm->capacity) {
+    const xr_status st = sm_reserve_images(sm, sm->num_mov);
+    if (st != XR_OK) return st;
+  }
   const int64_t npix = sm->rows * sm->cols;
   const float* mov = nullptr;
   if (xr_raycaster rc = sm->live_rc()) {
@@ -2097,9 +2119,8 @@ static xr_status metric_job(xr_objective obj, int64_t pop, FusedJob& J, std::vec
     m->proj_offset = (int64_t)v * pop;
     if (J.metric) {
       XR_CHECK_ARG(m->nblk == J.mt_x * J.mt_y, "evaluation: metric buffers do not fit");
-      // a metric allocated again for fewer images than this population
-      XR_CUDA_TRY(m->d_partials.reserve((size_t)pop * m->nblk * 6 * 8));
-      XR_CUDA_TRY(m->d_sims.reserve((size_t)pop * 4));
+      const xr_status st = sm_reserve_images(m, pop);
+      if (st != XR_OK) return st;
       FusedView V{};
       V.fhx = m->fx.fhat;
       V.fhy = m->fy.fhat;
