@@ -80,3 +80,19 @@ def test_in_a_job_set(xr, kind, options):
     m.set_num_moving_images(1)
     m.allocate_resources()
     np.testing.assert_array_equal(xr.JobSet().eval([obj], [poses])[0], obj0.eval(poses))
+
+
+def test_a_refused_step_binds_the_metric_to_its_population(xr):
+    """A job step larger than the metric's allocation is refused, and allocating again
+    then makes room for that step's population."""
+    m = _metric(xr, "ImgSimMetric2DGradNCCCUDA")
+    _, obj, poses = _objective(xr, m)
+    want = obj.eval(poses[:40])
+    m.set_num_moving_images(3)
+    m.allocate_resources()
+    js = xr.JobSet()
+    with pytest.raises(xr.XRegError):
+        js.eval([obj], [poses[:40]])
+    assert m.num_moving_images() == 40
+    m.allocate_resources()
+    np.testing.assert_array_equal(js.eval([obj], [poses[:40]])[0], want)

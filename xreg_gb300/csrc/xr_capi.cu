@@ -2102,8 +2102,10 @@ static int metric_launches(const xr_simmetric_s* m) {
 
 // Binds an objective's metrics to the images of a population of `pop` and, when
 // J.metric is set, fills J's part of the batched (or fused) grad-NCC: its tiles, its
-// views and its counters.
-static xr_status metric_job(xr_objective obj, int64_t pop, FusedJob& J, std::vector<FusedView>& views, cudaStream_t s) {
+// views and its counters.  A metric allocated for fewer images grows its buffers, or
+// (grow false: job steps) refuses.
+static xr_status metric_job(xr_objective obj, int64_t pop, FusedJob& J, std::vector<FusedView>& views, bool grow,
+                            cudaStream_t s) {
   xr_raycaster rc = obj->rc;
   const int32_t nv = (int32_t)obj->metrics.size();
   J.nviews = nv;
@@ -2118,7 +2120,8 @@ static xr_status metric_job(xr_objective obj, int64_t pop, FusedJob& J, std::vec
     m->rc_id = rc->id;
     m->proj_offset = (int64_t)v * pop;
     if (J.metric) {
-      XR_CHECK_ARG(m->nblk == J.mt_x * J.mt_y, "evaluation: metric buffers do not fit");
+      XR_CHECK_ARG(m->nblk == J.mt_x * J.mt_y && (grow || m->capacity >= pop),
+                   "evaluation: metric buffers do not fit");
       const xr_status st = sm_reserve_images(m, pop);
       if (st != XR_OK) return st;
       FusedView V{};
@@ -2155,7 +2158,7 @@ static xr_status obj_grad_metric(xr_objective obj, int64_t pop, cudaStream_t s) 
   FusedJob J{};
   std::vector<FusedView> views;
   J.metric = 1;
-  xr_status st = metric_job(obj, pop, J, views, s);
+  xr_status st = metric_job(obj, pop, J, views, true, s);
   if (st != XR_OK) return st;
   J.d.p.out = rc_out(obj->rc, nullptr);
   J.d.p.rows = (int32_t)obj->rc->rows();
@@ -2298,9 +2301,7 @@ static xr_status step_enqueue(FusedWork& fw, int device, int32_t n, const xr_obj
     gj.push_back(G);
     // the metric behind the DRR
     J.metric = obj_metric_fusable(obj) ? 1 : 0;
-    for (xr_simmetric m : obj->metrics)
-      XR_CHECK_ARG(!J.metric || m->capacity >= pop, "evaluation: metric buffers do not fit");
-    if ((st = metric_job(obj, pop, J, fv[(size_t)i], s)) != XR_OK) return st;
+    if ((st = metric_job(obj, pop, J, fv[(size_t)i], false, s)) != XR_OK) return st;
     if (dopt) {
       J.report = d_report + i;
       if (!fused && J.metric) J.cma = cma[i].state;  // updated by the batched grad-NCC launch
